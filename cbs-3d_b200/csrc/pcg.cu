@@ -906,29 +906,6 @@ __device__ __forceinline__ bool grid_allreduce_v(double (&v)[NV], const PcgDev& 
     return ok;
 }
 
-template <int NT>
-__device__ __forceinline__ bool grid_allreduce3(Acc6 v, const PcgDev& D, const SegView& g, int phase, Acc6& out)
-{
-    double a[5] = {v.a, v.b, v.c, v.mx, v.flag}, o[5];
-    const bool ok = grid_allreduce_v<5, 3, NT>(a, D, g, phase, o);
-    out = Acc6{o[0], o[1], o[2], o[3], o[4]};
-    return ok;
-}
-
-// Five sums, a max and a flag (the mixed solver's refresh after a correction).
-struct Acc8 {
-    double a, b, c, d, e, mx, flag;
-};
-
-template <int NT>
-__device__ __forceinline__ bool grid_allreduce5(Acc8 v, const PcgDev& D, const SegView& g, int phase, Acc8& out)
-{
-    double a[7] = {v.a, v.b, v.c, v.d, v.e, v.mx, v.flag}, o[7];
-    const bool ok = grid_allreduce_v<7, 5, NT>(a, D, g, phase, o);
-    out = Acc8{o[0], o[1], o[2], o[3], o[4], o[5], o[6]};
-    return ok;
-}
-
 // Grid all-reduce of (sum a, sum b, sum c, max mx, max flag) that also
 // gathers one per-CTA sum: every CTA's block sum of `x` lands in cvec[CTA]
 // of every CTA (the aggregated vectors of the two-level preconditioner).
@@ -1018,6 +995,239 @@ __device__ __forceinline__ bool grid_allreduce3g(Acc6 v, double x, const PcgDev&
     return ok;
 }
 
+// ------------------------------------------------------ tagged exchange
+// The single-reduction kernels (k_pcg64c, k_pcg64g) exchange values between
+// CTAs as 16-byte records {value, tag} that are written and read whole
+// (.b128 accesses are single-copy atomic), so a reader that finds the tag it
+// waits for holds the value of that exchange: no counter, and for the values
+// themselves no fence.  The tag is the solve's epoch (a counter in device
+// memory, one more per solve) in the high word and the exchange's number in
+// the solve in the low word, so nothing has to be cleared between solves.
+// Two buffers alternate by the exchange's parity.  A CTA writes exchange k+2
+// over exchange k only after all-reduce k+1, to which every CTA contributes
+// after it has read its records of exchange k.
+__device__ __forceinline__ void st_tag(TagVal* p, double v, unsigned long long tag)
+{
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_tag(const TagVal* p, double& v, unsigned long long& tag)
+{
+    long long b;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(b), "=l"(tag)
+                 : "l"(p)
+                 : "memory");
+    v = __longlong_as_double(b);
+}
+
+// One solve's side of the exchange, for this CTA.
+struct TagComm {
+    TagVal* rec;                 // 2 x G all-reduce records of REC_STRIDE
+    int G, b;
+    unsigned long long epoch;    // the solve's epoch in the high word
+    DevStatus* status;
+    __device__ __forceinline__ unsigned long long tag(int phase) const { return epoch | (unsigned)(phase + 1); }
+};
+__device__ __forceinline__ TagComm tag_comm(const PcgDev& D, const SegView& g, unsigned long long epoch)
+{
+    return TagComm{g.k < 0 ? D.rec : D.inst[g.k].rec, g.G, g.b, epoch, seg_status(D, g)};
+}
+__device__ __forceinline__ unsigned long long* seg_epoch(const PcgDev& D, const SegView& g) { return g.k < 0 ? D.epoch : D.inst[g.k].epoch; }
+
+// A wait's slow path: every 64 unsuccessful polls look for a status raised
+// elsewhere, and give up (TIMEOUT) after about a second.
+struct SpinLimit {
+    int spins = 0;
+    long long t0 = 0;
+    __device__ __forceinline__ bool expired(DevStatus* status)
+    {
+        if ((++spins & 63) != 0) return false;
+        if (ld_relaxed_int(&status->code) != 0) return true;
+        const long long t = clock64();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > (1LL << 31)) {
+            set_status(status, 5 /*CBS3D_TIMEOUT*/, ST_PCG, 0, R_PCG_BARRIER);
+            return true;
+        }
+        return false;
+    }
+};
+
+// The maximum is taken over the bits of magnitudes, whose order is that of
+// the values with infinities and NaN above every finite one: a non-finite
+// entry anywhere shows in the total.
+__device__ __forceinline__ double max_bits(double a, double b)
+{
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return __longlong_as_double(x > y ? x : y);
+}
+template <bool MX>
+__device__ __forceinline__ double red4(int q, double a, double b)
+{
+    if constexpr (MX) return q == 3 ? max_bits(a, b) : a + b;
+    else return a + b;
+}
+
+// All-reduce of three sums and, with MX, a maximum of magnitudes, in two
+// halves so that a kernel can put work between them.  The all-reduce is a
+// serial chain (shuffles, a store, a poll, shuffles), so its instructions
+// count: the maximum, whose comparisons double them, is left out of the
+// iterations that need none.  Publish: a warp halves its values with its
+// lanes (6 exchanges for four values instead of 20), one warp folds the
+// CTA's warps, and four of its lanes write the CTA's record with one store.
+// Every CTA's record has a 128-byte line of its own: a line that other SMs
+// poll costs a store to it about 0.4 us on B200 (each poll leaves a copy
+// that the store has to recall), so with eight CTAs' values to a line a
+// 148-CTA all-reduce took 4-6 us, with one 2.0 us (against 2.4 us for a
+// counter and separate partials).
+// ORDERED: the CTA's earlier plain stores are made visible before the record
+// (a fence), for kernels that exchange vectors by plain stores.
+constexpr int REC_STRIDE = 8;    // TagVals per record: one 128-byte line
+template <int NT, bool ORDERED, bool MX>
+__device__ __forceinline__ void tag_allreduce_publish(const TagComm& c, int phase, const double (&v)[4])
+{
+    constexpr int NW = NT / 32;
+    static_assert(NW == 8 || NW == 16, "warps per CTA");
+    __shared__ double sm[4][NW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool h = lane & 16, e = lane & 8;
+    const int q = lane >> 3;     // the value this lane ends up with
+    const double v3 = MX ? v[3] : 0.0;
+    double k0 = h ? v[2] : v[0], k1 = h ? v3 : v[1];
+    const double x0 = __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+    const double x1 = __shfl_xor_sync(0xffffffffu, h ? v[1] : v3, 16);
+    k0 += x0;
+    k1 = red4<MX>(h ? 3 : 1, k1, x1);
+    double k = e ? k1 : k0;
+    k = red4<MX>(q, k, __shfl_xor_sync(0xffffffffu, e ? k0 : k1, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) k = red4<MX>(q, k, __shfl_xor_sync(0xffffffffu, k, o));
+    if ((lane & 7) == 0) sm[q][warp] = k;
+    __syncthreads();
+    if (warp == 0) {
+        double x = sm[q][lane & 7];
+        if (NW == 16) x = red4<MX>(q, x, sm[q][(lane & 7) + 8]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) x = red4<MX>(q, x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (ORDERED) __threadfence();
+        if ((lane & 7) == 0) st_tag(c.rec + ((phase & 1) * c.G + c.b) * REC_STRIDE + q, x, c.tag(phase));
+    }
+}
+
+// Wait: thread t polls value t%4 of CTAs t/4, t/4 + NT/4, ...; lanes, then
+// warps in a fixed order, so every CTA computes the same totals bit for bit.
+// all_in() runs when every record has come in, before the last fold.  `ok`:
+// false when an earlier wait of this thread gave up; the result is false for
+// the whole CTA then, when this wait gives up, or when another CTA raised a
+// status.
+// A poll that comes before its record costs the record's writer a recall and
+// the reader another round trip (24 CTAs: 4,150 cycles from the publish to
+// the totals, 3,180 with the first poll held back by 1,200), so each warp
+// holds its first poll back by `hold` cycles, adapted to the last exchanges:
+// a little longer after a miss, a little shorter after a hit.
+struct PollHold {
+    unsigned cycles = 0;
+    __device__ __forceinline__ void wait() const
+    {
+        const unsigned t0 = clock_lo();
+        while (clock_lo() - t0 < cycles) {}
+    }
+    __device__ __forceinline__ void learn(bool missed)
+    {
+        if (__any_sync(0xffffffffu, missed)) cycles = cycles < 4096u ? cycles + 64u : cycles;
+        else cycles = cycles > 16u ? cycles - 16u : 0u;
+    }
+    static __device__ __forceinline__ unsigned clock_lo()
+    {
+        unsigned t;
+        asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+        return t;
+    }
+};
+
+template <int NT, bool ORDERED, bool MX, typename F>
+__device__ __forceinline__ bool tag_allreduce_wait(const TagComm& c, int phase, double (&out)[4], bool ok, PollHold& hold,
+                                                   F&& all_in)
+{
+    constexpr int NW = NT / 32, STEP = NT / 4;
+    constexpr int MP = NT >= 512 ? 2 : 5;   // records per thread: grids of up to 256 or 320 CTAs
+    __shared__ double sm[NW][4];
+    const int lane = threadIdx.x & 31, q = threadIdx.x & 3, j = threadIdx.x >> 2;
+    const TagVal* r = c.rec + ((phase & 1) * c.G + j) * REC_STRIDE + q;
+    const unsigned long long want = c.tag(phase);
+    double a = 0.0;
+    if ((j & ~7) < c.G) {        // this warp has records to poll
+        double x[MP];
+        unsigned long long t[MP];
+        hold.wait();
+        // every record requested before the first is looked at
+        bool missed = false;
+#pragma unroll
+        for (int u = 0; u < MP; ++u) {
+            x[u] = 0.0;
+            t[u] = want;
+            if (j + u * STEP < c.G) ld_tag(r + u * STEP * REC_STRIDE, x[u], t[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < MP; ++u) missed = missed || t[u] != want;
+        hold.learn(missed);
+        if (missed) {
+            SpinLimit lim;
+#pragma unroll
+            for (int u = 0; u < MP; ++u)
+                while (t[u] != want) {
+                    if (lim.expired(c.status)) { ok = false; break; }
+                    ld_tag(r + u * STEP * REC_STRIDE, x[u], t[u]);
+                }
+        }
+        __syncwarp();
+        if (ORDERED) __threadfence();
+        a = x[0];
+#pragma unroll
+        for (int u = 1; u < MP; ++u) a = red4<MX>(q, a, x[u]);
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) a = red4<MX>(q, a, __shfl_xor_sync(0xffffffffu, a, o));
+    }
+    if (lane < 4) sm[threadIdx.x >> 5][lane] = a;
+    ok = __syncthreads_and(ok);
+    all_in();
+    a = sm[lane >> 2][q];
+    if (NW == 16) a = red4<MX>(q, a, sm[(lane >> 2) + 8][q]);
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) a = red4<MX>(q, a, __shfl_xor_sync(0xffffffffu, a, o));
+#pragma unroll
+    for (int p = 0; p < (MX ? 4 : 3); ++p) out[p] = __shfl_sync(0xffffffffu, a, p);
+    if (!MX) out[3] = 0.0;
+    return ok;
+}
+
+// Stopping test of the single-reduction kernels.  The exact test (a square
+// root, a division, max|r|) is made only where it may hold: with test 2 not
+// while (r,r) is above the square of rtol*||r0|| with a margin of 1e-12.
+struct StopTest {
+    int test;
+    double rtol, atol, init, bound;
+    __device__ __forceinline__ StopTest(const SegView& g, double init_)
+        : test(g.conv_test), rtol(g.rel_tol), atol(g.abs_tol), init(init_)
+    {
+        const double x = g.rel_tol * init_;
+        bound = x * x * (1.0 + 1.0e-12);
+        // near underflow, or with a test on max|r|: always the exact test
+        if (test != 2 || !(bound > 1.0e-280)) bound = __longlong_as_double(0x7ff0000000000000LL);
+    }
+    // the maximum is part of every iteration's all-reduce
+    __device__ __forceinline__ bool needs_max() const { return test != 2; }
+    // the iteration can go on without the exact test (a NaN or an infinite
+    // (r,r) is not above the bound, or not below infinity)
+    __device__ __forceinline__ bool clear(double rr) const { return rr > bound && rr < __longlong_as_double(0x7ff0000000000000LL); }
+    __device__ __forceinline__ bool exact(double rr, double mx) const
+    {
+        return cg_converged(test, sqrt(rr) / init, mx, rtol, atol);
+    }
+};
+
 // ------------------------------------ global-vector single-reduction PCG
 // The Chronopoulos-Gear iteration of k_pcg64c for meshes whose rows do not
 // fit the register tiling: the rows' r, s, w (double-buffered by iteration
@@ -1029,7 +1239,7 @@ __device__ __forceinline__ bool grid_allreduce3g(Acc6 v, double x, const PcgDev&
 // search direction lives in the engine's permuted right-hand side, which is
 // dead once r0 is formed.  Where the whole halo fits (one part) the inverse
 // diagonal of the halo stays in shared memory for the solve.
-__global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev D)
+__device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long epoch)
 {
     constexpr int NT = PCG_THREADS;
     const SegView g = seg_view<false>(D);
@@ -1042,6 +1252,8 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
     const bool dzres = KP == 1;   // the halo's inverse diagonal resident in shared memory
     double* vh = reinterpret_cast<double*>(smem_raw);
     double* dzh = vh + D.halo_max;
+    const TagComm comm = tag_comm(D, g, epoch);
+    PollHold hold;
     int phase = 0;
     const int N = D.N;
     double* rb[2] = {D.r, D.r + N};
@@ -1088,8 +1300,22 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
         return off;
     };
 
-    // ---- phase 0a: r0 = b - A x0 (constraints as the reference), dz, p = s = 0
-    Acc6 acc{0.0, 0.0, 0.0, 0.0, 0.0};
+    double t[4];
+    auto allreduce = [&](const double (&v)[4], bool with_max) {
+        bool ok;
+        if (with_max) {
+            tag_allreduce_publish<NT, true, true>(comm, phase, v);
+            ok = tag_allreduce_wait<NT, true, true>(comm, phase, t, true, hold, [] {});
+        } else {
+            tag_allreduce_publish<NT, true, false>(comm, phase, v);
+            ok = tag_allreduce_wait<NT, true, false>(comm, phase, t, true, hold, [] {});
+        }
+        ++phase;
+        return ok;
+    };
+    // ---- phase 0a: r0 = b - A x0 (constraints as the reference), dz, p = s = 0;
+    // partials: invalid diagonals, non-finite residuals, (r,r), max|r|
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int part = 0; part < KP; ++part) {
         const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
         const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
@@ -1110,32 +1336,31 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
             if (!fr) ri = 0.0;
             if (fr) {
                 if (g.precond) {
-                    if (!(isfinite(pd) && pd > 1.0e-30)) acc.flag = fmax(acc.flag, 1.0);
+                    if (!(isfinite(pd) && pd > 1.0e-30)) acc[0] += 1.0;
                     dd = 1.0 / pd;
                 } else {
                     dd = 1.0;
                 }
-                if (!isfinite(ri)) acc.flag = fmax(acc.flag, 2.0);
-                acc.c = fma(ri, ri, acc.c);
-                acc.mx = fmax(acc.mx, fabs(ri));
+                if (!isfinite(ri)) acc[1] += 1.0;
+                acc[2] = fma(ri, ri, acc[2]);
+                acc[3] = max_bits(acc[3], fabs(ri));
             }
             rb[0][i] = ri;
             dz[i] = dd;
             sb[0][i] = 0.0;
         }
     }
-    Acc6 t{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce3<NT>(acc, D, g, phase, t)) return;
-    ++phase;
-    const double init = sqrt(t.c);
-    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t.mx); return; }
-    if (cg_converged(g.conv_test, 1.0, t.mx, g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t.mx); return; }
-    if (t.flag >= 2.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
-    if (t.flag >= 1.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
+    if (!allreduce(acc, true)) return;
+    const double init = sqrt(t[2]);
+    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t[3]); return; }
+    if (cg_converged(g.conv_test, 1.0, t[3], g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t[3]); return; }
+    if (t[1] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
+    if (t[0] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
+    const StopTest stop(g, init);
 
     // ---- phase 0b: z0 = M^-1 r0, w0 = A z0, gamma0 = (r0,z0), delta0 = (z0,w0);
     // the right-hand side is no longer needed: p = 0 from here
-    acc = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
     for (int part = 0; part < KP; ++part) {
         const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
         const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
@@ -1160,18 +1385,16 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
             wb[0][i] = wi;
             pv[i] = 0.0;
             if (fr) {
-                acc.a = fma(ri, zi, acc.a);
-                acc.b = fma(zi, wi, acc.b);
+                acc[0] = fma(ri, zi, acc[0]);
+                acc[1] = fma(zi, wi, acc[1]);
             }
         }
     }
-    t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce3<NT>(acc, D, g, phase, t)) return;
-    ++phase;
-    double gam = t.a;
+    if (!allreduce(acc, false)) return;
+    double gam = t[0];
     if (gam <= 1.0e-300 || !isfinite(gam)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, 0, R_PCG_RZ0); return; }
-    double den = t.b;
-    double beta = 0.0, fin = init, rel = 1.0, mx = 0.0, alpha = 0.0;
+    double den = t[1];
+    double beta = 0.0, rr = t[2], mx = 0.0, alpha = 0.0;
     int it = 0, conv = 0;
     for (it = 1; it <= g.max_iter; ++it) {
         if (fabs(den) <= 1.0e-300 || !isfinite(den)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_PAP); return; }
@@ -1180,7 +1403,7 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
         const double* so = sb[po];
         const double* wo = wb[po];
         const double* ro = rb[po];
-        Acc6 a6{0.0, 0.0, 0.0, 0.0, 0.0};
+        acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
         for (int part = 0; part < KP; ++part) {
             const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
             const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
@@ -1236,31 +1459,65 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
                 const double wi = fr ? fma(D.pdiag[i], zi, off) : 0.0;
                 wb[pn][i] = wi;
                 if (fr) {
-                    if (!isfinite(ri)) a6.flag = 1.0;
-                    a6.a = fma(ri, zi, a6.a);
-                    a6.b = fma(zi, wi, a6.b);
-                    a6.c = fma(ri, ri, a6.c);
-                    a6.mx = fmax(a6.mx, fabs(ri));
+                    acc[0] = fma(ri, zi, acc[0]);
+                    acc[1] = fma(zi, wi, acc[1]);
+                    acc[2] = fma(ri, ri, acc[2]);
+                    acc[3] = max_bits(acc[3], fabs(ri));
                 }
             }
         }
-        t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-        if (!grid_allreduce3<NT>(a6, D, g, phase, t)) return;
-        ++phase;
-        fin = sqrt(t.c);
-        mx = t.mx;
-        rel = fin / init;
-        if (cg_converged(g.conv_test, rel, mx, g.rel_tol, g.abs_tol)) { conv = 1; break; }
-        if (t.flag > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
-        const double gn = t.a;
-        if (gn <= 1.0e-300 || !isfinite(gn)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
+        if (!allreduce(acc, stop.needs_max())) return;
+        rr = t[2];
+        mx = t[3];
+        const double gn = t[0], delta = t[1];
+        if (!stop.clear(rr) || gn <= 1.0e-300 || !isfinite(gn)) {
+            if (!stop.needs_max()) {
+                acc[0] = acc[1] = acc[2] = 0.0;
+                if (!allreduce(acc, true)) return;
+                mx = t[3];
+            }
+            if (stop.exact(rr, mx)) { conv = 1; break; }
+            if (!isfinite(mx)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
+            if (gn <= 1.0e-300 || !isfinite(gn)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
+        }
         beta = gn / gam;
-        den = t.b - beta * gn / alpha;
+        den = fma(-beta * beta, den, delta);
         gam = gn;
     }
+    if (!conv && !stop.needs_max()) {
+        acc[0] = acc[1] = acc[2] = 0.0;
+        if (!allreduce(acc, true)) return;
+        mx = t[3];
+    }
     if (it > g.max_iter) it = g.max_iter;
-    cg_finish(D, g, it, conv, init, fin, rel, mx);
+    cg_finish(D, g, it, conv, init, sqrt(rr), sqrt(rr) / init, mx);
     if (!conv && b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 2, ST_PCG, it, R_PCG_MAXIT);
+}
+
+// The epoch of this solve, and whether an earlier stage has already failed
+// (then no CTA starts); after the solve the next one's epoch.  CTA 0 cannot
+// get past its first all-reduce, let alone here, before every CTA has read
+// the epoch.
+template <bool BATCH>
+__device__ __forceinline__ bool tag_begin(const PcgDev& D, unsigned long long& epoch)
+{
+    const SegView g = seg_view<BATCH>(D);
+    epoch = *seg_epoch(D, g) << 32;
+    return !__syncthreads_or(threadIdx.x == 0 && ld_relaxed_int(&seg_status(D, g)->code) != 0);
+}
+template <bool BATCH>
+__device__ __forceinline__ void tag_end(const PcgDev& D, unsigned long long epoch)
+{
+    const SegView g = seg_view<BATCH>(D);
+    if (g.b == 0 && threadIdx.x == 0) *seg_epoch(D, g) = (epoch >> 32) + 1;
+}
+
+__global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev D)
+{
+    unsigned long long epoch;
+    if (!tag_begin<false>(D, epoch)) return;
+    pcg64g_body(D, epoch);
+    tag_end<false>(D, epoch);
 }
 
 // ---------------------------------------------- tensor memory as storage
@@ -1324,39 +1581,59 @@ __device__ __forceinline__ void tmem_hold(uint32_t (&r)[N])
     for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
 }
 
+// The single-reduction iteration with the rows' vectors in registers.  Row by
+// row it performs the operations of pcg64g_body in the same order.
+//
+// Exchange.  A CTA keeps the neighbour values that other CTAs own ("remote"
+// entries of its halo) up to date itself: r and s of those rows follow the
+// same recurrences from the same alpha, beta as at their owners, so the only
+// vector that crosses CTAs is w, one tagged record per row and iteration
+// (staging r, s and w cost three values and a second trip to L2 after the
+// all-reduce).  The records are requested when the other CTAs' partials have
+// come in -- a CTA stores its w before its partials, so they are there, and
+// polling them earlier would slow their stores -- and travel while the
+// partials are folded; neither exchange needs a fence.  The own rows' new z go from registers into the halo.
+//
+// Bound at 64^3: shared-memory wavefronts of the gathers (27,000 per CTA and
+// iteration, at two 64-bit wavefronts per 32 and the bank conflicts left) and
+// the latency of the all-reduce.
+//
 // KT > 0: the coefficients of each thread's rows KS .. KS+KT-1 live in TMEM
 // for the solve (D.tm_w slots per row, zero-padded past the slice's width);
 // `tm` is the CTA's TMEM base address (0 when KT = 0).
 template <int RMAX, bool BATCH, int NT, int KS, int KT>
-__device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
+__device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsigned long long epoch)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SegView g = seg_view<BATCH>(D);
+    const TagComm comm = tag_comm(D, g, epoch);
+    PollHold hold;
     const int G = g.G, b = g.b;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s_beg = g.s0 + (int)((long long)b * (g.s1 - g.s0) / G);
     const int s_end = g.s0 + (int)((long long)(b + 1) * (g.s1 - g.s0) / G);
     const long long S0 = D.slice_off[s_beg];
-    const int nsl = (int)(D.slice_off[s_end] - S0);
     const int h0 = D.halo_ptr[blockIdx.x];
     const int nh = D.halo_ptr[blockIdx.x + 1] - h0;
-    double* vh = reinterpret_cast<double*>(smem_raw);
-    double* dzh = vh + D.halo_max;
-    int* hidx = reinterpret_cast<int*>(dzh + D.halo_max);
-    unsigned short* lcs = reinterpret_cast<unsigned short*>(hidx + D.halo_max);
-    // the own rows' pressure and diagonal, kept in shared memory for the
-    // solve when the engine sized it so (the two-CTAs-per-SM kernel of small
-    // meshes only; the other instantiations compile the global accesses alone)
-    constexpr bool XS = NT == 256 && !BATCH;
-    double* xs = XS && D.xs_off ? reinterpret_cast<double*>(smem_raw + D.xs_off) : nullptr;
-    double* pds = xs ? xs + RMAX * NT
-                : (NT == 512 && !BATCH && D.pds_off ? reinterpret_cast<double*>(smem_raw + D.pds_off) : nullptr);
-    // XR: the own rows' pressure held in registers for the solve and stored
-    // on every exit (the one-CTA-per-SM kernel: 12.18 -> 11.73 us per
-    // iteration at 64^3; holding the diagonal there too was slower, 14.0 us)
-    constexpr bool XR = NT == 512 && !BATCH;
-    for (int k = threadIdx.x; k < nh; k += NT) hidx[k] = D.halo_idx[h0 + k];
-    for (int k = threadIdx.x; k < nsl; k += NT) lcs[k] = D.lcol[S0 + k];
+    const int q0 = D.rem_ptr[blockIdx.x];
+    const int nr = D.rem_ptr[blockIdx.x + 1] - q0;
+    double* vh = reinterpret_cast<double*>(smem_raw);          // halo_max: z of every column, and one spare
+    double* rh = vh + D.halo_max;                              // rem_max: r, s, inverse diagonal of the remote ones
+    double* sh = rh + D.rem_max;
+    double* dzh = sh + D.rem_max;
+    int* rgi = reinterpret_cast<int*>(dzh + D.rem_max);        // rem_max: their row positions
+    unsigned short* rhp = reinterpret_cast<unsigned short*>(rgi + D.rem_max);   // ... and places in vh
+    // the own rows' diagonal, kept in shared memory for the solve where the
+    // engine sized it so
+    double* pds = NT == 512 && !BATCH && D.pds_off ? reinterpret_cast<double*>(smem_raw + D.pds_off) : nullptr;
+    for (int k = threadIdx.x; k < nr; k += NT) {
+        const int2 e = D.rem[q0 + k];
+        const uint8_t f = D.nflag[e.x];
+        rgi[k] = e.x;
+        rhp[k] = (unsigned short)e.y;
+        dzh[k] = (f & 1) && !(f & 4) ? (g.precond ? 1.0 / D.pdiag[e.x] : 1.0) : 0.0;
+        sh[k] = 0.0;
+    }
     // KS = 1: the coefficients of every warp's first row (the CTA's first
     // NT/32 slices, its leading slots) copied once into shared memory and
     // read from there in every iteration instead of from L2
@@ -1367,38 +1644,79 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
         for (int k = threadIdx.x; k < c0; k += NT) cvs[k] = __ldcg(D.val + S0 + k);
     }
     int phase = 0;
-    const int N = D.N;
-    // parity buffers: r in r/pA, w in q/pB, s in z/dz(+N)... laid out by the engine
-    double* rb[2] = {D.r, D.r + N};
-    double* wb[2] = {D.q, D.q + N};
-    double* sb[2] = {D.pA, D.pB};
-    double* dz = D.z;   // free ? 1/diagonal : 0  (z = r * dz)
 
+    // the own rows (row k of this thread is row0 + k*NT): r, p, s, w and the
+    // reciprocal of the Jacobi diagonal (0 off the free rows) in registers
+    // for the solve.  Rows off the free ones, and the empty rows of a short
+    // warp, have r = dd = 0 and stay 0 without branches.
     double r[RMAX], p[RMAX], s[RMAX], w[RMAX], dd[RMAX];
-    double xr[RMAX];
-    bool fr[RMAX];
-    int row[RMAX], lbase[RMAX], wr[RMAX];
-    int wmax = 0;
+    // Registers bound the kernel (128 at 512 threads).  Past four rows per
+    // thread p and the pressure live in memory: the pressure in shared memory
+    // where that has room (else global; both at the rows' distance NT),
+    // updated once the CTA's partials are on their way, and p in global
+    // memory except from there to the next update.  At three rows the
+    // pressure in shared memory measured faster (56^3: 4.82 us per iteration
+    // against 4.99), at four slower (64^3: 7.45 against 7.16).
+    constexpr bool XM = RMAX == 3 || RMAX > 4, PM = RMAX > 4;
+    double xr[XM ? 1 : RMAX];
+    const int row0 = (s_beg + warp) * 32 + lane;
+    // per row: place of its z in vh (the last, unused one where it is no
+    // column of this CTA), whether other CTAs read it, whether it is free
+    constexpr int PLACE = 0xffff, PUB = 1 << 16, FREE = 1 << 17;
+    int own[RMAX], lbase[RMAX], wr[RMAX];
+    int wmax = 0, nk = 0;        // the warp's widest row and its rows (uniform)
 #pragma unroll
     for (int k = 0; k < RMAX; ++k) {
         const int sl = s_beg + warp + (NT / 32) * k;
-        row[k] = (sl < s_end) ? sl * 32 + lane : -1;
         lbase[k] = 0;
         wr[k] = 0;
+        own[k] = D.halo_max - 1;
         if (sl < s_end) {
+            ++nk;
             lbase[k] = (int)(D.slice_off[sl] - S0) + lane;
             wr[k] = D.slice_w[sl];
             wmax = wr[k] > wmax ? wr[k] : wmax;
+            const int o = D.own[row0 + k * NT];
+            own[k] = (o & PUB) | ((o & PLACE) == PLACE ? D.halo_max - 1 : (o & PLACE));
         }
         r[k] = p[k] = s[k] = w[k] = 0.0;
-        xr[k] = 0.0;
-        dd[k] = 0.0;   // reciprocal of the Jacobi diagonal; 0 off the free rows
-        fr[k] = false;
+        dd[k] = 0.0;
     }
-    // coefficient columns loaded per round (measured: 2 rather than 4 at four
-    // rows per thread takes the 64^3 iteration from 13.0 to 12.2 us)
-    constexpr int CH = (RMAX >= 8) ? 2 : (RMAX >= 4) ? 2 : 8;
+    double* xs = !XM ? nullptr
+               : D.xs_off ? reinterpret_cast<double*>(smem_raw + D.xs_off) + threadIdx.x : D.pres + row0;
+    double* ps = PM ? D.pA + row0 : nullptr;
+    // slots per round (measured at four rows per thread: 2 rather than 4)
+    constexpr int CH = RMAX >= 3 ? 2 : 8;
     static_assert(KT == 0 || KS + KT <= RMAX, "TMEM rows follow the shared-memory rows");
+    // rows past the tensor memory's: their coefficients stream from L2, the
+    // first XW slots of one row requested together (one row's before the
+    // barrier ahead of the products)
+    constexpr int KX = KT > 0 ? RMAX - KS - KT : 0, XW = 16;
+    // The warp's local columns, as byte offsets into vh, two slots to a word:
+    // word j of row k is at lcp[(k * wmax/2 + j) * 32].  Every row of a warp
+    // is padded to the warp's widest (rounded up to CH) with a column whose
+    // coefficient is zero, so the rounds carry no guards.  (A non-finite z in
+    // such a column can only come with a non-finite residual or r.z, which
+    // end the solve in the same iteration.)
+    wmax = (wmax + CH - 1) / CH * CH;
+    const unsigned* lcp;
+    {
+        __shared__ int s_words[NT / 32];
+        if (lane == 0) s_words[warp] = nk * (wmax / 2) * 32;
+        __syncthreads();
+        int o = 0;
+        for (int q = 0; q < warp; ++q) o += s_words[q];
+        unsigned* mine = reinterpret_cast<unsigned*>(smem_raw + D.lcs_off) + o + lane;
+        for (int k = 0; k < nk; ++k) {
+            const unsigned short* src = D.lcol + S0 + lbase[k];
+            const unsigned pad = wr[k] > 0 ? src[0] : 0;
+            for (int j = 0; j < wmax / 2; ++j) {
+                const unsigned lo = 2 * j < wr[k] ? src[64 * j] : pad, hi = 2 * j + 1 < wr[k] ? src[64 * j + 32] : pad;
+                mine[(k * (wmax / 2) + j) * 32] = lo * 8 | hi * 8 << 16;
+            }
+        }
+        lcp = mine;
+    }
     // TMEM rows: row KS+q of this thread starts at column
     // 128*(warp/4) + 2*tm_w*q of lane 32*(warp%4)+lane; slot u of the row is
     // the double in columns 2u, 2u+1.  Every warp runs the same (uniform)
@@ -1418,11 +1736,17 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
         }
         tmem_wait_st();
     }
+    double vx[KX > 0 ? XW : 1];
+    auto extra_load = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < XW; ++u) vx[u] = u < wr[k] ? __ldcg(D.val + S0 + lbase[k] + 32 * u) : 0.0;
+    };
     auto offdiag_all = [&](double* off) {
 #pragma unroll
         for (int k = 0; k < RMAX; ++k) off[k] = 0.0;
-        for (int k0 = 0; k0 < wmax; k0 += CH) {
-            double v[RMAX][CH];
+        const unsigned* lc = lcp;
+        for (int k0 = 0; k0 < wmax; k0 += CH, lc += CH / 2 * 32) {
+            double v[RMAX][CH], x[RMAX][CH];
             uint32_t tv[KT > 0 ? KT : 1][2 * CH];
             if constexpr (KT > 0) {
 #pragma unroll
@@ -1430,13 +1754,23 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
             }
 #pragma unroll
             for (int k = 0; k < RMAX; ++k) {
-                if (k >= KS && k < KS + KT) continue;
+                if (k >= KS && (KT > 0 || k < KS + KT)) continue;
 #pragma unroll
                 for (int u = 0; u < CH; ++u)
                     v[k][u] = (k0 + u < wr[k]) ? (k < KS ? cvs[lbase[k] + 32 * (k0 + u)]
                                                          : __ldcg(D.val + S0 + lbase[k] + 32 * (k0 + u)))
                                                : 0.0;
             }
+#pragma unroll
+            for (int k = 0; k < RMAX - KX; ++k)
+                if (k < nk) {
+#pragma unroll
+                    for (int j = 0; j < CH / 2; ++j) {
+                        const unsigned c = lc[(k * (wmax / 2) + j) * 32];
+                        x[k][2 * j] = *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu));
+                        x[k][2 * j + 1] = *reinterpret_cast<const double*>(smem_raw + (c >> 16));
+                    }
+                }
             if constexpr (KT > 0) {
                 tmem_wait_ld();
 #pragma unroll
@@ -1444,226 +1778,273 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
                     tmem_hold<2 * CH>(tv[q]);
 #pragma unroll
                     for (int u = 0; u < CH; ++u)
-                        v[KS + q][u] = (k0 + u < wr[KS + q])
-                                           ? __hiloint2double(static_cast<int>(tv[q][2 * u + 1]),
-                                                              static_cast<int>(tv[q][2 * u]))
-                                           : 0.0;
+                        v[KS + q][u] = __hiloint2double(static_cast<int>(tv[q][2 * u + 1]), static_cast<int>(tv[q][2 * u]));
                 }
             }
 #pragma unroll
-            for (int k = 0; k < RMAX; ++k)
+            for (int k = 0; k < RMAX - KX; ++k)
+                if (k < nk) {
 #pragma unroll
-                for (int u = 0; u < CH; ++u) {
-                    const double g = (k0 + u < wr[k]) ? vh[lcs[lbase[k] + 32 * (k0 + u)]] : 0.0;
-                    off[k] = fma(v[k][u], g, off[k]);
+                    for (int u = 0; u < CH; ++u) off[k] = fma(v[k][u], x[k][u], off[k]);
+                }
+        }
+        if constexpr (KX > 0) {
+#pragma unroll
+            for (int k = RMAX - KX; k < RMAX; ++k)
+                if (k < nk) {
+                    if (k > RMAX - KX) extra_load(k);
+                    const unsigned* lx = lcp + k * (wmax / 2) * 32;
+#pragma unroll
+                    for (int j = 0; j < XW / 2; ++j)
+                        if (2 * j < wmax) {
+                            const unsigned c = lx[j * 32];
+                            off[k] = fma(vx[2 * j], *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[k]);
+                            off[k] = fma(vx[2 * j + 1], *reinterpret_cast<const double*>(smem_raw + (c >> 16)), off[k]);
+                        }
+                    for (int u = XW; u < wr[k]; ++u) {
+                        const unsigned c = lx[(u >> 1) * 32] >> (16 * (u & 1));
+                        off[k] = fma(__ldcg(D.val + S0 + lbase[k] + 32 * u),
+                                     *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[k]);
+                    }
                 }
         }
     };
+    auto extra_first = [&]() {
+        if constexpr (KX > 0)
+            if (RMAX - KX < nk) extra_load(RMAX - KX);
+    };
 
-    // ---- phase 0a: r0 = b - A x0 (constraints as the reference), dz
-    double off[RMAX];
-    __syncthreads();
-    for (int k0 = threadIdx.x; k0 < nh; k0 += 4 * NT) {
-        double a[4];
+    auto diag = [&](int k) -> double {
+        return pds ? pds[k * NT + threadIdx.x] : (k < nk ? D.pdiag[row0 + k * NT] : 0.0);
+    };
+
+    // exchange of one value per row (exchange number `phase`): the rows that
+    // other CTAs read are stored as records; the first RP remote entries of
+    // this thread are requested with request() and all are waited for and
+    // handed to use(entry, value) by collect()
+    constexpr int RP = RMAX >= 8 ? 2 : RMAX;
+    auto store = [&](const double (&v)[RMAX]) {
+        TagVal* o = D.xw + (size_t)(phase & 1) * D.N;
+        const unsigned long long tg = comm.tag(phase);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u * NT;
-            a[u] = __ldcg(D.pres + (k < nh ? hidx[k] : 0));
+        for (int k = 0; k < RMAX; ++k)
+            if (own[k] & PUB) st_tag(o + row0 + k * NT, v[k], tg);
+    };
+    double xv[RP];
+    unsigned long long xt[RP];
+    auto request = [&](int ph) {
+        const TagVal* o = D.xw + (size_t)(ph & 1) * D.N;
+#pragma unroll
+        for (int u = 0; u < RP; ++u) {
+            const int e = threadIdx.x + u * NT;
+            xt[u] = 0;
+            if (e < nr) ld_tag(o + rgi[e], xv[u], xt[u]);
         }
+    };
+    auto collect = [&](int ph, auto&& use) -> bool {
+        const TagVal* o = D.xw + (size_t)(ph & 1) * D.N;
+        const unsigned long long want = comm.tag(ph);
+        bool ok = true;
+        SpinLimit lim;
+        for (int e0 = threadIdx.x; e0 < nr && ok; e0 += RP * NT) {
+            if (e0 != threadIdx.x) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (k0 + u * NT < nh) vh[k0 + u * NT] = a[u];
-    }
+                for (int u = 0; u < RP; ++u) {
+                    const int e = e0 + u * NT;
+                    xt[u] = 0;
+                    if (e < nr) ld_tag(o + rgi[e], xv[u], xt[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < RP; ++u) {
+                const int e = e0 + u * NT;
+                if (e < nr) {
+                    while (xt[u] != want) {
+                        if (lim.expired(comm.status)) { ok = false; break; }
+                        ld_tag(o + rgi[e], xv[u], xt[u]);
+                    }
+                    use(e, xv[u]);
+                }
+            }
+        }
+        return ok;
+    };
+
+    // ---- phase 0a: r0 = b - A x0 (constraints as the reference); partials:
+    // invalid diagonals, non-finite residuals, (r,r), max|r|
+    double off[RMAX], acc[4] = {0.0, 0.0, 0.0, 0.0}, t[4];
+    for (int k = threadIdx.x; k < nh; k += NT) vh[k] = __ldcg(D.pres + D.halo_idx[h0 + k]);
+    extra_first();
     __syncthreads();
     offdiag_all(off);
-    Acc6 acc{0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int k = 0; k < RMAX; ++k) {
-        const int i = row[k];
-        if (i < 0) continue;
+        if (k >= nk) continue;
+        const int i = row0 + k * NT;
         const uint8_t f = D.nflag[i];
-        const bool active = f & 1;
-        fr[k] = (f & 1) && !(f & 4);
+        const bool active = f & 1, fr = (f & 1) && !(f & 4);
+        if (fr) own[k] |= FREE;
         const double pd = D.pdiag[i];
         const double xi = D.pres[i];
-        if (xs) xs[k * NT + threadIdx.x] = xi;
         if (pds) pds[k * NT + threadIdx.x] = pd;
-        if (XR) xr[k] = xi;
+        if (!XM) xr[XM ? 0 : k] = xi;
+        else if (D.xs_off) xs[k * NT] = xi;
+        if (PM) ps[k * NT] = 0.0;
         const double y = fma(pd, xi, off[k]);
         double ri = active ? D.rhs1[i] - y : 0.0;
-        if (!fr[k]) ri = 0.0;
-        if (fr[k]) {
+        if (!fr) ri = 0.0;
+        if (fr) {
             if (g.precond) {
-                if (!(isfinite(pd) && pd > 1.0e-30)) acc.flag = fmax(acc.flag, 1.0);
+                if (!(isfinite(pd) && pd > 1.0e-30)) acc[0] += 1.0;
                 dd[k] = 1.0 / pd;
             } else {
                 dd[k] = 1.0;
             }
-            if (!isfinite(ri)) acc.flag = fmax(acc.flag, 2.0);
-            acc.c = fma(ri, ri, acc.c);
-            acc.mx = fmax(acc.mx, fabs(ri));
+            if (!isfinite(ri)) acc[1] += 1.0;
+            acc[2] = fma(ri, ri, acc[2]);
+            acc[3] = max_bits(acc[3], fabs(ri));
         }
         r[k] = ri;
-        rb[0][i] = ri;
-        dz[i] = dd[k];
-        sb[0][i] = 0.0;
     }
     // the pressure of the free own rows back to global memory
     auto store_x = [&]() {
-        if (XR) {
-#pragma unroll
-            for (int k = 0; k < RMAX; ++k)
-                if (row[k] >= 0 && fr[k]) D.pres[row[k]] = xr[k];
-            return;
-        }
-        if (!xs) return;
+        if (XM && !D.xs_off) return;
 #pragma unroll
         for (int k = 0; k < RMAX; ++k)
-            if (row[k] >= 0 && fr[k]) D.pres[row[k]] = xs[k * NT + threadIdx.x];
+            if (own[k] & FREE) D.pres[row0 + k * NT] = XM ? xs[k * NT] : xr[XM ? 0 : k];
     };
-    Acc6 t{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce3<NT>(acc, D, g, phase, t)) return;
-    ++phase;
-    const double init = sqrt(t.c);
-    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t.mx); return; }
-    if (cg_converged(g.conv_test, 1.0, t.mx, g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t.mx); return; }
-    if (t.flag >= 2.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
-    if (t.flag >= 1.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
+    store(r);
+    tag_allreduce_publish<NT, false, true>(comm, phase, acc);
+    if (!tag_allreduce_wait<NT, false, true>(comm, phase, t, true, hold, [&] { request(phase); })) return;
+    const double init = sqrt(t[2]);
+    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t[3]); return; }
+    if (cg_converged(g.conv_test, 1.0, t[3], g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t[3]); return; }
+    if (t[1] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
+    if (t[0] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
+    const StopTest stop(g, init);
 
     // ---- phase 0b: z0 = M^-1 r0, w0 = A z0, gamma0 = (r0,z0), delta0 = (z0,w0)
-    __syncthreads();
-    for (int k0 = threadIdx.x; k0 < nh; k0 += 4 * NT) {
-        double a[4], c[4];
+    bool got = collect(phase, [&](int e, double v) {
+        rh[e] = v;
+        vh[rhp[e]] = v * dzh[e];
+    });
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u * NT;
-            const int j = k < nh ? hidx[k] : 0;
-            a[u] = __ldcg(dz + j);
-            c[u] = __ldcg(rb[0] + j);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u * NT;
-            if (k < nh) { dzh[k] = a[u]; vh[k] = c[u] * a[u]; }
-        }
-    }
+    for (int k = 0; k < RMAX; ++k)
+        vh[own[k] & PLACE] = r[k] * dd[k];
+    ++phase;
+    extra_first();
     __syncthreads();
     offdiag_all(off);
-    acc = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
 #pragma unroll
     for (int k = 0; k < RMAX; ++k) {
-        const int i = row[k];
-        if (i < 0) continue;
         const double zi = r[k] * dd[k];
-        w[k] = fr[k] ? fma(pds ? pds[k * NT + threadIdx.x] : D.pdiag[i], zi, off[k]) : 0.0;
-        wb[0][i] = w[k];
-        if (fr[k]) {
-            acc.a = fma(r[k], zi, acc.a);
-            acc.b = fma(zi, w[k], acc.b);
-        }
+        w[k] = (own[k] & FREE) ? fma(diag(k), zi, off[k]) : 0.0;
+        acc[0] = fma(r[k], zi, acc[0]);
+        acc[1] = fma(zi, w[k], acc[1]);
     }
-    t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce3<NT>(acc, D, g, phase, t)) { store_x(); return; }
-    ++phase;
-    double gam = t.a;
+    store(w);
+    tag_allreduce_publish<NT, false, false>(comm, phase, acc);
+    if (!tag_allreduce_wait<NT, false, false>(comm, phase, t, got, hold, [&] { request(phase); })) return;
+    double gam = t[0];
     if (gam <= 1.0e-300 || !isfinite(gam)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, 0, R_PCG_RZ0); return; }
-    double den = t.b;
-    double beta = 0.0, fin = init, rel = 1.0, mx = 0.0, alpha = 0.0;
+    double den = t[1], alpha = gam / den, beta = 0.0, rr = init * init, mx = 0.0;
     int it = 0, conv = 0;
+    int wph = phase;             // exchange that carries the w to collect
+    // max|r| where the iterations carry none: an all-reduce of its own
+    auto final_max = [&]() {
+        double m[4] = {0.0, 0.0, 0.0, 0.0}, o[4];
+#pragma unroll
+        for (int k = 0; k < RMAX; ++k)
+            if (own[k] & FREE) m[3] = max_bits(m[3], fabs(r[k]));
+        ++phase;
+        tag_allreduce_publish<NT, false, true>(comm, phase, m);
+        const bool ok = tag_allreduce_wait<NT, false, true>(comm, phase, o, true, hold, [] {});
+        mx = o[3];
+        return ok;
+    };
     for (it = 1; it <= g.max_iter; ++it) {
         if (fabs(den) <= 1.0e-300 || !isfinite(den)) { store_x(); if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_PAP); return; }
-        alpha = gam / den;
-        const int po = (it - 1) & 1, pn = it & 1;
-        // stage z_it of the halo: s = w_o + beta*s_o, r = r_o - alpha*s, z = r / dz
-        // (SU halo nodes per thread per round, all their loads issued first);
-        // the all-reduce above ended with a barrier, so vh is free to write
-        {
-            constexpr int SU = 4;
-            const double* so = sb[po];
-            const double* wo = wb[po];
-            const double* ro = rb[po];
-            for (int k0 = threadIdx.x; k0 < nh; k0 += SU * NT) {
-                double a[SU], c[SU], e[SU];
-#pragma unroll
-                for (int u = 0; u < SU; ++u) {
-                    const int k = k0 + u * NT;
-                    const int j = k < nh ? hidx[k] : 0;
-                    a[u] = __ldcg(so + j);
-                    c[u] = __ldcg(wo + j);
-                    e[u] = __ldcg(ro + j);
-                }
-#pragma unroll
-                for (int u = 0; u < SU; ++u) {
-                    const int k = k0 + u * NT;
-                    if (k < nh) {
-                        const double sj = fma(beta, a[u], c[u]);
-                        const double rj = fma(-alpha, sj, e[u]);
-                        vh[k] = rj * dzh[k];
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        // own rows: p = z_o + beta*p, s = w + beta*s, x += alpha*p, r -= alpha*s
+        // z_it of the halo: s = w + beta*s, r -= alpha*s, z = r * dz, for the
+        // remote entries from their owners' w and for the own rows
+        got = collect(wph, [&](int e, double v) {
+            const double sj = fma(beta, sh[e], v);
+            const double rj = fma(-alpha, sj, rh[e]);
+            sh[e] = sj;
+            rh[e] = rj;
+            vh[rhp[e]] = rj * dzh[e];
+        });
+        // own rows: p = z_o + beta*p, s = w + beta*s, r -= alpha*s
 #pragma unroll
         for (int k = 0; k < RMAX; ++k) {
-            const int i = row[k];
-            if (i < 0) continue;
-            const double zo = r[k] * dd[k];
-            p[k] = fr[k] ? fma(beta, p[k], zo) : 0.0;
+            p[k] = fma(beta, p[k], r[k] * dd[k]);
+            if (PM && (own[k] & FREE)) ps[k * NT] = p[k];
             s[k] = fma(beta, s[k], w[k]);
-            if (fr[k]) {
-                if (XR) xr[k] = fma(alpha, p[k], xr[k]);
-                else if (xs) xs[k * NT + threadIdx.x] = fma(alpha, p[k], xs[k * NT + threadIdx.x]);
-                else D.pres[i] = fma(alpha, p[k], D.pres[i]);
-            }
             r[k] = fma(-alpha, s[k], r[k]);
-            rb[pn][i] = r[k];
-            sb[pn][i] = s[k];
-        }
-        offdiag_all(off);
-        Acc6 a6{0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < RMAX; ++k) {
-            const int i = row[k];
-            if (i < 0) continue;
-            const double zi = r[k] * dd[k];
-            w[k] = fr[k] ? fma(pds ? pds[k * NT + threadIdx.x] : D.pdiag[i], zi, off[k]) : 0.0;
-            wb[pn][i] = w[k];
-            if (fr[k]) {
-                if (!isfinite(r[k])) a6.flag = 1.0;
-                a6.a = fma(r[k], zi, a6.a);
-                a6.b = fma(zi, w[k], a6.b);
-                a6.c = fma(r[k], r[k], a6.c);
-                a6.mx = fmax(a6.mx, fabs(r[k]));
-            }
-        }
-        t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-        if constexpr (NT == 256) {
-            // four values: a non-finite residual is carried as an infinite
-            // max |r| (measured faster for the small-mesh kernel only)
-            double a4[4] = {a6.a, a6.b, a6.c, a6.flag > 0.0 ? __longlong_as_double(0x7ff0000000000000LL) : a6.mx};
-            double o4[4];
-            if (!grid_allreduce_v<4, 3, NT>(a4, D, g, phase, o4)) { store_x(); return; }
-            t = Acc6{o4[0], o4[1], o4[2], o4[3], isinf(o4[3]) ? 1.0 : 0.0};
-        } else {
-            if (!grid_allreduce3<NT>(a6, D, g, phase, t)) { store_x(); return; }
+            vh[own[k] & PLACE] = r[k] * dd[k];
         }
         ++phase;
-        fin = sqrt(t.c);
-        mx = t.mx;
-        rel = fin / init;
-        if (cg_converged(g.conv_test, rel, mx, g.rel_tol, g.abs_tol)) { conv = 1; break; }
-        if (t.flag > 0.0) { store_x(); if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
-        const double gn = t.a;
-        if (gn <= 1.0e-300 || !isfinite(gn)) { store_x(); if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
+        extra_first();
+        __syncthreads();
+        offdiag_all(off);
+        acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
+#pragma unroll
+        for (int k = 0; k < RMAX; ++k) {
+            const double zi = r[k] * dd[k];
+            w[k] = (own[k] & FREE) ? fma(diag(k), zi, off[k]) : 0.0;
+            acc[0] = fma(r[k], zi, acc[0]);
+            acc[1] = fma(zi, w[k], acc[1]);
+            acc[2] = fma(r[k], r[k], acc[2]);
+            if (stop.needs_max()) acc[3] = max_bits(acc[3], fabs(r[k]));
+        }
+        store(w);
+        wph = phase;
+        // x after the CTA's partials are on their way
+        auto update_x = [&]() {
+#pragma unroll
+            for (int k = 0; k < RMAX; ++k) {
+                if (!XM) xr[XM ? 0 : k] = fma(alpha, p[k], xr[XM ? 0 : k]);
+                else if (own[k] & FREE) {
+                    if (PM) p[k] = ps[k * NT];
+                    xs[k * NT] = fma(alpha, p[k], xs[k * NT]);
+                }
+            }
+        };
+        if (!stop.needs_max()) {
+            tag_allreduce_publish<NT, false, false>(comm, phase, acc);
+            update_x();
+            got = tag_allreduce_wait<NT, false, false>(comm, phase, t, got, hold, [&] { request(phase); });
+        } else {
+            tag_allreduce_publish<NT, false, true>(comm, phase, acc);
+            update_x();
+            got = tag_allreduce_wait<NT, false, true>(comm, phase, t, got, hold, [&] { request(phase); });
+        }
+        if (!got) { store_x(); return; }
+        rr = t[2];
+        mx = t[3];
+        const double gn = t[0];
+        // (p, Ap) of the next direction: delta - beta*gn/alpha, where
+        // gn/alpha = beta*den; the rare exits beside the two divisions
         beta = gn / gam;
-        den = t.b - beta * gn / alpha;
+        den = fma(-beta * beta, den, t[1]);
+        alpha = gn / den;
         gam = gn;
+        if (!stop.clear(rr) || gn <= 1.0e-300 || !isfinite(gn)) {
+            if (!stop.needs_max() && !final_max()) { store_x(); return; }
+            if (stop.exact(rr, mx)) { conv = 1; break; }
+            // a non-finite residual shows as a non-finite max |r|
+            if (!isfinite(mx)) { store_x(); if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
+            if (gn <= 1.0e-300 || !isfinite(gn)) { store_x(); if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
+            // rounding put (r,r) inside the margin: on, after one more
+            // all-reduce that keeps the records' two buffers apart (the next
+            // w may not overwrite the last one before every CTA has read it)
+            if (!stop.needs_max() && !final_max()) { store_x(); return; }
+        }
     }
+    if (!conv && !stop.needs_max() && !final_max()) { store_x(); return; }
     store_x();
     if (it > g.max_iter) it = g.max_iter;
-    cg_finish(D, g, it, conv, init, fin, rel, mx);
+    cg_finish(D, g, it, conv, init, sqrt(rr), sqrt(rr) / init, mx);
     if (!conv && b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 2, ST_PCG, it, R_PCG_MAXIT);
 }
 
@@ -1675,8 +2056,10 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm)
 template <int RMAX, bool BATCH, int NT, int KS = 0, int KT = 0>
 __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
 {
+    unsigned long long epoch;
+    if (!tag_begin<BATCH>(D, epoch)) return;
     if constexpr (KT == 0) {
-        pcg64c_body<RMAX, BATCH, NT, KS, 0>(D, 0u);
+        pcg64c_body<RMAX, BATCH, NT, KS, 0>(D, 0u, epoch);
     } else {
         static_assert(NT == 512 && !BATCH, "TMEM rows: one CTA per SM, single system");
         __shared__ uint32_t s_tm;
@@ -1686,12 +2069,13 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
         __syncthreads();
         tmem_fence_after_sync();
         const uint32_t tm = s_tm;
-        pcg64c_body<RMAX, BATCH, NT, KS, KT>(D, tm);
+        pcg64c_body<RMAX, BATCH, NT, KS, KT>(D, tm, epoch);
         tmem_fence_before_sync();
         __syncthreads();
         tmem_fence_after_sync();
         if (w0) tmem_free_all(tm);
     }
+    tag_end<BATCH>(D, epoch);
 }
 
 template <int RMAX>
@@ -2007,7 +2391,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg64d(PcgDev D, CoarseDev C)
 constexpr int RU_STALL = 256;   // iterations without a correction before one is forced
 
 template <int RMAX, bool BATCH, int NT>
-__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
+__device__ __forceinline__ void pcg32m_body(const PcgDev& D, unsigned long long epoch)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SegView g = seg_view<BATCH>(D);
@@ -2032,7 +2416,17 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
         lcs[k] = D.lcol[S0 + k];
         val32s[k] = D.val32[S0 + k];
     }
+    const TagComm comm = tag_comm(D, g, epoch);
+    PollHold hold;
     int phase = 0;
+    // three sums and a maximum; the vectors go by plain stores, made visible
+    // with the record
+    auto allreduce = [&](const double (&v)[4], double (&o)[4]) {
+        tag_allreduce_publish<NT, true, true>(comm, phase, v);
+        const bool ok = tag_allreduce_wait<NT, true, true>(comm, phase, o, true, hold, [] {});
+        ++phase;
+        return ok;
+    };
     const int N = D.N;
     float* rb[2] = {D.r32, D.r32 + N};
     float* wb[2] = {D.w32, D.w32 + N};
@@ -2107,8 +2501,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
         }
         __syncthreads();
     };
-    // true residual of the own rows into r[], rb[buf]; returns partials
-    auto true_residual = [&](int buf, Acc6& acc) {
+    // true residual of the own rows into r[], rb[buf]; partials: non-finite
+    // entries, (r,r), max|r|
+    auto true_residual = [&](int buf, double (&acc)[4]) {
         stage64(D.pres);
         double off[RMAX];
         offdiag64(off);
@@ -2120,9 +2515,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
             double ri = (D.nflag[i] & 1) ? D.rhs1[i] - y : 0.0;
             if (!fr[k]) ri = 0.0;
             if (fr[k]) {
-                if (!isfinite(ri)) acc.flag = fmax(acc.flag, 2.0);
-                acc.c = fma(ri, ri, acc.c);
-                acc.mx = fmax(acc.mx, fabs(ri));
+                if (!isfinite(ri)) acc[1] += 1.0;
+                acc[2] = fma(ri, ri, acc[2]);
+                acc[3] = max_bits(acc[3], fabs(ri));
             }
             r[k] = (float)ri;
             rb[buf][i] = r[k];
@@ -2133,7 +2528,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
     // zero_p, which restarts the direction); partials of r.z, z.w, z.s, p.w
     // and p.s, from which the step length of the next direction
     // (z + beta p).A(z + beta p) follows directly
-    auto refresh_ws = [&](int buf, bool zero_p, Acc8& acc) {
+    auto refresh_ws = [&](int buf, bool zero_p, double (&acc)[5]) {
         __syncthreads();
         for (int k0 = threadIdx.x; k0 < nh; k0 += 4 * NT) {
             float a[4], c[4];
@@ -2167,17 +2562,17 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
             sb[buf][i] = sv[k];
             if (fr[k]) {
                 const double zd = zi, pv = p[k];
-                acc.a = fma((double)r[k], zd, acc.a);
-                acc.b = fma(zd, (double)w[k], acc.b);
-                acc.c = fma(zd, (double)sv[k], acc.c);
-                acc.d = fma(pv, (double)w[k], acc.d);
-                acc.e = fma(pv, (double)sv[k], acc.e);
+                acc[0] = fma((double)r[k], zd, acc[0]);
+                acc[1] = fma(zd, (double)w[k], acc[1]);
+                acc[2] = fma(zd, (double)sv[k], acc[2]);
+                acc[3] = fma(pv, (double)w[k], acc[3]);
+                acc[4] = fma(pv, (double)sv[k], acc[4]);
             }
         }
     };
 
     // ---- phase 0a: FP64 r0 = b - A x0, its norm, dz
-    Acc6 acc{0.0, 0.0, 0.0, 0.0, 0.0};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0}, t[4];   // [0]: invalid diagonals
 #pragma unroll
     for (int k = 0; k < RMAX; ++k) {
         const int i = row[k];
@@ -2186,34 +2581,38 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
         fr[k] = (f & 1) && !(f & 4);
         const double pd = D.pdiag[i];
         if (fr[k]) {
-            if (g.precond && !(isfinite(pd) && pd > 1.0e-30)) acc.flag = fmax(acc.flag, 1.0);
+            if (g.precond && !(isfinite(pd) && pd > 1.0e-30)) acc[0] += 1.0;
             dd[k] = g.precond ? (float)(1.0 / pd) : 1.0f;
         }
         dz[i] = dd[k];
         sb[0][i] = 0.0f;
     }
     true_residual(0, acc);
-    Acc6 t{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce3<NT>(acc, D, g, phase, t)) return;
-    ++phase;
-    const double init = sqrt(t.c);
-    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t.mx); return; }
-    if (cg_converged(g.conv_test, 1.0, t.mx, g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t.mx); return; }
-    if (t.flag >= 2.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
-    if (t.flag >= 1.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
-    double rr_last = t.c;
+    if (!allreduce(acc, t)) return;
+    const double init = sqrt(t[2]);
+    if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t[3]); return; }
+    if (cg_converged(g.conv_test, 1.0, t[3], g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t[3]); return; }
+    if (t[1] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, 0, R_PCG_RESID); return; }
+    if (t[0] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 1, ST_PCG, 0, R_PCG_DIAG); return; }
+    double rr_last = t[2];
 
     // ---- phase 0b: z0, w0 = A z0 (p = 0, s = 0)
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += NT) dzh[k] = __ldcg(dz + hidx[k]);
-    Acc8 a8{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    // the five sums of a refresh, in two all-reduces
+    auto allreduce5 = [&](const double (&v)[5], double (&o)[5]) {
+        const double v0[4] = {v[0], v[1], v[2], 0.0}, v1[4] = {v[3], v[4], 0.0, 0.0};
+        double o0[4], o1[4];
+        if (!allreduce(v0, o0) || !allreduce(v1, o1)) return false;
+        o[0] = o0[0]; o[1] = o0[1]; o[2] = o0[2]; o[3] = o1[0]; o[4] = o1[1];
+        return true;
+    };
+    double a8[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, t8[5];
     refresh_ws(0, true, a8);
-    Acc8 t8{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!grid_allreduce5<NT>(a8, D, g, phase, t8)) return;
-    ++phase;
-    double gam = t8.a;
+    if (!allreduce5(a8, t8)) return;
+    double gam = t8[0];
     if (gam <= 1.0e-300 || !isfinite(gam)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, 0, R_PCG_RZ0); return; }
-    double den = t8.b;
+    double den = t8[1];
     double beta = 0.0, fin = init, rel = 1.0, mx = 0.0, alpha = 0.0;
     int it = 0, conv = 0, outer = 0, last_fix = 0;
     for (it = 1; it <= g.max_iter; ++it) {
@@ -2262,7 +2661,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
         }
         float off[RMAX];
         offdiag32(vz, off);
-        Acc6 a6{0.0, 0.0, 0.0, 0.0, 0.0};
+        double a6[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
         for (int k = 0; k < RMAX; ++k) {
             const int i = row[k];
@@ -2271,62 +2670,64 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
             w[k] = fr[k] ? fmaf((float)D.pdiag[i], zi, off[k]) : 0.0f;
             wb[pn][i] = w[k];
             if (fr[k]) {
-                if (!isfinite(r[k])) a6.flag = 1.0;
-                a6.a = fma((double)r[k], (double)zi, a6.a);
-                a6.b = fma((double)zi, (double)w[k], a6.b);
-                a6.c = fma((double)r[k], (double)r[k], a6.c);
-                a6.mx = fmax(a6.mx, fabs((double)r[k]));
+                a6[0] = fma((double)r[k], (double)zi, a6[0]);
+                a6[1] = fma((double)zi, (double)w[k], a6[1]);
+                a6[2] = fma((double)r[k], (double)r[k], a6[2]);
+                a6[3] = max_bits(a6[3], fabs((double)r[k]));
             }
         }
-        t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-        if (!grid_allreduce3<NT>(a6, D, g, phase, t)) return;
-        ++phase;
-        if (t.flag > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
-        fin = sqrt(t.c);
-        mx = t.mx;
+        if (!allreduce(a6, t)) return;
+        if (!isfinite(t[3])) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
+        fin = sqrt(t[2]);
+        mx = t[3];
         rel = fin / init;
         const bool candidate = cg_converged(g.conv_test, rel, mx, g.rel_tol, g.abs_tol);
-        if (candidate || t.c <= D.inner_tol * D.inner_tol * rr_last || it - last_fix >= RU_STALL) {
+        if (candidate || t[2] <= D.inner_tol * D.inner_tol * rr_last || it - last_fix >= RU_STALL) {
             // residual replacement from the FP64 coefficients and pressure
-            Acc6 u1{0.0, 0.0, 0.0, 0.0, 0.0};
+            double u1[4] = {0.0, 0.0, 0.0, 0.0};
             true_residual(pn, u1);
-            t = Acc6{0.0, 0.0, 0.0, 0.0, 0.0};
-            if (!grid_allreduce3<NT>(u1, D, g, phase, t)) return;
-            ++phase;
+            if (!allreduce(u1, t)) return;
             ++outer;
             last_fix = it;
-            if (t.flag > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
-            fin = sqrt(t.c);
-            mx = t.mx;
+            if (t[1] > 0.0) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 4, ST_PCG, it, R_PCG_RESID); return; }
+            fin = sqrt(t[2]);
+            mx = t[3];
             rel = fin / init;
             // no progress of the true residual since the last correction:
             // the FP32 recurrences have lost the Krylov relations, restart
-            const bool restart = t.c >= rr_last;
-            rr_last = t.c;
+            const bool restart = t[2] >= rr_last;
+            rr_last = t[2];
             if (cg_converged(g.conv_test, rel, mx, g.rel_tol, g.abs_tol)) { conv = 1; break; }
-            Acc8 u2{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            double u2[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
             refresh_ws(pn, restart, u2);
-            t8 = Acc8{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            if (!grid_allreduce5<NT>(u2, D, g, phase, t8)) return;
-            ++phase;
-            const double gn = t8.a;
+            if (!allreduce5(u2, t8)) return;
+            const double gn = t8[0];
             if (gn <= 1.0e-300 || !isfinite(gn)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
             // next direction z + beta p with its curvature computed, not recurred
             beta = restart ? 0.0 : gn / gam;
-            den = t8.b + beta * (t8.c + t8.d) + beta * beta * t8.e;
+            den = t8[1] + beta * (t8[2] + t8[3]) + beta * beta * t8[4];
             gam = gn;
             continue;
         }
-        const double gn = t.a;
+        const double gn = t[0];
         if (gn <= 1.0e-300 || !isfinite(gn)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, it, R_PCG_RZ); return; }
         beta = gn / gam;
-        den = t.b - beta * gn / alpha;
+        den = t[1] - beta * gn / alpha;
         gam = gn;
     }
     if (it > g.max_iter) it = g.max_iter;
     cg_finish(D, g, it, conv, init, fin, rel, mx);
     if (b == 0 && threadIdx.x == 0) seg_out(D, g)->outer = outer;
     if (!conv && b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 2, ST_PCG, it, R_PCG_MAXIT);
+}
+
+template <int RMAX, bool BATCH, int NT>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg32m(PcgDev D)
+{
+    unsigned long long epoch;
+    if (!tag_begin<BATCH>(D, epoch)) return;
+    pcg32m_body<RMAX, BATCH, NT>(D, epoch);
+    tag_end<BATCH>(D, epoch);
 }
 
 // ------------------------------------------------- two-level set-up kernels
@@ -2499,17 +2900,22 @@ cbs3d_status selftest_wait_timeout(int device, int* observed)
 }
 
 namespace {
-// Back-to-back grid all-reduces of the single-reduction kernel's kind (five
-// values per CTA, 512-thread CTAs, one per SM), each depending on the last.
+// Back-to-back grid all-reduces of the single-reduction kernel's kind (three
+// sums per CTA, 512-thread CTAs, one per SM), each depending on the last.
 __global__ void __launch_bounds__(512, 1) k_allreduce_probe(PcgDev D, int iters, double* out)
 {
-    const SegView g = seg_view<false>(D);
-    Acc6 t{0.0, 0.0, 0.0, 0.0, 0.0};
+    unsigned long long epoch;
+    if (!tag_begin<false>(D, epoch)) return;
+    const TagComm comm = tag_comm(D, seg_view<false>(D), epoch);
+    PollHold hold;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
     for (int i = 0; i < iters; ++i) {
-        Acc6 v{1.0 + t.a * 1.0e-300, (double)blockIdx.x, 0.0, 0.0, (double)threadIdx.x};
-        if (!grid_allreduce3<512>(v, D, g, i, t)) return;
+        const double v[4] = {1.0 + t[0] * 1.0e-300, (double)blockIdx.x, (double)threadIdx.x, 0.0};
+        tag_allreduce_publish<512, false, false>(comm, i, v);
+        if (!tag_allreduce_wait<512, false, false>(comm, i, t, true, hold, [] {})) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = t.a;
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = t[0];
+    tag_end<false>(D, epoch);
 }
 }  // namespace
 
@@ -2524,8 +2930,12 @@ cbs3d_status allreduce_probe(int device, int iters, double* us)
     if (per < 1) return CBS3D_CUDA_ERROR;
     PcgDev D{};
     D.nslices = sms;
-    D.part = dalloc<double>(static_cast<size_t>(sms) * 16);
-    D.bar = dalloc<unsigned>(4);
+    const size_t nrec = static_cast<size_t>(sms) * 2 * REC_STRIDE;
+    const unsigned long long one = 1;
+    D.rec = dalloc<TagVal>(nrec);
+    D.epoch = dalloc<unsigned long long>(1);
+    CUDA_OK(cudaMemset(D.rec, 0, nrec * sizeof(TagVal)));
+    CUDA_OK(cudaMemcpy(D.epoch, &one, sizeof one, cudaMemcpyHostToDevice));
     D.status = dalloc<DevStatus>(1);
     double* out = dalloc<double>(1);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -2534,7 +2944,6 @@ cbs3d_status allreduce_probe(int device, int iters, double* us)
     CUDA_OK(cudaEventCreate(&e0));
     CUDA_OK(cudaEventCreate(&e1));
     for (int rep = 0; rep < 2 && rc == CBS3D_OK; ++rep) {   // the first launch warms up
-        CUDA_OK(cudaMemset(D.bar, 0, 4 * sizeof(unsigned)));
         CUDA_OK(cudaMemset(D.status, 0, sizeof(DevStatus)));
         void* args[] = {&D, &iters, &out};
         CUDA_OK(cudaEventRecord(e0));
@@ -2549,8 +2958,8 @@ cbs3d_status allreduce_probe(int device, int iters, double* us)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFree(D.part);
-    cudaFree(D.bar);
+    cudaFree(D.rec);
+    cudaFree(D.epoch);
     cudaFree(D.status);
     cudaFree(out);
     if (rc == CBS3D_OK) *us = 1.0e3 * ms / iters;
@@ -2674,15 +3083,66 @@ long long gather_wavefronts(const unsigned short* lc, const long long* slice_off
     return w;
 }
 
+// Remote halo entries and own rows' places of the single-reduction kernel,
+// built CTA by CTA from its halo's columns in order of their place.
+struct RemoteLists {
+    std::vector<int> ptr{0}, own;
+    std::vector<int2> rem;
+    int most = 0;
+    explicit RemoteLists(size_t rows) : own(rows, 0xffff) {}
+    // rows [r0, r1) belong to the CTA; cols[place] = row position
+    void add_cta(int r0, int r1, const std::vector<int>& cols)
+    {
+        const size_t first = rem.size();
+        for (size_t e = 0; e < cols.size(); ++e) {
+            const int c = cols[e], place = static_cast<int>(e);
+            int& o = own[static_cast<size_t>(c)];
+            if (c >= r0 && c < r1) {
+                o = (o & ~0xffff) | place;
+            } else {
+                o |= 1 << 16;
+                rem.push_back(make_int2(c, place));
+            }
+        }
+        // by row: a warp's requests touch neighbouring records
+        std::sort(rem.begin() + static_cast<std::ptrdiff_t>(first), rem.end(), [](const int2& a, const int2& b) { return a.x < b.x; });
+        ptr.push_back(static_cast<int>(rem.size()));
+        most = std::max(most, static_cast<int>(rem.size() - first));
+    }
+};
+
+// k_pcg64c's dynamic shared memory: the halo's z, the remote entries (r, s,
+// inverse diagonal, row, place), then the local columns at lcs_off
+size_t cgcg_lcs_off(int hmax, int rem_max)
+{
+    return (static_cast<size_t>(hmax) * 8 + static_cast<size_t>(rem_max) * 30 + 15) & ~static_cast<size_t>(15);
+}
+// bytes of local columns of a CTA's slices [sb, se): every warp's rows padded
+// to its widest slice, rounded up to `ch` slots
+size_t cgcg_lcs_bytes(const int* slice_w, int sb, int se, int nwarps, int ch)
+{
+    size_t n = 0;
+    for (int w = 0; w < nwarps && sb + w < se; ++w) {
+        int m = 0, rows = 0;
+        for (int q = sb + w; q < se; q += nwarps, ++rows) m = std::max(m, slice_w[q]);
+        n += static_cast<size_t>(rows) * ((m + ch - 1) / ch * ch) * 64;
+    }
+    return n;
+}
+// slots per round of k_pcg64c at `rmax` rows per thread, and the largest halo
+// whose byte offsets fit 16 bits
+constexpr int cgcg_round(int rmax) { return rmax >= 3 ? 2 : 8; }
+constexpr int CGCG_HALO_MAX = 8190;
+
 // Instantiations of the single-reduction kernels by rows per thread, batch
 // mode and CTA size.
-template <bool BATCH, int NT, int KS = 0>
-const void* fn_cgcg(int rmax)
+template <int NT>
+const void* fn_cgcg_batch(int rmax)
 {
-    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, BATCH, NT, KS>)
-         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, BATCH, NT, KS>)
-         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, BATCH, NT, KS>)
-                     : reinterpret_cast<const void*>(k_pcg64c<8, BATCH, NT, KS>);
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, true, NT>)
+         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, true, NT>)
+         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, true, NT>)
+                     : reinterpret_cast<const void*>(k_pcg64c<8, true, NT>);
 }
 template <bool BATCH, int NT>
 const void* fn_mixed(int rmax)
@@ -2699,26 +3159,31 @@ const void* fn_twolevel(int rmax)
          : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64d<4>)
                      : reinterpret_cast<const void*>(k_pcg64d<8>);
 }
-// rows per thread read from tensor memory by the one-CTA-per-SM kernel with
-// its first row in shared memory (0: that kernel has no such form)
-int cgcg_tmem_rows(int rmax) { return rmax == 2 ? 1 : rmax == 4 ? 3 : rmax == 8 ? 4 : 0; }
-const void* fn_cgcg_single(int rmax, int nt, int ks = 0, bool tmem = false)
+// The single-case kernel by rows per thread: kt > 0 with that many rows'
+// coefficients in tensor memory (every row up to four per thread, else the
+// first four), ks = 1 with the first row's in shared memory ahead of them,
+// kt = 0 with all of them streamed from L2.
+const void* fn_cgcg_single(int rmax, int ks, int kt)
 {
-    // every row of the thread in tensor memory (no shared-memory copy); at
-    // eight rows the first four, the rest from L2
-    if (!ks && tmem && nt == 512)
-        return rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2>)
-             : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 0, 4>)
-                         : reinterpret_cast<const void*>(k_pcg64c<8, false, 512, 0, 4>);
-    if (ks && tmem && nt == 512) {
+    if (ks && kt)
         return rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 1, 1>)
-             : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 1, 3>)
-                         : reinterpret_cast<const void*>(k_pcg64c<8, false, 512, 1, 4>);
-    }
-    if (ks) return nt == 256 ? fn_cgcg<false, 256, 1>(rmax) : fn_cgcg<false, 512, 1>(rmax);
-    return nt == 256 ? fn_cgcg<false, 256>(rmax) : fn_cgcg<false, 512>(rmax);
+                         : reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 1, 3>);
+    if (kt)
+        return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 1>)
+             : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2>)
+             : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, false, 512, 0, 3>)
+             : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 0, 4>)
+             : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512, 0, 4>)
+             : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512, 0, 4>)
+                         : reinterpret_cast<const void*>(k_pcg64c<8, false, 512, 0, 4>);
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512>)
+         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512>)
+         : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, false, 512>)
+         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512>)
+         : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512>)
+         : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512>)
+                     : reinterpret_cast<const void*>(k_pcg64c<8, false, 512>);
 }
-const void* fn_mixed_single(int rmax, int nt) { return nt == 256 ? fn_mixed<false, 256>(rmax) : fn_mixed<false, 512>(rmax); }
 
 // The batch runs 256-thread CTAs, two per SM: its instances are small and
 // many, and more, smaller CTAs spread them better.
@@ -2899,25 +3364,27 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     rmax = 0;
     variant = 1;
     nblocks = grid_for(reinterpret_cast<const void*>(k_pcg64<false>));
-    const int rm[4] = {1, 2, 4, 8};
     if (kernel_choice == 0 || kernel_choice == 3 || kernel_choice == 4 || kernel_choice == 10 || kernel_choice == 11) {
         const void* hc3[4] = {reinterpret_cast<const void*>(k_pcg64h<1>), reinterpret_cast<const void*>(k_pcg64h<2>),
                               reinterpret_cast<const void*>(k_pcg64h<4>), reinterpret_cast<const void*>(k_pcg64h<8>)};
         const int want = kernel_choice == 3 ? 3 : 4;
-        // CTA size of the single-reduction kernel: one 512-thread CTA per SM
-        // once every warp of such a grid has rows (fewer partials per
-        // all-reduce), two 256-thread CTAs per SM below that
-        const int nt = (want == 4 && nslices < 16 * sms) ? 256 : 512;
-        const int nwarps = nt / 32;
-        for (int c = 0; c < 4 && variant == 1; ++c) {
-            const void* fn = want == 4 ? fn_cgcg_single(rm[c], nt) : hc3[c];
+        const int nt = PCG_THREADS, nwarps = nt / 32;
+        // rows per thread: the mixed and the two-level kernel, which share the
+        // single-reduction kernel's partition, have 1, 2, 4 and 8; that one
+        // itself up to six (beyond, the global-vector kernel is as fast:
+        // 76^3 22.0 us per iteration against 25.4 with eight rows)
+        const int pow2[4] = {1, 2, 4, 8}, upto6[6] = {1, 2, 3, 4, 5, 6};
+        const bool few = want == 3 || mixed || two_level;
+        for (int c = 0; c < (few ? 4 : 6) && variant == 1; ++c) {
+            const int rr = few ? pow2[c] : upto6[c];
+            const void* fn = want == 4 ? fn_cgcg_single(rr, 0, 0) : hc3[c];
             int per_sm = 0;
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, 0));
-            int g = sms * (per_sm < 2 ? per_sm : 2);
+            int g = want == 4 ? sms : sms * (per_sm < 2 ? per_sm : 2);
             if (blocks_override > 0 && blocks_override < g) g = blocks_override;
             if (g > nslices) g = nslices > 0 ? nslices : 1;
             const int per_cta = (nslices + g - 1) / g;
-            if ((per_cta + nwarps - 1) / nwarps > rm[c]) continue;
+            if ((per_cta + nwarps - 1) / nwarps > rr) continue;
             // halo of every CTA: distinct columns of its slot range
             std::vector<int> hptr(static_cast<size_t>(g) + 1, 0), hidx;
             std::vector<unsigned short> lcol(static_cast<size_t>(nslots), 0);
@@ -2925,6 +3392,8 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             long long smax = 0;
             bool fits = true;
             std::vector<int> cols, hpos, hcols;
+            RemoteLists remote(static_cast<size_t>(NP));
+            size_t lcsb = 0;
             for (int bb = 0; bb < g && fits; ++bb) {
                 const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
                 const int se = static_cast<int>(static_cast<long long>(bb + 1) * nslices / g);
@@ -2947,128 +3416,85 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 hptr[static_cast<size_t>(bb) + 1] = static_cast<int>(hidx.size());
                 hmax = std::max(hmax, static_cast<int>(cols.size()));
                 smax = std::max(smax, a1 - a0);
+                remote.add_cta(sb * 32, se * 32, hcols);
+                lcsb = std::max(lcsb, cgcg_lcs_bytes(P.slice_w.data(), sb, se, nwarps, cgcg_round(rr)));
             }
-            if (!fits) continue;
-            const size_t smem = static_cast<size_t>(hmax) * (want == 4 ? 20 : 12) + static_cast<size_t>(smax) * 2 + 16;
-            if (smem > 200 * 1024) continue;
+            if (!fits || (want == 4 && hmax > CGCG_HALO_MAX)) continue;
+            if (want == 4) ++hmax;   // the spare place
+            const size_t smem = want == 4 ? cgcg_lcs_off(hmax, remote.most) + lcsb
+                                          : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
+            if (smem > (want == 4 ? 220 : 200) * 1024) continue;
             CUDA_OK(raise_smem_limit(fn, smem));
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, smem));
             if (per_sm * sms < g) continue;
             variant = want;
             nthreads = nt;
-            rmax = rm[c];
+            rmax = rr;
             nblocks = g;
             halo_smem = smem;
-            // the CG-CG kernel's own rows (pressure, diagonal) in shared
-            // memory: measured faster for the two-CTAs-per-SM kernel of small
-            // meshes (5.2 instead of 5.4 us per iteration at 16^3) and slower
-            // for the one-CTA kernel of large ones (13.4 instead of 13.1 us at
-            // 64^3, where those rows already hit in L1 and a larger shared-
-            // memory carve-out leaves less L1 for the rest)
             cgcg_smem = smem;
-            cgcg_xs_off = 0;
-            if (want == 4 && nt == 256) {
-                const size_t off = (smem + 15) & ~static_cast<size_t>(15);
-                const size_t with = off + static_cast<size_t>(rm[c]) * nt * 16;
+            // Tensor memory: 128 columns = 64 doubles per thread, the slots
+            // of a row padded to the widest slice of the mesh.  Up to four
+            // rows all live there, of more the first four; choice 11 (two or
+            // four rows) keeps the first in shared memory instead, where it
+            // fits beside the halo.  The grid must be resident with one CTA
+            // per SM: each CTA takes all 512 columns, so a second one on the
+            // SM would wait for the first to finish.
+            cgcg_ks = cgcg_kt = 0;
+            cgcg_coef_off = cgcg_tm_w = 0;
+            auto resident = [&](int ks, int kt, size_t bytes) {
+                const void* fk = fn_cgcg_single(rr, ks, kt);
                 int per2 = 0;
-                if (with <= 227 * 1024 && raise_smem_limit(fn, with) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fn, nt, with) == cudaSuccess &&
-                    per2 * sms >= g) {
-                    cgcg_smem = with;
-                    cgcg_xs_off = static_cast<int>(off);
-                }
+                const bool ok = bytes <= 227 * 1024 && raise_smem_limit(fk, bytes) == cudaSuccess &&
+                                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fk, nt, bytes) == cudaSuccess &&
+                                per2 * sms >= g;
                 cudaGetLastError();
-            }
-            // the kernel that reads every warp's first row's coefficients
-            // from shared memory, where the CTAs' first slices fit beside
-            // the halo
-            cgcg_ks = 0;
-            cgcg_coef_off = 0;
-            // tensor memory (one-CTA-per-SM kernel): 128 columns = 64 doubles
-            // per thread, the slots of a row padded to the widest slice of
-            // the mesh.  Where all the thread's rows fit, they all live there
-            // and no coefficients are copied into shared memory; otherwise
-            // the rows after the shared-memory one that fit.
-            cgcg_kt = 0;
-            cgcg_tm_w = 0;
-            int tm_tw = 0;
-            if (want == 4 && nt == 512 && kernel_choice != 10) {
+                return ok;
+            };
+            if (want == 4 && kernel_choice != 10) {
                 int wmx = 0;
                 for (int q = 0; q < nslices; ++q) wmx = std::max(wmx, P.slice_w[static_cast<size_t>(q)]);
-                const int chw = rm[c] >= 4 ? 2 : 8;
-                tm_tw = (wmx + chw - 1) / chw * chw;
-                if (kernel_choice != 11 && (rm[c] == 2 || rm[c] == 4) && tm_tw > 0 && rm[c] * tm_tw <= 64) {
-                    cgcg_kt = rm[c];
-                    cgcg_tm_w = tm_tw;
+                const int chw = cgcg_round(rr), tw = (wmx + chw - 1) / chw * chw;
+                if (kernel_choice == 11 && (rr == 2 || rr == 4) && tw > 0 && (rr - 1) * tw <= 64) {
+                    long long cmax = 0;
+                    for (int bb = 0; bb < g; ++bb) {
+                        const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
+                        const int se = static_cast<int>(static_cast<long long>(bb + 1) * nslices / g);
+                        const int sc = std::min(sb + nwarps, se);
+                        cmax = std::max(cmax, P.slice_off[static_cast<size_t>(sc)] - P.slice_off[static_cast<size_t>(sb)]);
+                    }
+                    const size_t off = (cgcg_smem + 15) & ~static_cast<size_t>(15);
+                    if (resident(1, rr - 1, off + static_cast<size_t>(cmax) * 8)) {
+                        cgcg_ks = 1;
+                        cgcg_kt = rr - 1;
+                        cgcg_smem = off + static_cast<size_t>(cmax) * 8;
+                        cgcg_coef_off = static_cast<int>(off);
+                    }
                 }
+                const int kt = std::min(rr, 4);
+                if (!cgcg_ks && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
+                if (cgcg_kt) cgcg_tm_w = tw;
             }
-            if (want == 4 && cgcg_kt == 0) {
-                long long cmax = 0;
-                for (int bb = 0; bb < g; ++bb) {
-                    const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
-                    const int se = static_cast<int>(static_cast<long long>(bb + 1) * nslices / g);
-                    const int sc = std::min(sb + nwarps, se);
-                    cmax = std::max(cmax, P.slice_off[static_cast<size_t>(sc)] - P.slice_off[static_cast<size_t>(sb)]);
-                }
-                const long long per_need = (g + sms - 1) / sms;
-                const long long cap = std::min<long long>(227 * 1024, 228 * 1024 / per_need - 1024);
-                const size_t off = (cgcg_smem + 15) & ~static_cast<size_t>(15);
-                const size_t with = off + static_cast<size_t>(cmax) * 8;
-                const void* fk = fn_cgcg_single(rm[c], nt, 1);
-                int per2 = 0;
-                if (static_cast<long long>(with) <= cap && raise_smem_limit(fk, with) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fk, nt, with) == cudaSuccess &&
-                    per2 * sms >= g) {
-                    cgcg_ks = 1;
-                    cgcg_smem = with;
-                    cgcg_coef_off = static_cast<int>(off);
-                }
-                cudaGetLastError();
-            }
-            // the one-CTA-per-SM kernel with its first row in shared memory
-            // keeps the coefficients of its next rows in the SM's tensor
-            // memory for the solve: 128 columns (64 doubles) per thread, the
-            // slots of a row padded to the widest slice of the mesh
-            if (cgcg_ks && tm_tw > 0 && cgcg_tmem_rows(rm[c]) * tm_tw <= 64) {
-                cgcg_kt = cgcg_tmem_rows(rm[c]);
-                cgcg_tm_w = tm_tw;
-            }
-            // eight rows per thread where the shared-memory copy did not fit:
-            // the first four rows in tensor memory
-            if (!cgcg_ks && cgcg_kt == 0 && rm[c] == 8 && tm_tw > 0 && 4 * tm_tw <= 64) {
-                cgcg_kt = 4;
-                cgcg_tm_w = tm_tw;
-            }
-            // the one-CTA-per-SM kernel's rows' diagonal in shared memory
-            // (64^3: 12.05 -> 11.95 us per iteration; in registers it was
-            // slower)
+            // the rows' diagonal in shared memory (64^3: 12.05 -> 11.95 us
+            // per iteration; in registers it was slower)
             cgcg_pds_off = 0;
-            if (want == 4 && nt == 512) {
+            if (want == 4) {
                 const size_t off = (cgcg_smem + 15) & ~static_cast<size_t>(15);
-                const size_t with = off + static_cast<size_t>(rm[c]) * nt * 8;
-                const void* fk = fn_cgcg_single(rm[c], nt, cgcg_ks, cgcg_kt > 0);
-                int per2 = 0;
-                if (with <= 227 * 1024 && raise_smem_limit(fk, with) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fk, nt, with) == cudaSuccess &&
-                    per2 * sms >= g) {
+                const size_t with = off + static_cast<size_t>(rr) * nt * 8;
+                if (resident(cgcg_ks, cgcg_kt, with)) {
                     cgcg_smem = with;
                     cgcg_pds_off = static_cast<int>(off);
                 }
-                cudaGetLastError();
             }
-            if (cgcg_kt > 0) {
-                // the tensor-memory kernel must hold the whole grid resident
-                // with one CTA per SM: each CTA takes all 512 columns, so a
-                // second CTA on the SM would wait for the first to finish
-                const void* fk = fn_cgcg_single(rm[c], nt, cgcg_ks, true);
-                int per2 = 0;
-                if (g > sms || !(raise_smem_limit(fk, cgcg_smem) == cudaSuccess &&
-                      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fk, nt, cgcg_smem) == cudaSuccess &&
-                      per2 * sms >= g)) {
-                    cgcg_kt = 0;
-                    cgcg_tm_w = 0;
+            // ... and their pressure, where the kernel keeps it in memory
+            cgcg_xs_off = 0;
+            if (want == 4 && (rr == 3 || rr > 4)) {
+                const size_t off = (cgcg_smem + 15) & ~static_cast<size_t>(15);
+                const size_t with = off + static_cast<size_t>(rr) * nt * 8;
+                if (resident(cgcg_ks, cgcg_kt, with)) {
+                    cgcg_smem = with;
+                    cgcg_xs_off = static_cast<int>(off);
                 }
-                cudaGetLastError();
             }
             d_halo_ptr = dalloc<int>(hptr.size());
             d_halo_idx = dalloc<int>(hidx.size());
@@ -3080,9 +3506,19 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             dev_slot_max = static_cast<int>(smax);
             h_hptr = hptr;
             h_hidx = hidx;
+            if (want == 4) {
+                dev_rem_max = remote.most;
+                cgcg_lcs = static_cast<int>(cgcg_lcs_off(hmax, remote.most));
+                d_rem_ptr = dalloc<int>(remote.ptr.size());
+                d_rem = dalloc<int2>(remote.rem.size());
+                d_own = dalloc<int>(remote.own.size());
+                CUDA_OK(cudaMemcpy(d_rem_ptr, remote.ptr.data(), remote.ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+                if (!remote.rem.empty()) CUDA_OK(cudaMemcpy(d_rem, remote.rem.data(), remote.rem.size() * sizeof(int2), cudaMemcpyHostToDevice));
+                CUDA_OK(cudaMemcpy(d_own, remote.own.data(), remote.own.size() * sizeof(int), cudaMemcpyHostToDevice));
+            }
             if (mixed && want == 4) {
-                const void* mc[4] = {fn_mixed_single(1, nt), fn_mixed_single(2, nt), fn_mixed_single(4, nt),
-                                     fn_mixed_single(8, nt)};
+                const void* mc[4] = {fn_mixed<false, 512>(1), fn_mixed<false, 512>(2), fn_mixed<false, 512>(4),
+                                     fn_mixed<false, 512>(8)};
                 const size_t ms = static_cast<size_t>(hmax) * 16 + static_cast<size_t>(smax) * 6 + 16;
                 int per = 0;
                 if (ms <= 220 * 1024 &&
@@ -3096,16 +3532,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             }
         }
     }
-    if (variant == 1 && kernel_choice != 1 && kernel_choice != 5) {
-        const void* cands[4] = {reinterpret_cast<const void*>(k_pcg64r<1>), reinterpret_cast<const void*>(k_pcg64r<2>),
-                                reinterpret_cast<const void*>(k_pcg64r<4>), reinterpret_cast<const void*>(k_pcg64r<8>)};
-        for (int c = 0; c < 4; ++c) {
-            const int g = grid_for(cands[c]);
-            const int per_cta = (nslices + g - 1) / g;
-            if ((per_cta + PCG_WARPS - 1) / PCG_WARPS <= rm[c]) { rmax = rm[c]; nblocks = g; variant = 2; break; }
-        }
-    }
-    if (variant == 1 && N > 0) {
+    if (variant == 1 && N > 0 && kernel_choice != 2) {
         // the global-vector kernel with its neighbour values staged in shared
         // memory: each CTA's slices in the fewest parts (at most 8) whose
         // halos fit
@@ -3161,7 +3588,20 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         }
         cudaGetLastError();
     }
-    if (two_level && variant == 4 && nthreads == 512 && !mixed_ok) build_coarse(m, colp);
+    // register-resident rows with their neighbours gathered from L2: choice 2,
+    // and where no halo fits (80^3: 71 us per iteration against 24 with one)
+    if (variant == 1 && (kernel_choice == 2 || (kernel_choice != 1 && kernel_choice != 5 && !global_halo))) {
+        const int rm[4] = {1, 2, 4, 8};
+        const void* cands[4] = {reinterpret_cast<const void*>(k_pcg64r<1>), reinterpret_cast<const void*>(k_pcg64r<2>),
+                                reinterpret_cast<const void*>(k_pcg64r<4>), reinterpret_cast<const void*>(k_pcg64r<8>)};
+        for (int c = 0; c < 4; ++c) {
+            const int g = grid_for(cands[c]);
+            const int per_cta = (nslices + g - 1) / g;
+            if ((per_cta + PCG_WARPS - 1) / PCG_WARPS <= rm[c]) { rmax = rm[c]; nblocks = g; variant = 2; break; }
+        }
+    }
+    // the two-level preconditioner needs rows for every warp of the grid
+    if (two_level && variant == 4 && nslices >= 16 * sms && !mixed_ok) build_coarse(m, colp);
     if (multigrid && !mixed && !coarse) {
         mgh = new MgHierarchy;
         bool ok = false;
@@ -3186,6 +3626,16 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     d_bar = dalloc<unsigned>(4);
     d_out = dalloc<CgOut>(1);
     CUDA_OK(cudaMemset(d_bar, 0, 4 * sizeof(unsigned)));
+    if (variant == 4 || global_cgcg) {
+        const size_t nx = variant == 4 ? 2 * n : 0, nrec = static_cast<size_t>(nblocks) * 2 * REC_STRIDE;
+        d_rec = dalloc<TagVal>(nrec);
+        d_xw = dalloc<TagVal>(nx);
+        d_epoch = dalloc<unsigned long long>(1);
+        const unsigned long long one = 1;   // tags are never 0, the records' first content
+        CUDA_OK(cudaMemset(d_rec, 0, nrec * sizeof(TagVal)));
+        if (nx) CUDA_OK(cudaMemset(d_xw, 0, nx * sizeof(TagVal)));
+        CUDA_OK(cudaMemcpy(d_epoch, &one, sizeof one, cudaMemcpyHostToDevice));
+    }
 
     dev = PcgDev{};
     dev.N = NP; dev.NN = N; dev.E = E; dev.nslices = nslices; dev.nblocks = nblocks;
@@ -3200,9 +3650,12 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     dev.slot_max = dev_slot_max;
     dev.part = d_part; dev.bar = d_bar; dev.status = d_status; dev.out = d_out;
     dev.halo_ptr = d_halo_ptr; dev.halo_idx = d_halo_idx; dev.lcol = d_lcol; dev.halo_max = dev_halo_max;
-    dev.xs_off = cgcg_xs_off;
+    dev.rec = d_rec; dev.xw = d_xw; dev.epoch = d_epoch;
+    dev.rem_ptr = d_rem_ptr; dev.rem = d_rem; dev.own = d_own; dev.rem_max = dev_rem_max;
+    dev.lcs_off = cgcg_lcs;
     dev.coef_off = cgcg_coef_off;
     dev.pds_off = cgcg_pds_off;
+    dev.xs_off = cgcg_xs_off;
     dev.tm_w = cgcg_tm_w;
     dev.halo_parts = global_halo ? global_halo_parts : 0;
     dev.row_node = d_row_node;
@@ -3218,11 +3671,13 @@ void PcgEngine::release()
     mg_ready = false;
     void* ptrs[] = {d_slice_off, d_slice_w, d_col, d_cptr, d_cent, d_val, d_val32, d_r, d_z, d_pA,
                     d_pB, d_q, d_f32, d_part, d_bar, d_out, d_halo_ptr, d_halo_idx, d_lcol, d_row_node,
+                    d_rec, d_xw, d_epoch, d_rem_ptr, d_rem, d_own,
                     d_xp, d_bp, d_dp, d_fp, d_pair_ptr, d_pair_ij, d_pair_ent, d_ac, d_nbr_ptr, d_nbr_ids, d_hown};
     for (void* p : ptrs) if (p) cudaFree(p);
     d_pair_ptr = nullptr; d_pair_ij = nullptr; d_pair_ent = nullptr; d_ac = nullptr;
     d_nbr_ptr = nullptr; d_nbr_ids = nullptr; d_hown = nullptr;
     coarse = false;
+    d_rec = d_xw = nullptr; d_epoch = nullptr; d_rem_ptr = d_own = nullptr; d_rem = nullptr;
     d_slice_off = nullptr; d_slice_w = nullptr; d_col = nullptr; d_cptr = nullptr; d_cent = nullptr;
     d_val = nullptr; d_val32 = nullptr; d_r = d_z = d_pA = d_pB = d_q = nullptr; d_f32 = nullptr;
     d_part = nullptr; d_bar = nullptr; d_out = nullptr;
@@ -3305,10 +3760,10 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
         else fn = reinterpret_cast<const void*>(k_pcg64h<8>);
         smem = halo_smem;
     } else if (variant == 4 && mixed_ok) {
-        fn = fn_mixed_single(rmax, nthreads);
+        fn = fn_mixed<false, 512>(rmax);
         smem = mixed_smem;
     } else if (variant == 4) {
-        fn = fn_cgcg_single(rmax, nthreads, cgcg_ks, cgcg_kt > 0);
+        fn = fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
         smem = cgcg_smem;
     }
     CoarseDev C = cdev;
@@ -3460,6 +3915,7 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
         d_cent.push_back(ce);
     }
     h_slice_off[static_cast<size_t>(nslices)] = nslots;
+    h_slice_w = sw;
     d_slice_off = dalloc<long long>(h_slice_off.size());
     d_slice_w = dalloc<int>(sw.size());
     d_col = dalloc<int>(h_col.size());
@@ -3484,6 +3940,16 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
     }
     d_part = dalloc<double>(K * static_cast<size_t>(gmax) * 16);
     d_bar = dalloc<unsigned>(4 * K);
+    d_own = dalloc<int>(n);
+    d_rec = dalloc<TagVal>(K * static_cast<size_t>(gmax) * 2 * REC_STRIDE);
+    d_xw = dalloc<TagVal>(2 * n);
+    d_epoch = dalloc<unsigned long long>(K);
+    {
+        const std::vector<unsigned long long> one(K, 1);   // tags are never 0, the records' first content
+        CUDA_OK(cudaMemset(d_rec, 0, K * static_cast<size_t>(gmax) * 2 * REC_STRIDE * sizeof(TagVal)));
+        CUDA_OK(cudaMemset(d_xw, 0, 2 * n * sizeof(TagVal)));
+        CUDA_OK(cudaMemcpy(d_epoch, one.data(), K * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+    }
     d_out = dalloc<CgOut>(K);
     CUDA_OK(cudaMemset(d_bar, 0, 4 * K * sizeof(unsigned)));
     CUDA_OK(cudaMemset(d_out, 0, K * sizeof(CgOut)));
@@ -3499,12 +3965,13 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
         base.p32 = d_f32 + 6 * n; base.dz32 = d_f32 + 7 * n;
     }
     base.lcol = d_lcol;
+    base.xw = d_xw; base.own = d_own;
 }
 
 void PcgBatch::free_waves()
 {
     for (Wave& w : waves) {
-        void* ptrs[] = {w.d_cta_inst, w.d_inst, w.d_hptr, w.d_hidx};
+        void* ptrs[] = {w.d_cta_inst, w.d_inst, w.d_hptr, w.d_hidx, w.d_rptr, w.d_rem};
         for (void* p : ptrs) if (p) cudaFree(p);
     }
     waves.clear();
@@ -3539,8 +4006,8 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         packs[w].push_back(k);
         used[w] += minc[static_cast<size_t>(k)];
     }
-    const void* c64[4] = {fn_cgcg<true, BATCH_THREADS>(1), fn_cgcg<true, BATCH_THREADS>(2), fn_cgcg<true, BATCH_THREADS>(4),
-                          fn_cgcg<true, BATCH_THREADS>(8)};
+    const void* c64[4] = {fn_cgcg_batch<BATCH_THREADS>(1), fn_cgcg_batch<BATCH_THREADS>(2), fn_cgcg_batch<BATCH_THREADS>(4),
+                          fn_cgcg_batch<BATCH_THREADS>(8)};
     const void* c32[4] = {fn_mixed<true, BATCH_THREADS>(1), fn_mixed<true, BATCH_THREADS>(2), fn_mixed<true, BATCH_THREADS>(4),
                           fn_mixed<true, BATCH_THREADS>(8)};
     const int ci = p.rmax == 1 ? 0 : p.rmax == 2 ? 1 : p.rmax == 4 ? 2 : 3;
@@ -3548,10 +4015,14 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
     struct HostWave {
         int G = 0, hmax = 0;
         long long smax = 0;
-        std::vector<int> cta_inst, hptr, hidx;
+        std::vector<int> cta_inst, hptr, hidx, rptr;
+        std::vector<int2> rem;
+        int rmost = 0;
+        size_t lcsb = 0;
         std::vector<PcgInst> inst;
     };
     std::vector<HostWave> hw(packs.size());
+    std::vector<int> own(static_cast<size_t>(NP), 0xffff);
     std::vector<unsigned short> lcol(static_cast<size_t>(nslots), 0);
     for (size_t w = 0; w < packs.size(); ++w) {
         HostWave& H = hw[w];
@@ -3576,6 +4047,8 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         }
         H.G = tot;
         H.hptr.push_back(0);
+        RemoteLists remote(0);
+        remote.own.swap(own);   // the rows of all waves, each in one of them
         int cta = 0;
         for (size_t j = 0; j < mk.size(); ++j) {
             const int k = mk[j];
@@ -3590,6 +4063,8 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
             I.abs_tol = mem[static_cast<size_t>(k)].m->p.absToler;
             I.bar = d_bar + 4 * k;
             I.part = d_part + static_cast<size_t>(k) * static_cast<size_t>(gmax) * 16;
+            I.rec = d_rec + static_cast<size_t>(k) * static_cast<size_t>(gmax) * 2 * REC_STRIDE;
+            I.epoch = d_epoch + k;
             I.status = mem[static_cast<size_t>(k)].d_status;
             I.out = d_out + k;
             H.inst.push_back(I);
@@ -3614,9 +4089,15 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
                 H.hptr.push_back(static_cast<int>(H.hidx.size()));
                 H.hmax = std::max(H.hmax, static_cast<int>(cols.size()));
                 H.smax = std::max(H.smax, a1 - a0);
+                remote.add_cta(sb * 32, se * 32, cols);
+                H.lcsb = std::max(H.lcsb, cgcg_lcs_bytes(h_slice_w.data(), sb, se, BATCH_THREADS / 32, cgcg_round(p.rmax)));
             }
             cta += G[j];
         }
+        own.swap(remote.own);
+        H.rptr = std::move(remote.ptr);
+        H.rem = std::move(remote.rem);
+        H.rmost = remote.most;
     }
     // kernels and shared memory of every wave, before anything is replaced
     std::vector<Wave> nw(hw.size());
@@ -3624,7 +4105,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         const HostWave& H = hw[w];
         Wave& W = nw[w];
         W.G = H.G; W.rmax = p.rmax;
-        const size_t s64 = static_cast<size_t>(H.hmax) * 20 + static_cast<size_t>(H.smax) * 2 + 16;
+        const size_t s64 = cgcg_lcs_off(H.hmax + 1, H.rmost) + H.lcsb;
         const size_t s32 = static_cast<size_t>(H.hmax) * 16 + static_cast<size_t>(H.smax) * 6 + 16;
         auto fits = [&](const void* fn, size_t smem) {
             if (smem > 220 * 1024) return false;
@@ -3640,7 +4121,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
             return per * sms >= H.G;
         };
         if (mixed && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
-        else if (fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
+        else if (H.hmax <= CGCG_HALO_MAX && fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
         else {
             if (why) *why = "a wave does not fit co-resident at this tiling";
             return false;
@@ -3649,6 +4130,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
     free_waves();
     mixed_any = false;
     CUDA_OK(cudaMemcpy(d_lcol, lcol.data(), lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMemcpy(d_own, own.data(), own.size() * sizeof(int), cudaMemcpyHostToDevice));
     for (size_t w = 0; w < hw.size(); ++w) {
         const HostWave& H = hw[w];
         Wave& W = nw[w];
@@ -3660,6 +4142,10 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         CUDA_OK(cudaMemcpy(W.d_inst, H.inst.data(), H.inst.size() * sizeof(PcgInst), cudaMemcpyHostToDevice));
         CUDA_OK(cudaMemcpy(W.d_hptr, H.hptr.data(), H.hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
         if (!H.hidx.empty()) CUDA_OK(cudaMemcpy(W.d_hidx, H.hidx.data(), H.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
+        W.d_rptr = dalloc<int>(H.rptr.size());
+        W.d_rem = dalloc<int2>(H.rem.size());
+        CUDA_OK(cudaMemcpy(W.d_rptr, H.rptr.data(), H.rptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+        if (!H.rem.empty()) CUDA_OK(cudaMemcpy(W.d_rem, H.rem.data(), H.rem.size() * sizeof(int2), cudaMemcpyHostToDevice));
         W.dev = base;
         W.dev.nblocks = W.G;
         W.dev.cta_inst = W.d_cta_inst;
@@ -3667,6 +4153,13 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         W.dev.halo_ptr = W.d_hptr;
         W.dev.halo_idx = W.d_hidx;
         W.dev.halo_max = H.hmax;
+        W.dev.rem_ptr = W.d_rptr;
+        W.dev.rem = W.d_rem;
+        W.dev.rem_max = H.rmost;
+        if (!W.mixed) {
+            W.dev.halo_max = H.hmax + 1;   // the spare place
+            W.dev.lcs_off = static_cast<int>(cgcg_lcs_off(H.hmax + 1, H.rmost));
+        }
         W.dev.slot_max = static_cast<int>(H.smax);
         mixed_any = mixed_any || W.mixed;
     }
@@ -3683,8 +4176,9 @@ void PcgBatch::release()
     d_cptr.clear();
     d_cent.clear();
     void* ptrs[] = {d_slice_off, d_slice_w, d_col, d_row_node, d_lcol, d_val, d_val32, d_r, d_z, d_pA, d_pB, d_q,
-                    d_xp, d_bp, d_dp, d_fp, d_f32, d_part, d_bar, d_out};
+                    d_xp, d_bp, d_dp, d_fp, d_f32, d_part, d_bar, d_out, d_own, d_rec, d_xw, d_epoch};
     for (void* p : ptrs) if (p) cudaFree(p);
+    d_own = nullptr; d_rec = d_xw = nullptr; d_epoch = nullptr;
     d_slice_off = nullptr; d_slice_w = d_col = d_row_node = nullptr; d_lcol = nullptr; d_val = nullptr;
     d_val32 = nullptr; d_r = d_z = d_pA = d_pB = d_q = nullptr; d_xp = d_bp = d_dp = nullptr; d_fp = nullptr;
     d_f32 = nullptr; d_part = nullptr; d_bar = nullptr; d_out = nullptr;

@@ -12,6 +12,13 @@
 
 namespace cbs3d {
 
+// A value in flight between CTAs: written and read as one 16-byte access, so
+// a reader that sees the tag it waits for has the value that belongs to it.
+struct __align__(16) TagVal {
+    double v;
+    unsigned long long tag;
+};
+
 // One instance of a batched solve: CTAs [cta0, cta0+ncta) of the launch own
 // slices [s0, s1); its own scalars, barrier counter, partials, status, result.
 struct PcgInst {
@@ -20,6 +27,8 @@ struct PcgInst {
     double rel_tol, abs_tol;
     unsigned* bar;               // 64-bit arrival counter (zeroed before each launch)
     double* part;                // 2 * ncta * 8 partials (double-buffered by phase)
+    TagVal* rec;                 // 2 x ncta all-reduce records, a line each (single-reduction kernel)
+    unsigned long long* epoch;   // ... and the number of its next solve
     DevStatus* status;
     CgOut* out;
 };
@@ -52,18 +61,26 @@ struct PcgDev {
     int halo_max;                // largest halo (shared-memory sizing)
     double* part;                // 2 * nblocks * 8 partials (double-buffered by phase)
     unsigned* bar;               // 64-bit arrival counter
+    // single-reduction kernels: tagged exchange between CTAs
+    TagVal* rec;                 // 2 x nblocks all-reduce records, a line each
+    TagVal* xw;                  // 2 x N records of one row's value (k_pcg64c)
+    unsigned long long* epoch;   // number of the next solve
+    const int* rem_ptr;          // nblocks+1: each CTA's remote halo entries in rem
+    const int2* rem;             // (row position at its owner, place in this CTA's halo)
+    const int* own;              // N: place of the row in its own CTA's halo (0xffff: none), bit 16: other CTAs read it
+    int lcs_off;                 // byte offset in shared memory of the local columns (k_pcg64c)
+    int rem_max;                 // most remote entries of a CTA (shared-memory sizing)
     DevStatus* status;
     CgOut* out;
     const int* cta_inst;         // batched launch: instance of each CTA (else null)
     const PcgInst* inst;         // batched launch: instance descriptors (else null)
-    int xs_off;                  // CG-CG kernel: byte offset in shared memory of its rows' pressure
-                                 // and diagonal (2*RMAX*threads doubles); 0: read from global memory
     int halo_parts;              // global-vector kernel with a shared-memory halo: parts per CTA, each
                                  // with its own halo (halo_ptr indexed by CTA*parts + part)
     int coef_off;                // CG-CG kernel with its warps' first rows' coefficients in shared
                                  // memory: byte offset of that copy
     int pds_off;                 // one-CTA-per-SM CG-CG kernel: byte offset in shared memory of its
                                  // rows' diagonal (RMAX*threads doubles); 0: read from global memory
+    int xs_off;                  // ... and of its rows' pressure (0: in registers or global memory)
     int tm_w;                    // CG-CG kernel with rows in tensor memory: slots per row there (the
                                  // widest slice, rounded up to the kernel's load width)
 };
@@ -140,18 +157,24 @@ public:
     long long global_halo_total = 0;   // halo entries over all CTAs
     int global_halo_parts = 1;         // parts per CTA, each with its own halo
     size_t halo_smem = 0;    // dynamic shared memory of the halo kernel
-    size_t cgcg_smem = 0;    // ... of the CG-CG kernel (halo + its rows' pressure and diagonal)
-    int cgcg_xs_off = 0;     // where those rows start (0: kept in global memory)
+    size_t cgcg_smem = 0;    // ... of the CG-CG kernel (halo, remote entries, its rows' diagonal)
     int cgcg_ks = 0;         // 1: the kernel reads its warps' first rows' coefficients from shared memory
     int cgcg_coef_off = 0;   // where they start
     int cgcg_kt = 0;         // >0: that many rows per thread, after the shared-memory one, read from tensor memory
     int cgcg_tm_w = 0;       // slots per row in tensor memory
     int cgcg_pds_off = 0;    // where the rows' diagonal starts in shared memory (0: global memory)
+    int cgcg_xs_off = 0;     // ... and their pressure
     size_t mixed_smem = 0;   // dynamic shared memory of the mixed-precision kernel
     bool mixed_ok = false;   // mixed precision runs on the FP32 kernel (else FP64)
     int dev_slot_max = 0;
     int *d_halo_ptr = nullptr, *d_halo_idx = nullptr;
     unsigned short* d_lcol = nullptr;
+    int *d_rem_ptr = nullptr, *d_own = nullptr;   // remote halo entries and own rows' places (k_pcg64c)
+    int2* d_rem = nullptr;
+    int dev_rem_max = 0;
+    int cgcg_lcs = 0;        // byte offset of the CG-CG kernel's local columns
+    TagVal *d_rec = nullptr, *d_xw = nullptr;
+    unsigned long long* d_epoch = nullptr;
     int* d_row_node = nullptr;
     double *d_xp = nullptr, *d_bp = nullptr, *d_dp = nullptr;   // pressure, rhs, diagonal by position
     uint8_t* d_fp = nullptr;
@@ -227,7 +250,8 @@ private:
         PcgDev dev{};
         int* d_cta_inst = nullptr;
         PcgInst* d_inst = nullptr;
-        int *d_hptr = nullptr, *d_hidx = nullptr;
+        int *d_hptr = nullptr, *d_hidx = nullptr, *d_rptr = nullptr;
+        int2* d_rem = nullptr;
     };
     void free_waves();
     std::vector<PcgBatchMember> mem;
@@ -241,7 +265,7 @@ private:
     int nslices = 0, NP = 0;
     long long nslots = 0;
     std::vector<long long> h_slice_off;
-    std::vector<int> h_col;
+    std::vector<int> h_col, h_slice_w;
     long long* d_slice_off = nullptr;
     int *d_slice_w = nullptr, *d_col = nullptr, *d_row_node = nullptr;
     unsigned short* d_lcol = nullptr;
@@ -253,6 +277,9 @@ private:
     float* d_f32 = nullptr;
     double* d_part = nullptr;
     unsigned* d_bar = nullptr;
+    int* d_own = nullptr;
+    TagVal *d_rec = nullptr, *d_xw = nullptr;
+    unsigned long long* d_epoch = nullptr;
     CgOut* d_out = nullptr;
     PcgDev base{};
 };

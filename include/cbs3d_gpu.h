@@ -101,8 +101,9 @@ typedef struct cbs3d_options {
                                 5 vectors in global memory + one grid sync per iteration,
                                 10 as 4 with no coefficients kept in tensor memory,
                                 11 as 4 with the first row per thread in shared memory and the
-                                next ones in tensor memory (0 and 4 keep every row in tensor
-                                memory where they all fit, else as 11) */
+                                next ones in tensor memory, at two and four rows per thread
+                                (0 and 4 keep every row in tensor memory where they all fit,
+                                else the first four) */
     int case_cache;          /* cbs3d_create_from_case: keep the parsed case in <case>.cbscache
                                 (keyed by every source file's size and time) and reuse it */
     int pcg_two_level;       /* extension: Jacobi plus a coarse correction on one aggregate of rows
@@ -411,8 +412,8 @@ cbs3d_status cbs3d_coarse_inverse(int device, int g, const double* a, double* ai
  * bandwidth, a larger one the HBM bandwidth.  Back-to-back launches cost
  * about 4 us each on B200, so the passes run inside one launch.
  * cbs3d_probe_allreduce: microseconds per grid-wide all-reduce
- * of the persistent PCG kernel's kind (one 512-thread CTA per SM, five
- * values, `iters` dependent all-reduces in one cooperative launch) -- the
+ * of the persistent PCG kernel's kind (one 512-thread CTA per SM, three
+ * sums, `iters` dependent all-reduces in one cooperative launch) -- the
  * per-iteration latency floor of the single-reduction PCG.  Both allocate
  * and free their own device memory. */
 cbs3d_status cbs3d_probe_bandwidth(int device, long long bytes, int passes, int mode, double* gbs);

@@ -1,0 +1,75 @@
+"""The register-resident single-reduction PCG at the edges of its tilings (one
+to six rows per thread, grids of a few CTAs) against the global-vector
+single-reduction kernel, which performs the same operations row by row with
+its vectors in global memory: fields and iteration counts agree bit for bit.
+Their grids are the same, so no tolerance is involved."""
+import pytest
+
+from helpers import bitwise, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _gpu():
+    from cbs3d import gpu
+    return gpu
+
+
+def _same(case, steps=2, **over):
+    gpu = _gpu()
+    a, b = gpu.Context(case, pcg_kernel=4, **over), gpu.Context(case, pcg_kernel=5, **over)
+    sa, sb = a.step(steps), b.step(steps)
+    assert sa.pcg_kernel == 9 and sb.pcg_kernel == 8
+    assert sa.cg_iterations_total == sb.cg_iterations_total
+    assert sa.cg.final_max_abs == sb.cg.final_max_abs and sa.cg.final_l2 == sb.cg.final_l2
+    for x, y in zip(a.fields(), b.fields()):
+        assert bitwise(x, y)
+    a.close()
+    b.close()
+
+
+# 1 slice; a few CTAs; and on 148 SMs the last size of one, two and three rows
+# per thread with the first size of the next (41/42, 52/53, 60/61), five (67)
+@pytest.mark.parametrize("n", [2, 5, 11, 41, 42, 52, 53, 60, 61, 67])
+def test_tilings_match_the_global_vector_kernel(n):
+    from cbs3d import cases
+    _same(cases.cavity(n, re=400.0, ntime=10 ** 6, jitter=0.15 if n > 2 else 0.0, seed=1234))
+
+
+@pytest.mark.parametrize("conv_test,abs_tol", [(1, 1e-9), (3, 1e-9)])
+def test_stopping_tests_on_the_largest_residual(conv_test, abs_tol):
+    """Tests 1 and 3 carry max|r| in every iteration's all-reduce; also against
+    the two-reduction kernel, which forms it in its own way."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(13, re=100.0, ntime=10 ** 6, cg_conv_test=conv_test, absToler=abs_tol, relToler=1e-9)
+    _same(case)
+    a, c = gpu.Context(case), gpu.Context(case, pcg_kernel=1)
+    sa, sc = a.step(2), c.step(2)
+    assert abs(sa.cg.iterations - sc.cg.iterations) <= 2
+    # solves to 1e-9 whose sums are grouped differently
+    assert rel_l2(a.fields()[1], c.fields()[1]) <= 1e-8
+
+
+def test_fixed_and_inactive_rows():
+    """Outlet rows (fixed pressure) and solid rows (no pressure) stay 0 in the
+    recurrences without branches."""
+    from cbs3d import cases
+    _same(cases.channel(21, 5, 6, ntime=10 ** 6))
+    _same(cases.cht_slab(17, 6, 3, 5, ntime=10 ** 6))
+
+
+def test_global_vector_kernel_rows_in_tensor_memory():
+    """The global-vector kernel on few CTAs (several parts per CTA, rows in
+    tensor memory and streamed rows alternating) against the default engine:
+    the same solutions to the solver's tolerance."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(33, re=400.0, ntime=10 ** 6, jitter=0.15, seed=1234)
+    a = gpu.Context(case)
+    a.step(2)
+    for blocks in (1, 3, 50):
+        b = gpu.Context(case, pcg_kernel=5, pcg_blocks=blocks)
+        assert b.step(2).pcg_kernel == 8
+        assert rel_l2(b.fields()[1], a.fields()[1]) <= 1e-8
+        b.close()
