@@ -1012,9 +1012,16 @@ __device__ __forceinline__ void st_tag(TagVal* p, double v, unsigned long long t
                  "l"(__double_as_longlong(v)), "l"(tag)
                  : "memory");
 }
+template <bool ACQ = false>
 __device__ __forceinline__ void ld_tag(const TagVal* p, double& v, unsigned long long& tag)
 {
     long long b;
+    if constexpr (ACQ)
+        asm volatile("{ .reg .b128 t; ld.acquire.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                     : "=l"(b), "=l"(tag)
+                     : "l"(p)
+                     : "memory");
+    else
     asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
                  : "=l"(b), "=l"(tag)
                  : "l"(p)
@@ -1083,7 +1090,8 @@ __device__ __forceinline__ double red4(int q, double a, double b)
 // 148-CTA all-reduce took 4-6 us, with one 2.0 us (against 2.4 us for a
 // counter and separate partials).
 // ORDERED: the CTA's earlier plain stores are made visible before the record
-// (a fence), for kernels that exchange vectors by plain stores.
+// (a fence) and the polls acquire, for kernels that exchange vectors by plain
+// stores.
 constexpr int REC_STRIDE = 8;    // TagVals per record: one 128-byte line
 template <int NT, bool ORDERED, bool MX>
 __device__ __forceinline__ void tag_allreduce_publish(const TagComm& c, int phase, const double (&v)[4])
@@ -1168,7 +1176,7 @@ __device__ __forceinline__ bool tag_allreduce_wait(const TagComm& c, int phase, 
         for (int u = 0; u < MP; ++u) {
             x[u] = 0.0;
             t[u] = want;
-            if (j + u * STEP < c.G) ld_tag(r + u * STEP * REC_STRIDE, x[u], t[u]);
+            if (j + u * STEP < c.G) ld_tag<ORDERED>(r + u * STEP * REC_STRIDE, x[u], t[u]);
         }
 #pragma unroll
         for (int u = 0; u < MP; ++u) missed = missed || t[u] != want;
@@ -1179,11 +1187,10 @@ __device__ __forceinline__ bool tag_allreduce_wait(const TagComm& c, int phase, 
             for (int u = 0; u < MP; ++u)
                 while (t[u] != want) {
                     if (lim.expired(c.status)) { ok = false; break; }
-                    ld_tag(r + u * STEP * REC_STRIDE, x[u], t[u]);
+                    ld_tag<ORDERED>(r + u * STEP * REC_STRIDE, x[u], t[u]);
                 }
         }
         __syncwarp();
-        if (ORDERED) __threadfence();
         a = x[0];
 #pragma unroll
         for (int u = 1; u < MP; ++u) a = red4<MX>(q, a, x[u]);
@@ -1228,6 +1235,71 @@ struct StopTest {
     }
 };
 
+// ---------------------------------------------- tensor memory as storage
+// The SM's 256 KB tensor memory (TMEM: 128 lanes x 512 columns of 32 bits)
+// holds, for the whole solve, coefficients that would otherwise stream from
+// L2 in every iteration.  No MMA touches it: it is read with tcgen05.ld into
+// registers.  With the 32x32b access shape, warp w reads and writes lanes
+// 32*(w%4) .. 32*(w%4)+31, one lane per thread, so the four warps that share
+// a lane quarter split the 512 columns into four ranges of 128.  One warp
+// allocates all 512 columns (one CTA per SM, nothing else in this library
+// uses TMEM) and frees them before the CTA exits, on every path.
+__device__ __forceinline__ void tmem_alloc_all(uint32_t* slot)
+{
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(slot));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(a) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free_all(uint32_t base)
+{
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
+__device__ __forceinline__ void tmem_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// one double into two consecutive columns of this thread's lane (low word first)
+__device__ __forceinline__ void tmem_st_f64(uint32_t addr, double v)
+{
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr),
+                 "r"(static_cast<uint32_t>(b)), "r"(static_cast<uint32_t>(b >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_b32(uint32_t addr, uint32_t v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// N consecutive 32-bit columns of this thread's lane; the registers are
+// undefined until tmem_wait_ld, after which tmem_hold pins their uses
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[N]);
+template <>
+__device__ __forceinline__ void tmem_ld<4>(uint32_t addr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+template <>
+__device__ __forceinline__ void tmem_ld<16>(uint32_t addr, uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                   "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                   "=r"(r[14]), "=r"(r[15])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// after tmem_wait_ld: an empty statement that "rewrites" the loaded registers,
+// so no use of them can be scheduled before the wait
+template <int N>
+__device__ __forceinline__ void tmem_hold(uint32_t (&r)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+
 // ------------------------------------ global-vector single-reduction PCG
 // The Chronopoulos-Gear iteration of k_pcg64c for meshes whose rows do not
 // fit the register tiling: the rows' r, s, w (double-buffered by iteration
@@ -1239,7 +1311,16 @@ struct StopTest {
 // search direction lives in the engine's permuted right-hand side, which is
 // dead once r0 is formed.  Where the whole halo fits (one part) the inverse
 // diagonal of the halo stays in shared memory for the solve.
-__device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long epoch)
+//
+// Bound by memory traffic (96^3: 248 MB per iteration, more than L2 holds)
+// and, with one row per lane at a time, by the latency of a row's loads: so a
+// warp requests the first 16 slots of its next streamed row while it works on
+// the present one (into the registers just consumed), and the SM's tensor
+// memory keeps the coefficients and local columns of D.tm_rows of its rows
+// (three of Kuhn meshes' 14 slots) for the solve.  Those alternate with the
+// streamed ones, so that memory stays busy while they are processed: four of
+// them ahead of the streamed rows took 88^3 from 31.5 to 33.7 us.
+__device__ __forceinline__ void pcg64g_body(const PcgDev& D, uint32_t tm, unsigned long long epoch)
 {
     constexpr int NT = PCG_THREADS;
     const SegView g = seg_view<false>(D);
@@ -1267,37 +1348,107 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
         h0 = D.halo_ptr[b * KP + q];
         nh = D.halo_ptr[b * KP + q + 1] - h0;
     };
-    // off-diagonal sum of row s*32+lane over the staged halo: rounds of eight
-    // slots, the next round's local columns and coefficients requested before
-    // this round's shared-memory reads; the sum runs over the slots in order
-    auto offdiag = [&](int s) -> double {
-        const long long base = D.slice_off[s] + lane;
-        const int w = D.slice_w[s];
-        constexpr int CH = 8;
-        double off = 0.0;
-        int cn[CH];
-        double vn[CH];
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            cn[u] = u < w ? (int)__ldcs(D.lcol + base + 32LL * u) : 0;
-            vn[u] = u < w ? __ldcs(D.val + base + 32LL * u) : 0.0;
+    // first slot (from the CTA's first) and width of the CTA's slices
+    int2* meta = reinterpret_cast<int2*>(smem_raw + D.lcs_off);
+    const long long S0 = D.slice_off[s_beg];
+    for (int k = threadIdx.x; k < s_end - s_beg; k += NT) meta[k] = make_int2((int)(D.slice_off[s_beg + k] - S0), D.slice_w[s_beg + k]);
+    __syncthreads();
+    const double* vbase = D.val + S0 + lane;
+    const unsigned short* cbase = D.lcol + S0 + lane;
+    // The warp's rows of part q are slices ps0 + warp + 16*i; row i is in
+    // tensor memory when i is even and fewer than tm_rows rows came before.
+    // The t-th row there: columns TC*t .. of lane 32*(warp%4)+lane, from
+    // 128*(warp/4) on: tm_w doubles, then tm_w/2 words of two local columns.
+    const uint32_t tm0 = tm + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(128 * (warp >> 2));
+    const int TC = 2 * D.tm_w + D.tm_w / 2;
+    auto part_slices = [&](int part, int& ps0, int& n) {
+        ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP) + warp;
+        const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
+        n = ps1 > ps0 ? (ps1 - ps0 + PCG_WARPS - 1) / PCG_WARPS : 0;
+    };
+    auto tm_used = [&](int t0, int n) { const int e = (n + 1) / 2, f = D.tm_rows - t0; return e < f ? e : f; };
+    for (int part = 0, t0 = 0; part < KP; ++part) {
+        int ps0, n;
+        part_slices(part, ps0, n);
+        const int nt = tm_used(t0, n);
+        for (int t = 0; t < nt; ++t) {
+            const int2 m = meta[ps0 + 2 * t * PCG_WARPS - s_beg];
+            const uint32_t at = tm0 + TC * (t0 + t);
+            for (int u = 0; u < D.tm_w; u += 2) {
+                const bool h0 = u < m.y, h1 = u + 1 < m.y;
+                tmem_st_f64(at + 2 * u, h0 ? __ldcs(vbase + m.x + 32 * u) : 0.0);
+                tmem_st_f64(at + 2 * u + 2, h1 ? __ldcs(vbase + m.x + 32 * u + 32) : 0.0);
+                const unsigned lo = h0 ? __ldcs(cbase + m.x + 32 * u) : 0, hi = h1 ? __ldcs(cbase + m.x + 32 * u + 32) : 0;
+                tmem_st_b32(at + 2 * D.tm_w + u / 2, lo | hi << 16);
+            }
         }
-        for (int k0 = 0; k0 < w; k0 += CH) {
-            int c[CH];
-            double v[CH];
-#pragma unroll
-            for (int u = 0; u < CH; ++u) { c[u] = cn[u]; v[u] = vn[u]; }
+        t0 += nt;
+    }
+    if (D.tm_rows) tmem_wait_st();
+    // Every row of a part, in order: pre(i) (loads the row's vectors), the
+    // off-diagonal sum over the staged halo (the slots in order), post(i, sum)
+    auto rows = [&](int part, int t0, auto&& pre, auto&& post) {
+        constexpr int CH = 8, PH = 2;    // slots per round, rounds requested ahead
+        int ps0, n;
+        part_slices(part, ps0, n);
+        auto in_tm = [&](int i) { return !(i & 1) && t0 + (i >> 1) < D.tm_rows; };
+        double v[PH][CH];
+        int c[PH][CH];
+        auto request = [&](int h, const int2& m) {
 #pragma unroll
             for (int u = 0; u < CH; ++u) {
-                const int k = k0 + CH + u;
-                cn[u] = k < w ? (int)__ldcs(D.lcol + base + 32LL * k) : 0;
-                vn[u] = k < w ? __ldcs(D.val + base + 32LL * k) : 0.0;
+                const int k = CH * h + u;
+                v[h][u] = k < m.y ? __ldcs(vbase + m.x + 32 * k) : 0.0;
+                c[h][u] = k < m.y ? (int)__ldcs(cbase + m.x + 32 * k) : 0;
             }
+        };
+        int nx = in_tm(0) ? 1 : 0;       // next streamed row
+        if (nx < n) {
+            const int2 m = meta[ps0 + nx * PCG_WARPS - s_beg];
 #pragma unroll
-            for (int u = 0; u < CH; ++u)
-                if (k0 + u < w) off = fma(v[u], vh[c[u]], off);
+            for (int h = 0; h < PH; ++h) request(h, m);
         }
-        return off;
+        for (int i = 0; i < n; ++i) {
+            const int s = ps0 + i * PCG_WARPS;
+            const int2 m = meta[s - s_beg];
+            pre(s * 32 + lane);
+            double off = 0.0;
+            if (i == nx) {
+                nx = in_tm(i + 1) ? i + 2 : i + 1;
+                const int2 mn = nx < n ? meta[ps0 + nx * PCG_WARPS - s_beg] : make_int2(0, 0);
+#pragma unroll
+                for (int h = 0; h < PH; ++h) {
+                    double x[CH];
+#pragma unroll
+                    for (int u = 0; u < CH; ++u) x[u] = vh[c[h][u]];
+#pragma unroll
+                    for (int u = 0; u < CH; ++u)
+                        if (CH * h + u < m.y) off = fma(v[h][u], x[u], off);
+                    request(h, mn);
+                }
+                for (int k = PH * CH; k < m.y; ++k)
+                    off = fma(__ldcs(vbase + m.x + 32 * k), vh[__ldcs(cbase + m.x + 32 * k)], off);
+            } else {
+                const uint32_t at = tm0 + TC * (t0 + (i >> 1));
+                for (int k0 = 0; k0 < m.y; k0 += CH) {
+                    uint32_t tv[2 * CH], tc[CH / 2];
+                    tmem_ld<CH / 2>(at + 2 * D.tm_w + k0 / 2, tc);
+                    tmem_ld<2 * CH>(at + 2 * k0, tv);
+                    tmem_wait_ld();
+                    tmem_hold<CH / 2>(tc);
+                    tmem_hold<2 * CH>(tv);
+                    double x[CH];
+#pragma unroll
+                    for (int u = 0; u < CH; ++u) x[u] = vh[u & 1 ? tc[u / 2] >> 16 : tc[u / 2] & 0xffffu];
+#pragma unroll
+                    for (int u = 0; u < CH; ++u)
+                        if (k0 + u < m.y)
+                            off = fma(__hiloint2double(static_cast<int>(tv[2 * u + 1]), static_cast<int>(tv[2 * u])), x[u], off);
+                }
+            }
+            post(s * 32 + lane, off);
+        }
+        return t0 + tm_used(t0, n);
     };
 
     double t[4];
@@ -1316,17 +1467,13 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
     // ---- phase 0a: r0 = b - A x0 (constraints as the reference), dz, p = s = 0;
     // partials: invalid diagonals, non-finite residuals, (r,r), max|r|
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int part = 0; part < KP; ++part) {
-        const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
-        const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
+    for (int part = 0, q = 0; part < KP; ++part) {
         int h0, nh;
         halo_of(part, h0, nh);
         __syncthreads();
         for (int k = threadIdx.x; k < nh; k += NT) vh[k] = __ldcg(D.pres + D.halo_idx[h0 + k]);
         __syncthreads();
-        for (int s = ps0 + warp; s < ps1; s += PCG_WARPS) {
-            const int i = s * 32 + lane;
-            const double off = offdiag(s);
+        q = rows(part, q, [](int) {}, [&](int i, double off) {
             const uint8_t f = D.nflag[i];
             const bool active = f & 1, fr = (f & 1) && !(f & 4);
             const double pd = D.pdiag[i];
@@ -1348,7 +1495,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
             rb[0][i] = ri;
             dz[i] = dd;
             sb[0][i] = 0.0;
-        }
+        });
     }
     if (!allreduce(acc, true)) return;
     const double init = sqrt(t[2]);
@@ -1361,9 +1508,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
     // ---- phase 0b: z0 = M^-1 r0, w0 = A z0, gamma0 = (r0,z0), delta0 = (z0,w0);
     // the right-hand side is no longer needed: p = 0 from here
     acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
-    for (int part = 0; part < KP; ++part) {
-        const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
-        const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
+    for (int part = 0, q = 0; part < KP; ++part) {
         int h0, nh;
         halo_of(part, h0, nh);
         __syncthreads();
@@ -1374,9 +1519,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
             vh[k] = __ldcg(rb[0] + j) * dj;
         }
         __syncthreads();
-        for (int s = ps0 + warp; s < ps1; s += PCG_WARPS) {
-            const int i = s * 32 + lane;
-            const double off = offdiag(s);
+        q = rows(part, q, [](int) {}, [&](int i, double off) {
             const uint8_t f = D.nflag[i];
             const bool fr = (f & 1) && !(f & 4);
             const double ri = rb[0][i];
@@ -1388,7 +1531,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
                 acc[0] = fma(ri, zi, acc[0]);
                 acc[1] = fma(zi, wi, acc[1]);
             }
-        }
+        });
     }
     if (!allreduce(acc, false)) return;
     double gam = t[0];
@@ -1404,9 +1547,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
         const double* wo = wb[po];
         const double* ro = rb[po];
         acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
-        for (int part = 0; part < KP; ++part) {
-            const int ps0 = s_beg + (int)((long long)part * (s_end - s_beg) / KP);
-            const int ps1 = s_beg + (int)((long long)(part + 1) * (s_end - s_beg) / KP);
+        for (int part = 0, q = 0; part < KP; ++part) {
             int h0, nh;
             halo_of(part, h0, nh);
             // stage z_it of the halo: s = w_o + beta*s_o, r = r_o - alpha*s,
@@ -1440,23 +1581,24 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
             }
             // own rows: p = z_o + beta*p, s = w_o + beta*s_o, x += alpha*p,
             // r = r_o - alpha*s; then w = A z, the partials
-            for (int s = ps0 + warp; s < ps1; s += PCG_WARPS) {
-                const int i = s * 32 + lane;
-                const uint8_t f = D.nflag[i];
+            uint8_t f;
+            double r_o, s_o, w_o, dd, p_o, x_o, pd;
+            q = rows(part, q, [&](int i) {
+                f = D.nflag[i];
+                r_o = ro[i], s_o = so[i], w_o = wo[i], dd = dz[i];
+                p_o = pv[i], x_o = D.pres[i], pd = D.pdiag[i];
+            }, [&](int i, double off) {
                 const bool fr = (f & 1) && !(f & 4);
-                const double r_o = ro[i], s_o = so[i], w_o = wo[i], dd = dz[i];
-                const double p_o = pv[i];
-                const double off = offdiag(s);
                 const double zo = r_o * dd;
                 const double pi = fr ? fma(beta, p_o, zo) : 0.0;
                 const double si = fma(beta, s_o, w_o);
-                if (fr) D.pres[i] = fma(alpha, pi, D.pres[i]);
+                if (fr) D.pres[i] = fma(alpha, pi, x_o);
                 const double ri = fma(-alpha, si, r_o);
                 pv[i] = pi;
                 rb[pn][i] = ri;
                 sb[pn][i] = si;
                 const double zi = ri * dd;
-                const double wi = fr ? fma(D.pdiag[i], zi, off) : 0.0;
+                const double wi = fr ? fma(pd, zi, off) : 0.0;
                 wb[pn][i] = wi;
                 if (fr) {
                     acc[0] = fma(ri, zi, acc[0]);
@@ -1464,7 +1606,7 @@ __device__ __forceinline__ void pcg64g_body(const PcgDev& D, unsigned long long 
                     acc[2] = fma(ri, ri, acc[2]);
                     acc[3] = max_bits(acc[3], fabs(ri));
                 }
-            }
+            });
         }
         if (!allreduce(acc, stop.needs_max())) return;
         rr = t[2];
@@ -1512,73 +1654,25 @@ __device__ __forceinline__ void tag_end(const PcgDev& D, unsigned long long epoc
     if (g.b == 0 && threadIdx.x == 0) *seg_epoch(D, g) = (epoch >> 32) + 1;
 }
 
+// one CTA per SM: with rows in tensor memory warp 0 takes all of it before
+// the solve and returns it after, every exit of the body being CTA-uniform
 __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev D)
 {
     unsigned long long epoch;
     if (!tag_begin<false>(D, epoch)) return;
-    pcg64g_body(D, epoch);
+    __shared__ uint32_t s_tm;
+    const bool w0 = (threadIdx.x >> 5) == 0;
+    if (w0 && D.tm_rows) tmem_alloc_all(&s_tm);
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    const uint32_t tm = D.tm_rows ? s_tm : 0u;
+    pcg64g_body(D, tm, epoch);
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    if (w0 && D.tm_rows) tmem_free_all(tm);
     tag_end<false>(D, epoch);
-}
-
-// ---------------------------------------------- tensor memory as storage
-// The SM's 256 KB tensor memory (TMEM: 128 lanes x 512 columns of 32 bits)
-// holds, for the whole solve, coefficients that would otherwise stream from
-// L2 in every iteration.  No MMA touches it: it is read with tcgen05.ld into
-// registers.  With the 32x32b access shape, warp w reads and writes lanes
-// 32*(w%4) .. 32*(w%4)+31, one lane per thread, so the four warps that share
-// a lane quarter split the 512 columns into four ranges of 128.  One warp
-// allocates all 512 columns (one CTA per SM, nothing else in this library
-// uses TMEM) and frees them before the CTA exits, on every path.
-__device__ __forceinline__ void tmem_alloc_all(uint32_t* slot)
-{
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(slot));
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(a) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_free_all(uint32_t base)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
-}
-__device__ __forceinline__ void tmem_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// one double into two consecutive columns of this thread's lane (low word first)
-__device__ __forceinline__ void tmem_st_f64(uint32_t addr, double v)
-{
-    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr),
-                 "r"(static_cast<uint32_t>(b)), "r"(static_cast<uint32_t>(b >> 32))
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// N consecutive 32-bit columns of this thread's lane; the registers are
-// undefined until tmem_wait_ld, after which tmem_hold pins their uses
-template <int N>
-__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[N]);
-template <>
-__device__ __forceinline__ void tmem_ld<4>(uint32_t addr, uint32_t (&r)[4])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-template <>
-__device__ __forceinline__ void tmem_ld<16>(uint32_t addr, uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                   "=r"(r[14]), "=r"(r[15])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// after tmem_wait_ld: an empty statement that "rewrites" the loaded registers,
-// so no use of them can be scheduled before the wait
-template <int N>
-__device__ __forceinline__ void tmem_hold(uint32_t (&r)[N])
-{
-#pragma unroll
-    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
 }
 
 // The single-reduction iteration with the rows' vectors in registers.  Row by
@@ -3571,7 +3665,21 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         // the two-reduction one (bitwise the same arithmetic as choices 2, 3)
         global_cgcg = kernel_choice != 1;
         const void* fh = global_cgcg ? reinterpret_cast<const void*>(k_pcg64g) : reinterpret_cast<const void*>(k_pcg64<true>);
-        const size_t smem = static_cast<size_t>(hmax) * 16 + 16;
+        size_t smem = static_cast<size_t>(hmax) * 16 + 16;
+        // the slices' slots and widths behind the halo, and rows per warp in
+        // tensor memory: rounds of eight slots, 2.5 columns per slot of 128
+        cgcg_tm_w = g_tm_rows = cgcg_lcs = 0;
+        if (global_cgcg) {
+            cgcg_lcs = static_cast<int>(smem);
+            smem += static_cast<size_t>((nslices + g - 1) / g) * sizeof(int2);
+            int wmx = 0;
+            for (int q = 0; q < nslices; ++q) wmx = std::max(wmx, P.slice_w[static_cast<size_t>(q)]);
+            const int tw = (wmx + 7) / 8 * 8;
+            if (tw > 0 && 5 * tw <= 256 && g <= sms) {
+                cgcg_tm_w = tw;
+                g_tm_rows = 256 / (5 * tw);
+            }
+        }
         int per = 0;
         if (fits && raise_smem_limit(fh, smem) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fh, PCG_THREADS, smem) == cudaSuccess && per * sms >= g) {
@@ -3585,6 +3693,8 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             global_halo = true;
             global_halo_smem = smem;
             global_halo_total = static_cast<long long>(hidx.size());
+        } else {
+            cgcg_tm_w = g_tm_rows = cgcg_lcs = 0;
         }
         cudaGetLastError();
     }
@@ -3657,6 +3767,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     dev.pds_off = cgcg_pds_off;
     dev.xs_off = cgcg_xs_off;
     dev.tm_w = cgcg_tm_w;
+    dev.tm_rows = g_tm_rows;
     dev.halo_parts = global_halo ? global_halo_parts : 0;
     dev.row_node = d_row_node;
 }

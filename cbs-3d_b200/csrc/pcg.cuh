@@ -74,6 +74,7 @@ struct PcgDev {
     CgOut* out;
     const int* cta_inst;         // batched launch: instance of each CTA (else null)
     const PcgInst* inst;         // batched launch: instance descriptors (else null)
+    int tm_rows;                 // global-vector single-reduction kernel: rows per warp in tensor memory
     int halo_parts;              // global-vector kernel with a shared-memory halo: parts per CTA, each
                                  // with its own halo (halo_ptr indexed by CTA*parts + part)
     int coef_off;                // CG-CG kernel with its warps' first rows' coefficients in shared
@@ -161,6 +162,7 @@ public:
     int cgcg_ks = 0;         // 1: the kernel reads its warps' first rows' coefficients from shared memory
     int cgcg_coef_off = 0;   // where they start
     int cgcg_kt = 0;         // >0: that many rows per thread, after the shared-memory one, read from tensor memory
+    int g_tm_rows = 0;       // rows per warp of the global-vector CG-CG kernel in tensor memory
     int cgcg_tm_w = 0;       // slots per row in tensor memory
     int cgcg_pds_off = 0;    // where the rows' diagonal starts in shared memory (0: global memory)
     int cgcg_xs_off = 0;     // ... and their pressure
