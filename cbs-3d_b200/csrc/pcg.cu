@@ -27,6 +27,7 @@
 #include <map>
 #include <mutex>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace cbs3d {
@@ -1093,8 +1094,10 @@ __device__ __forceinline__ double red4(int q, double a, double b)
 // (a fence) and the polls acquire, for kernels that exchange vectors by plain
 // stores.
 constexpr int REC_STRIDE = 8;    // TagVals per record: one 128-byte line
-template <int NT, bool ORDERED, bool MX>
-__device__ __forceinline__ void tag_allreduce_publish(const TagComm& c, int phase, const double (&v)[4])
+// Sums (and with MX the maximum) of the CTA: every lane of warp 0 returns
+// value lane/8; send() is called there.
+template <int NT, bool MX, typename F>
+__device__ __forceinline__ void cta_reduce4(const double (&v)[4], F&& send)
 {
     constexpr int NW = NT / 32;
     static_assert(NW == 8 || NW == 16, "warps per CTA");
@@ -1119,9 +1122,16 @@ __device__ __forceinline__ void tag_allreduce_publish(const TagComm& c, int phas
         if (NW == 16) x = red4<MX>(q, x, sm[q][(lane & 7) + 8]);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) x = red4<MX>(q, x, __shfl_xor_sync(0xffffffffu, x, o));
-        if (ORDERED) __threadfence();
-        if ((lane & 7) == 0) st_tag(c.rec + ((phase & 1) * c.G + c.b) * REC_STRIDE + q, x, c.tag(phase));
+        send(q, lane & 7, x);
     }
+}
+template <int NT, bool ORDERED, bool MX>
+__device__ __forceinline__ void tag_allreduce_publish(const TagComm& c, int phase, const double (&v)[4])
+{
+    cta_reduce4<NT, MX>(v, [&](int q, int j, double x) {
+        if (ORDERED) __threadfence();
+        if (j == 0) st_tag(c.rec + ((phase & 1) * c.G + c.b) * REC_STRIDE + q, x, c.tag(phase));
+    });
 }
 
 // Wait: thread t polls value t%4 of CTAs t/4, t/4 + NT/4, ...; lanes, then
@@ -1233,6 +1243,56 @@ struct StopTest {
     {
         return cg_converged(test, sqrt(rr) / init, mx, rtol, atol);
     }
+};
+
+// ------------------------------------------------------ cluster exchange
+// Meshes whose rows fit one thread-block cluster exchange through the SMs'
+// shared memory instead of L2: st.async writes a value into another CTA and
+// counts its bytes on that CTA's mbarrier, so one wait on the CTA's own
+// mbarrier covers the partial sums of every CTA and every neighbour value.
+// Two mbarriers and two sets of buffers alternate by the exchange's parity,
+// under the same rule as the tagged records.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async_f64(uint32_t addr, double v, uint32_t bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// This CTA's side of a cluster's exchange.  In shared memory: two mbarriers
+// and 2 x 16 x 4 partial sums.
+constexpr int CLUSTER_MAX = 16;
+struct ClusterShared {
+    unsigned long long bar[2];
+    double part[2][CLUSTER_MAX][4];
 };
 
 // ---------------------------------------------- tensor memory as storage
@@ -1695,7 +1755,7 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
 // KT > 0: the coefficients of each thread's rows KS .. KS+KT-1 live in TMEM
 // for the solve (D.tm_w slots per row, zero-padded past the slice's width);
 // `tm` is the CTA's TMEM base address (0 when KT = 0).
-template <int RMAX, bool BATCH, int NT, int KS, int KT>
+template <int RMAX, bool BATCH, int NT, int KS, int KT, bool CL>
 __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsigned long long epoch)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1723,10 +1783,34 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     for (int k = threadIdx.x; k < nr; k += NT) {
         const int2 e = D.rem[q0 + k];
         const uint8_t f = D.nflag[e.x];
-        rgi[k] = e.x;
+        if (!CL) rgi[k] = e.x;
         rhp[k] = (unsigned short)e.y;
         dzh[k] = (f & 1) && !(f & 4) ? (g.precond ? 1.0 / D.pdiag[e.x] : 1.0) : 0.0;
         sh[k] = 0.0;
+    }
+    // CL: the exchange through the cluster's shared memory.  cwx: 2 x rem_max
+    // values of the remote entries, as their owners push them; cwo: the own
+    // rows' value; cpu, cpl: where each pushed value goes (in the consumer's
+    // first buffer) and consumer << 12 | own row.
+    static_assert(!CL || RMAX * NT <= 4096, "own rows in 12 bits");
+    __shared__ ClusterShared cs;
+    double* cwx = reinterpret_cast<double*>(smem_raw + D.cl_off);
+    double* cwo = cwx + 2 * D.rem_max;
+    uint32_t* cpu = reinterpret_cast<uint32_t*>(cwo + RMAX * NT);
+    unsigned short* cpl = reinterpret_cast<unsigned short*>(cpu + D.push_max);
+    int npush = 0;
+    if constexpr (CL) {
+        const int p0 = D.push_ptr[b];
+        npush = D.push_ptr[b + 1] - p0;
+        for (int k = threadIdx.x; k < npush; k += NT) {
+            const int2 e = D.push[p0 + k];     // own row, consumer << 16 | entry
+            cpu[k] = cluster_addr(smem_addr(cwx + (e.y & 0xffff)), e.y >> 16);
+            cpl[k] = (unsigned short)(e.x | (e.y >> 16) << 12);
+        }
+        for (int k = threadIdx.x; k < 2 * CLUSTER_MAX * 4; k += NT) (&cs.part[0][0][0])[k] = 0.0;
+        if (threadIdx.x < 2) mbar_init(smem_addr(&cs.bar[threadIdx.x]));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        cluster_sync();          // every CTA is there, its mbarriers ready
     }
     // KS = 1: the coefficients of every warp's first row (the CTA's first
     // NT/32 slices, its leading slots) copied once into shared memory and
@@ -1780,7 +1864,11 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
                : D.xs_off ? reinterpret_cast<double*>(smem_raw + D.xs_off) + threadIdx.x : D.pres + row0;
     double* ps = PM ? D.pA + row0 : nullptr;
     // slots per round (measured at four rows per thread: 2 rather than 4)
-    constexpr int CH = RMAX >= 3 ? 2 : 8;
+    constexpr int CH = RMAX == 2 ? 8 : 2;
+    // one row per thread: the first RW slots' coefficients and local columns
+    // in registers for the solve
+    constexpr int RW = RMAX == 1 ? 16 : 0;
+    static_assert(RMAX > 1 || (KS == 0 && KT == 0), "one row needs no other place for its coefficients");
     static_assert(KT == 0 || KS + KT <= RMAX, "TMEM rows follow the shared-memory rows");
     // rows past the tensor memory's: their coefficients stream from L2, the
     // first XW slots of one row requested together (one row's before the
@@ -1830,6 +1918,14 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         }
         tmem_wait_st();
     }
+    double vrow[RW > 0 ? RW : 1];
+    unsigned crow[RW > 0 ? RW / 2 : 1];
+    if constexpr (RW > 0) {
+#pragma unroll
+        for (int u = 0; u < RW; ++u) vrow[u] = u < wr[0] ? __ldcg(D.val + S0 + lbase[0] + 32 * u) : 0.0;
+#pragma unroll
+        for (int j = 0; j < RW / 2; ++j) crow[j] = 2 * j < wmax ? lcp[j * 32] : 0;
+    }
     double vx[KX > 0 ? XW : 1];
     auto extra_load = [&](int k) {
 #pragma unroll
@@ -1838,6 +1934,22 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     auto offdiag_all = [&](double* off) {
 #pragma unroll
         for (int k = 0; k < RMAX; ++k) off[k] = 0.0;
+        if constexpr (RW > 0) {
+#pragma unroll
+            for (int j = 0; j < RW / 2; ++j)
+                if (2 * j < wmax) {
+                    const double x0 = *reinterpret_cast<const double*>(smem_raw + (crow[j] & 0xffffu));
+                    const double x1 = *reinterpret_cast<const double*>(smem_raw + (crow[j] >> 16));
+                    off[0] = fma(vrow[2 * j], x0, off[0]);
+                    off[0] = fma(vrow[2 * j + 1], x1, off[0]);
+                }
+            for (int u = RW; u < wr[0]; ++u) {
+                const unsigned c = lcp[(u >> 1) * 32] >> (16 * (u & 1));
+                off[0] = fma(__ldcg(D.val + S0 + lbase[0] + 32 * u),
+                             *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[0]);
+            }
+            return;
+        }
         const unsigned* lc = lcp;
         for (int k0 = 0; k0 < wmax; k0 += CH, lc += CH / 2 * 32) {
             double v[RMAX][CH], x[RMAX][CH];
@@ -1918,6 +2030,11 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     // handed to use(entry, value) by collect()
     constexpr int RP = RMAX >= 8 ? 2 : RMAX;
     auto store = [&](const double (&v)[RMAX]) {
+        if constexpr (CL) {
+#pragma unroll
+            for (int k = 0; k < RMAX; ++k) cwo[k * NT + threadIdx.x] = v[k];
+            return;
+        }
         TagVal* o = D.xw + (size_t)(phase & 1) * D.N;
         const unsigned long long tg = comm.tag(phase);
 #pragma unroll
@@ -1927,6 +2044,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     double xv[RP];
     unsigned long long xt[RP];
     auto request = [&](int ph) {
+        if constexpr (CL) return;
         const TagVal* o = D.xw + (size_t)(ph & 1) * D.N;
 #pragma unroll
         for (int u = 0; u < RP; ++u) {
@@ -1936,6 +2054,10 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         }
     };
     auto collect = [&](int ph, auto&& use) -> bool {
+        if constexpr (CL) {
+            for (int e = threadIdx.x; e < nr; e += NT) use(e, cwx[(ph & 1) * D.rem_max + e]);
+            return true;
+        }
         const TagVal* o = D.xw + (size_t)(ph & 1) * D.N;
         const unsigned long long want = comm.tag(ph);
         bool ok = true;
@@ -1963,6 +2085,56 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         }
         return ok;
     };
+
+    // the all-reduce's two halves; MX (a tag) also takes the maximum
+    auto publish = [&](const double (&v)[4], auto mx_tag, bool values = true) {
+        constexpr bool MX = decltype(mx_tag)::value;
+        if constexpr (CL) {
+            const int par = phase & 1;
+            const uint32_t bar = smem_addr(&cs.bar[par]);
+            if (threadIdx.x == NT - 1) mbar_expect(bar, 32u * G + (values ? 8u * nr : 0u));
+            cta_reduce4<NT, MX>(v, [&](int q, int j, double x) {
+                const uint32_t at = smem_addr(&cs.part[par][b][q]);
+                for (int c = j; c < G; c += 8) st_async_f64(cluster_addr(at, c), x, cluster_addr(bar, c));
+            });
+            // the own rows' values (visible since the reduction's barrier)
+            if (values) {
+                const uint32_t shift = 8u * par * D.rem_max;
+                for (int k = threadIdx.x; k < npush; k += NT) {
+                    const uint32_t e = cpl[k];
+                    st_async_f64(cpu[k] + shift, cwo[e & 0xfffu], cluster_addr(bar, e >> 12));
+                }
+            }
+        } else {
+            tag_allreduce_publish<NT, false, MX>(comm, phase, v);
+        }
+    };
+    auto wait = [&](double (&o)[4], bool ok, auto mx_tag, auto&& all_in) -> bool {
+        constexpr bool MX = decltype(mx_tag)::value;
+        if constexpr (CL) {
+            const int par = phase & 1;
+            const uint32_t bar = smem_addr(&cs.bar[par]);
+            SpinLimit lim;
+            while (!mbar_try_wait(bar, (phase >> 1) & 1))
+                if (lim.expired(comm.status)) { ok = false; break; }
+            const int q = lane & 3;
+            double a0 = cs.part[par][lane >> 2][q], a1 = cs.part[par][(lane >> 2) + 8][q];
+#pragma unroll
+            for (int d = 16; d >= 4; d >>= 1) {
+                a0 = red4<MX>(q, a0, __shfl_xor_sync(0xffffffffu, a0, d));
+                a1 = red4<MX>(q, a1, __shfl_xor_sync(0xffffffffu, a1, d));
+            }
+            a0 = red4<MX>(q, a0, a1);
+#pragma unroll
+            for (int p = 0; p < (MX ? 4 : 3); ++p) o[p] = __shfl_sync(0xffffffffu, a0, p);
+            if (!MX) o[3] = 0.0;
+            return __syncthreads_and(ok);
+        } else {
+            return tag_allreduce_wait<NT, false, MX>(comm, phase, o, ok, hold, all_in);
+        }
+    };
+    using Max = std::true_type;
+    using Sums = std::false_type;
 
     // ---- phase 0a: r0 = b - A x0 (constraints as the reference); partials:
     // invalid diagonals, non-finite residuals, (r,r), max|r|
@@ -2008,8 +2180,8 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
             if (own[k] & FREE) D.pres[row0 + k * NT] = XM ? xs[k * NT] : xr[XM ? 0 : k];
     };
     store(r);
-    tag_allreduce_publish<NT, false, true>(comm, phase, acc);
-    if (!tag_allreduce_wait<NT, false, true>(comm, phase, t, true, hold, [&] { request(phase); })) return;
+    publish(acc, Max());
+    if (!wait(t, true, Max(), [&] { request(phase); })) return;
     const double init = sqrt(t[2]);
     if (init <= 1.0e-300) { cg_finish(D, g, 0, 1, init, init, 0.0, t[3]); return; }
     if (cg_converged(g.conv_test, 1.0, t[3], g.rel_tol, g.abs_tol)) { cg_finish(D, g, 0, 1, init, init, 1.0, t[3]); return; }
@@ -2038,8 +2210,8 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         acc[1] = fma(zi, w[k], acc[1]);
     }
     store(w);
-    tag_allreduce_publish<NT, false, false>(comm, phase, acc);
-    if (!tag_allreduce_wait<NT, false, false>(comm, phase, t, got, hold, [&] { request(phase); })) return;
+    publish(acc, Sums());
+    if (!wait(t, got, Sums(), [&] { request(phase); })) return;
     double gam = t[0];
     if (gam <= 1.0e-300 || !isfinite(gam)) { if (b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 3, ST_PCG, 0, R_PCG_RZ0); return; }
     double den = t[1], alpha = gam / den, beta = 0.0, rr = init * init, mx = 0.0;
@@ -2052,8 +2224,8 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         for (int k = 0; k < RMAX; ++k)
             if (own[k] & FREE) m[3] = max_bits(m[3], fabs(r[k]));
         ++phase;
-        tag_allreduce_publish<NT, false, true>(comm, phase, m);
-        const bool ok = tag_allreduce_wait<NT, false, true>(comm, phase, o, true, hold, [] {});
+        publish(m, Max(), false);
+        const bool ok = wait(o, true, Max(), [] {});
         mx = o[3];
         return ok;
     };
@@ -2105,13 +2277,13 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
             }
         };
         if (!stop.needs_max()) {
-            tag_allreduce_publish<NT, false, false>(comm, phase, acc);
+            publish(acc, Sums());
             update_x();
-            got = tag_allreduce_wait<NT, false, false>(comm, phase, t, got, hold, [&] { request(phase); });
+            got = wait(t, got, Sums(), [&] { request(phase); });
         } else {
-            tag_allreduce_publish<NT, false, true>(comm, phase, acc);
+            publish(acc, Max());
             update_x();
-            got = tag_allreduce_wait<NT, false, true>(comm, phase, t, got, hold, [&] { request(phase); });
+            got = wait(t, got, Max(), [&] { request(phase); });
         }
         if (!got) { store_x(); return; }
         rr = t[2];
@@ -2147,13 +2319,13 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 // tensor memory before the solve and returns it after; every exit of the
 // body (converged, an error status, a timed-out wait) is CTA-uniform and
 // comes back here, so the memory is freed on every path.
-template <int RMAX, bool BATCH, int NT, int KS = 0, int KT = 0>
+template <int RMAX, bool BATCH, int NT, int KS = 0, int KT = 0, bool CL = false>
 __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
 {
     unsigned long long epoch;
     if (!tag_begin<BATCH>(D, epoch)) return;
     if constexpr (KT == 0) {
-        pcg64c_body<RMAX, BATCH, NT, KS, 0>(D, 0u, epoch);
+        pcg64c_body<RMAX, BATCH, NT, KS, 0, CL>(D, 0u, epoch);
     } else {
         static_assert(NT == 512 && !BATCH, "TMEM rows: one CTA per SM, single system");
         __shared__ uint32_t s_tm;
@@ -2163,12 +2335,15 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
         __syncthreads();
         tmem_fence_after_sync();
         const uint32_t tm = s_tm;
-        pcg64c_body<RMAX, BATCH, NT, KS, KT>(D, tm, epoch);
+        pcg64c_body<RMAX, BATCH, NT, KS, KT, CL>(D, tm, epoch);
         tmem_fence_before_sync();
         __syncthreads();
         tmem_fence_after_sync();
         if (w0) tmem_free_all(tm);
     }
+    // no CTA leaves while another may still write into its shared memory
+    // (every wait before this one is bounded, so all of them get here)
+    if constexpr (CL) cluster_sync();
     tag_end<BATCH>(D, epoch);
 }
 
@@ -3205,6 +3380,28 @@ struct RemoteLists {
     }
 };
 
+// What each CTA of a cluster pushes to the others: (own row, consumer << 16 |
+// entry), from the remote lists of CTAs whose rows start at row0[c].
+void push_lists(const RemoteLists& r, const std::vector<int>& row0, std::vector<int>& ptr, std::vector<int2>& push, int& most)
+{
+    const int G = static_cast<int>(row0.size()) - 1;
+    std::vector<std::vector<int2>> of(static_cast<size_t>(G));
+    for (int c = 0; c < G; ++c)
+        for (int e = r.ptr[static_cast<size_t>(c)]; e < r.ptr[static_cast<size_t>(c) + 1]; ++e) {
+            const int row = r.rem[static_cast<size_t>(e)].x;
+            const int o = static_cast<int>(std::upper_bound(row0.begin(), row0.end(), row) - row0.begin()) - 1;
+            of[static_cast<size_t>(o)].push_back(make_int2(row - row0[static_cast<size_t>(o)], c << 16 | (e - r.ptr[static_cast<size_t>(c)])));
+        }
+    ptr.assign(1, 0);
+    push.clear();
+    most = 0;
+    for (auto& v : of) {
+        push.insert(push.end(), v.begin(), v.end());
+        ptr.push_back(static_cast<int>(push.size()));
+        most = std::max(most, static_cast<int>(v.size()));
+    }
+}
+
 // k_pcg64c's dynamic shared memory: the halo's z, the remote entries (r, s,
 // inverse diagonal, row, place), then the local columns at lcs_off
 size_t cgcg_lcs_off(int hmax, int rem_max)
@@ -3225,7 +3422,7 @@ size_t cgcg_lcs_bytes(const int* slice_w, int sb, int se, int nwarps, int ch)
 }
 // slots per round of k_pcg64c at `rmax` rows per thread, and the largest halo
 // whose byte offsets fit 16 bits
-constexpr int cgcg_round(int rmax) { return rmax >= 3 ? 2 : 8; }
+constexpr int cgcg_round(int rmax) { return rmax == 2 ? 8 : 2; }
 constexpr int CGCG_HALO_MAX = 8190;
 
 // Instantiations of the single-reduction kernels by rows per thread, batch
@@ -3256,15 +3453,15 @@ const void* fn_twolevel(int rmax)
 // The single-case kernel by rows per thread: kt > 0 with that many rows'
 // coefficients in tensor memory (every row up to four per thread, else the
 // first four), ks = 1 with the first row's in shared memory ahead of them,
-// kt = 0 with all of them streamed from L2.
+// kt = 0 with all of them streamed from L2 (one row per thread keeps them in
+// registers).
 const void* fn_cgcg_single(int rmax, int ks, int kt)
 {
     if (ks && kt)
         return rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 1, 1>)
                          : reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 1, 3>);
     if (kt)
-        return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 1>)
-             : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2>)
+        return rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2>)
              : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, false, 512, 0, 3>)
              : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 0, 4>)
              : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512, 0, 4>)
@@ -3277,6 +3474,13 @@ const void* fn_cgcg_single(int rmax, int ks, int kt)
          : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512>)
          : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512>)
                      : reinterpret_cast<const void*>(k_pcg64c<8, false, 512>);
+}
+
+// ... and the form that runs on one cluster
+const void* fn_cgcg_cluster(int rmax)
+{
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 0, true>)
+                     : reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2, true>);
 }
 
 // The batch runs 256-thread CTAs, two per SM: its instances are small and
@@ -3455,6 +3659,25 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         if (g > nslices) g = nslices > 0 ? nslices : 1;
         return g;
     };
+    // whether a cluster of `c` CTAs of a kernel can run with `bytes` of shared memory
+    auto cluster_fits = [&](const void* fk, int c, size_t bytes) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = static_cast<unsigned>(c);
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(static_cast<unsigned>(c));
+        cfg.blockDim = dim3(PCG_THREADS);
+        cfg.dynamicSmemBytes = bytes;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok = bytes <= 227 * 1024 && raise_smem_limit(fk, bytes) == cudaSuccess &&
+                        cudaFuncSetAttribute(fk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, fk, &cfg) == cudaSuccess && n >= 1;
+        cudaGetLastError();
+        return ok;
+    };
     rmax = 0;
     variant = 1;
     nblocks = grid_for(reinterpret_cast<const void*>(k_pcg64<false>));
@@ -3467,14 +3690,26 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         // single-reduction kernel's partition, have 1, 2, 4 and 8; that one
         // itself up to six (beyond, the global-vector kernel is as fast:
         // 76^3 22.0 us per iteration against 25.4 with eight rows)
-        const int pow2[4] = {1, 2, 4, 8}, upto6[6] = {1, 2, 3, 4, 5, 6};
-        const bool few = want == 3 || mixed || two_level;
-        for (int c = 0; c < (few ? 4 : 6) && variant == 1; ++c) {
-            const int rr = few ? pow2[c] : upto6[c];
+        struct Tiling { int rows; bool cluster; };
+        std::vector<Tiling> tilings;
+        if (want == 3 || mixed || two_level) {
+            tilings = {{1, false}, {2, false}, {4, false}, {8, false}};
+        } else {
+            // one cluster where it holds the mesh at one row per thread (16^3
+            // 2.00 us per iteration against 2.37 on the whole chip; at two
+            // rows 3.0 against 2.4, as the chip then has one row per thread)
+            if (kernel_choice == 0 && blocks_override <= 0 && nslices <= CLUSTER_MAX * nwarps) tilings.push_back({1, true});
+            for (int r = 1; r <= 6; ++r) tilings.push_back({r, false});
+        }
+        const int grid0 = nblocks;
+        for (int c = 0; c < static_cast<int>(tilings.size()) && variant == 1; ++c) {
+            const int rr = tilings[static_cast<size_t>(c)].rows;
+            const bool cl = tilings[static_cast<size_t>(c)].cluster;
             const void* fn = want == 4 ? fn_cgcg_single(rr, 0, 0) : hc3[c];
             int per_sm = 0;
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, 0));
             int g = want == 4 ? sms : sms * (per_sm < 2 ? per_sm : 2);
+            if (cl) g = (nslices + nwarps * rr - 1) / (nwarps * rr);
             if (blocks_override > 0 && blocks_override < g) g = blocks_override;
             if (g > nslices) g = nslices > 0 ? nslices : 1;
             const int per_cta = (nslices + g - 1) / g;
@@ -3518,6 +3753,20 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             const size_t smem = want == 4 ? cgcg_lcs_off(hmax, remote.most) + lcsb
                                           : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
             if (smem > (want == 4 ? 220 : 200) * 1024) continue;
+            std::vector<int> pptr;
+            std::vector<int2> push;
+            int pmost = 0;
+            cluster = 0;
+            size_t cl_off = 0, cl_smem = 0;
+            if (cl) {
+                std::vector<int> row0;
+                for (int bb = 0; bb <= g; ++bb) row0.push_back(32 * static_cast<int>(static_cast<long long>(bb) * nslices / g));
+                push_lists(remote, row0, pptr, push, pmost);
+                cl_off = (smem + 15) & ~static_cast<size_t>(15);
+                cl_smem = cl_off + static_cast<size_t>(remote.most) * 16 + static_cast<size_t>(rr) * nt * 8 + static_cast<size_t>(pmost) * 6;
+                if (cluster_fits(fn_cgcg_cluster(rr), g, cl_smem + static_cast<size_t>(rr) * nt * 8 + 16)) cluster = g;
+                else continue;
+            }
             CUDA_OK(raise_smem_limit(fn, smem));
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, smem));
             if (per_sm * sms < g) continue;
@@ -3536,7 +3785,9 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             // SM would wait for the first to finish.
             cgcg_ks = cgcg_kt = 0;
             cgcg_coef_off = cgcg_tm_w = 0;
+            if (cluster) cgcg_smem = cl_smem;
             auto resident = [&](int ks, int kt, size_t bytes) {
+                if (cluster) return cluster_fits(fn_cgcg_cluster(rr), g, bytes);
                 const void* fk = fn_cgcg_single(rr, ks, kt);
                 int per2 = 0;
                 const bool ok = bytes <= 227 * 1024 && raise_smem_limit(fk, bytes) == cudaSuccess &&
@@ -3565,8 +3816,14 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                         cgcg_coef_off = static_cast<int>(off);
                     }
                 }
-                const int kt = std::min(rr, 4);
-                if (!cgcg_ks && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
+                const int kt = rr == 1 ? 0 : std::min(rr, 4);
+                if (!cgcg_ks && kt > 0 && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
+                else if (cluster && kt > 0) {   // its rows are too wide for tensor memory
+                    variant = 1;
+                    cluster = 0;
+                    nblocks = grid0;
+                    continue;
+                }
                 if (cgcg_kt) cgcg_tm_w = tw;
             }
             // the rows' diagonal in shared memory (64^3: 12.05 -> 11.95 us
@@ -3609,6 +3866,14 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 CUDA_OK(cudaMemcpy(d_rem_ptr, remote.ptr.data(), remote.ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
                 if (!remote.rem.empty()) CUDA_OK(cudaMemcpy(d_rem, remote.rem.data(), remote.rem.size() * sizeof(int2), cudaMemcpyHostToDevice));
                 CUDA_OK(cudaMemcpy(d_own, remote.own.data(), remote.own.size() * sizeof(int), cudaMemcpyHostToDevice));
+                if (cluster) {
+                    cgcg_cl_off = static_cast<int>(cl_off);
+                    dev_push_max = pmost;
+                    d_push_ptr = dalloc<int>(pptr.size());
+                    d_push = dalloc<int2>(push.size());
+                    CUDA_OK(cudaMemcpy(d_push_ptr, pptr.data(), pptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+                    if (!push.empty()) CUDA_OK(cudaMemcpy(d_push, push.data(), push.size() * sizeof(int2), cudaMemcpyHostToDevice));
+                }
             }
             if (mixed && want == 4) {
                 const void* mc[4] = {fn_mixed<false, 512>(1), fn_mixed<false, 512>(2), fn_mixed<false, 512>(4),
@@ -3761,6 +4026,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     dev.part = d_part; dev.bar = d_bar; dev.status = d_status; dev.out = d_out;
     dev.halo_ptr = d_halo_ptr; dev.halo_idx = d_halo_idx; dev.lcol = d_lcol; dev.halo_max = dev_halo_max;
     dev.rec = d_rec; dev.xw = d_xw; dev.epoch = d_epoch;
+    dev.push_ptr = d_push_ptr; dev.push = d_push; dev.push_max = dev_push_max; dev.cl_off = cgcg_cl_off;
     dev.rem_ptr = d_rem_ptr; dev.rem = d_rem; dev.own = d_own; dev.rem_max = dev_rem_max;
     dev.lcs_off = cgcg_lcs;
     dev.coef_off = cgcg_coef_off;
@@ -3782,13 +4048,13 @@ void PcgEngine::release()
     mg_ready = false;
     void* ptrs[] = {d_slice_off, d_slice_w, d_col, d_cptr, d_cent, d_val, d_val32, d_r, d_z, d_pA,
                     d_pB, d_q, d_f32, d_part, d_bar, d_out, d_halo_ptr, d_halo_idx, d_lcol, d_row_node,
-                    d_rec, d_xw, d_epoch, d_rem_ptr, d_rem, d_own,
+                    d_rec, d_xw, d_epoch, d_rem_ptr, d_rem, d_own, d_push_ptr, d_push,
                     d_xp, d_bp, d_dp, d_fp, d_pair_ptr, d_pair_ij, d_pair_ent, d_ac, d_nbr_ptr, d_nbr_ids, d_hown};
     for (void* p : ptrs) if (p) cudaFree(p);
     d_pair_ptr = nullptr; d_pair_ij = nullptr; d_pair_ent = nullptr; d_ac = nullptr;
     d_nbr_ptr = nullptr; d_nbr_ids = nullptr; d_hown = nullptr;
     coarse = false;
-    d_rec = d_xw = nullptr; d_epoch = nullptr; d_rem_ptr = d_own = nullptr; d_rem = nullptr;
+    d_rec = d_xw = nullptr; d_epoch = nullptr; d_rem_ptr = d_own = d_push_ptr = nullptr; d_rem = d_push = nullptr;
     d_slice_off = nullptr; d_slice_w = nullptr; d_col = nullptr; d_cptr = nullptr; d_cent = nullptr;
     d_val = nullptr; d_val32 = nullptr; d_r = d_z = d_pA = d_pB = d_q = nullptr; d_f32 = nullptr;
     d_part = nullptr; d_bar = nullptr; d_out = nullptr;
@@ -3874,7 +4140,7 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
         fn = fn_mixed<false, 512>(rmax);
         smem = mixed_smem;
     } else if (variant == 4) {
-        fn = fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
+        fn = cluster ? fn_cgcg_cluster(rmax) : fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
         smem = cgcg_smem;
     }
     CoarseDev C = cdev;
@@ -3897,7 +4163,23 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
     } else {
         mg_ready = false;
         if (ev0) CUDA_OK(cudaEventRecord(ev0, st));
-        CUDA_OK(cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(nthreads), coarse ? args2 : args, smem, st));
+        if (cluster) {
+            // one cluster: its CTAs run together by that alone
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = static_cast<unsigned>(cluster);
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(static_cast<unsigned>(cluster));
+            cfg.blockDim = dim3(nthreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            CUDA_OK(cudaLaunchKernelExC(&cfg, fn, args));
+        } else {
+            CUDA_OK(cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(nthreads), coarse ? args2 : args, smem, st));
+        }
         if (ev1) CUDA_OK(cudaEventRecord(ev1, st));
     }
     k_perm_out<<<(NP + 255) / 256, 256, 0, st>>>(D, d_xp, pres);

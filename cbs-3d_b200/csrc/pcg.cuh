@@ -68,6 +68,10 @@ struct PcgDev {
     const int* rem_ptr;          // nblocks+1: each CTA's remote halo entries in rem
     const int2* rem;             // (row position at its owner, place in this CTA's halo)
     const int* own;              // N: place of the row in its own CTA's halo (0xffff: none), bit 16: other CTAs read it
+    const int* push_ptr;         // on one cluster: what each CTA pushes to the others,
+    const int2* push;            // (own row, consumer << 16 | its remote entry),
+    int push_max;                // the most of a CTA, and the byte offset in shared
+    int cl_off;                  // memory of the exchange's buffers
     int lcs_off;                 // byte offset in shared memory of the local columns (k_pcg64c)
     int rem_max;                 // most remote entries of a CTA (shared-memory sizing)
     DevStatus* status;
@@ -174,6 +178,10 @@ public:
     int *d_rem_ptr = nullptr, *d_own = nullptr;   // remote halo entries and own rows' places (k_pcg64c)
     int2* d_rem = nullptr;
     int dev_rem_max = 0;
+    int cluster = 0;         // >0: the CG-CG kernel runs on one cluster of that many CTAs
+    int cgcg_cl_off = 0, dev_push_max = 0;
+    int* d_push_ptr = nullptr;
+    int2* d_push = nullptr;
     int cgcg_lcs = 0;        // byte offset of the CG-CG kernel's local columns
     TagVal *d_rec = nullptr, *d_xw = nullptr;
     unsigned long long* d_epoch = nullptr;

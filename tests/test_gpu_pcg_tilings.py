@@ -19,7 +19,7 @@ def _same(case, steps=2, **over):
     gpu = _gpu()
     a, b = gpu.Context(case, pcg_kernel=4, **over), gpu.Context(case, pcg_kernel=5, **over)
     sa, sb = a.step(steps), b.step(steps)
-    assert sa.pcg_kernel == 9 and sb.pcg_kernel == 8
+    assert sa.pcg_kernel in (4, 9) and sb.pcg_kernel == 8
     assert sa.cg_iterations_total == sb.cg_iterations_total
     assert sa.cg.final_max_abs == sb.cg.final_max_abs and sa.cg.final_l2 == sb.cg.final_l2
     for x, y in zip(a.fields(), b.fields()):
@@ -73,3 +73,31 @@ def test_global_vector_kernel_rows_in_tensor_memory():
         assert b.step(2).pcg_kernel == 8
         assert rel_l2(b.fields()[1], a.fields()[1]) <= 1e-8
         b.close()
+
+
+# one CTA; two; a few; the largest cluster (16 CTAs, one row per thread)
+@pytest.mark.parametrize("n,ctas", [(2, 1), (7, 1), (8, 2), (13, 6), (19, 16)])
+def test_cluster_matches_the_grid_of_the_same_ctas(n, ctas):
+    """A mesh that fits one thread-block cluster is solved there, exchanging
+    through shared memory; a grid of as many CTAs that exchanges through L2
+    makes the same sums in the same order."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(n, re=400.0, ntime=10 ** 6, jitter=0.15 if n > 2 else 0.0, seed=1234)
+    a, b = gpu.Context(case), gpu.Context(case, pcg_kernel=4, pcg_blocks=ctas)
+    sa, sb = a.step(3), b.step(3)
+    assert sa.cg_iterations_total == sb.cg_iterations_total
+    assert sa.cg.final_max_abs == sb.cg.final_max_abs
+    for x, y in zip(a.fields(), b.fields()):
+        assert bitwise(x, y)
+
+
+def test_cluster_with_fixed_and_inactive_rows():
+    from cbs3d import cases
+    gpu = _gpu()
+    for case, ctas in ((cases.channel(21, 5, 6, ntime=10 ** 6), 2), (cases.cht_slab(17, 6, 3, 5, ntime=10 ** 6), 3)):
+        a, b = gpu.Context(case), gpu.Context(case, pcg_kernel=4, pcg_blocks=ctas)
+        a.step(2)
+        b.step(2)
+        for x, y in zip(a.fields(), b.fields()):
+            assert bitwise(x, y)
