@@ -1779,7 +1779,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     unsigned short* rhp = reinterpret_cast<unsigned short*>(rgi + D.rem_max);   // ... and places in vh
     // the own rows' diagonal, kept in shared memory for the solve where the
     // engine sized it so
-    double* pds = NT == 512 && !BATCH && D.pds_off ? reinterpret_cast<double*>(smem_raw + D.pds_off) : nullptr;
+    double* pds = NT == 512 && D.pds_off ? reinterpret_cast<double*>(smem_raw + D.pds_off) : nullptr;
     for (int k = threadIdx.x; k < nr; k += NT) {
         const int2 e = D.rem[q0 + k];
         const uint8_t f = D.nflag[e.x];
@@ -2327,7 +2327,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
     if constexpr (KT == 0) {
         pcg64c_body<RMAX, BATCH, NT, KS, 0, CL>(D, 0u, epoch);
     } else {
-        static_assert(NT == 512 && !BATCH, "TMEM rows: one CTA per SM, single system");
+        static_assert(NT == 512, "TMEM rows: one CTA per SM");
         __shared__ uint32_t s_tm;
         const bool w0 = (threadIdx.x >> 5) == 0;
         if (w0) tmem_alloc_all(&s_tm);
@@ -3476,6 +3476,17 @@ const void* fn_cgcg_single(int rmax, int ks, int kt)
                      : reinterpret_cast<const void*>(k_pcg64c<8, false, 512>);
 }
 
+// ... of the batch, one 512-thread CTA per SM
+const void* fn_cgcg_batch512(int rmax)
+{
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, true, 512>)
+         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, true, 512, 0, 2>)
+         : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, true, 512, 0, 3>)
+         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, true, 512, 0, 4>)
+         : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, true, 512, 0, 4>)
+         : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, true, 512, 0, 4>)
+                     : reinterpret_cast<const void*>(k_pcg64c<8, true, 512, 0, 4>);
+}
 // ... and the form that runs on one cluster
 const void* fn_cgcg_cluster(int rmax)
 {
@@ -3483,8 +3494,8 @@ const void* fn_cgcg_cluster(int rmax)
                      : reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2, true>);
 }
 
-// The batch runs 256-thread CTAs, two per SM: its instances are small and
-// many, and more, smaller CTAs spread them better.
+// The mixed batch, and tilings whose 512-thread CTAs do not fit, run
+// 256-thread CTAs, two per SM, with their coefficients streamed from L2.
 constexpr int BATCH_THREADS = 256;
 
 }  // namespace
@@ -4269,7 +4280,7 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
     mixed = mixed_mode;
     const size_t K = mem.size();
     CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    gmax = 2 * sms;   // two BATCH_THREADS CTAs per SM
+    gmax = 2 * sms;   // the most CTAs of a wave (two of BATCH_THREADS per SM)
     slice0.assign(K, 0); nsl.assign(K, 0); N_k.assign(K, 0);
     slot0.assign(K, 0); nslot.assign(K, 0);
     nslices = 0; nslots = 0;
@@ -4372,12 +4383,21 @@ void PcgBatch::free_waves()
 
 bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
 {
+    // One 512-thread CTA per SM with the coefficients in tensor memory (one
+    // row per thread: in registers), else two 256-thread CTAs per SM.  12
+    // cavities of 10..32 hexes per side, two steps: 10.2 -> 5.7 ms.
+    return (!mixed && plan_threads(p, 512, why)) || plan_threads(p, BATCH_THREADS, why);
+}
+
+bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, std::string* why)
+{
+    const int gmax = nt == 512 ? sms : 2 * sms, nwarps = nt / 32;
     if (p.rmax != 1 && p.rmax != 2 && p.rmax != 4 && p.rmax != 8) {
         if (why) *why = "rows per thread must be 1, 2, 4 or 8";
         return false;
     }
     const int K = static_cast<int>(mem.size());
-    const int cap = (BATCH_THREADS / 32) * p.rmax;   // slices one CTA holds in registers
+    const int cap = nwarps * p.rmax;   // slices one CTA holds in registers
     std::vector<int> minc(static_cast<size_t>(K));
     for (int k = 0; k < K; ++k) {
         minc[static_cast<size_t>(k)] = std::max(1, (nsl[static_cast<size_t>(k)] + cap - 1) / cap);
@@ -4412,6 +4432,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         std::vector<int2> rem;
         int rmost = 0;
         size_t lcsb = 0;
+        int rows = 1;            // rows per thread of the wave's kernel
         std::vector<PcgInst> inst;
     };
     std::vector<HostWave> hw(packs.size());
@@ -4439,6 +4460,15 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
             }
         }
         H.G = tot;
+        if (nt == 512) {
+            // the fewest rows per thread that hold every CTA's slices
+            int most = 1;
+            for (size_t j = 0; j < mk.size(); ++j) most = std::max(most, (nsl[static_cast<size_t>(mk[j])] + G[j] - 1) / G[j]);
+            H.rows = (most + nwarps - 1) / nwarps;
+            if (H.rows > 6) H.rows = 8;
+        } else {
+            H.rows = p.rmax;
+        }
         H.hptr.push_back(0);
         RemoteLists remote(0);
         remote.own.swap(own);   // the rows of all waves, each in one of them
@@ -4455,8 +4485,8 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
             I.rel_tol = mem[static_cast<size_t>(k)].m->p.relToler;
             I.abs_tol = mem[static_cast<size_t>(k)].m->p.absToler;
             I.bar = d_bar + 4 * k;
-            I.part = d_part + static_cast<size_t>(k) * static_cast<size_t>(gmax) * 16;
-            I.rec = d_rec + static_cast<size_t>(k) * static_cast<size_t>(gmax) * 2 * REC_STRIDE;
+            I.part = d_part + static_cast<size_t>(k) * static_cast<size_t>(this->gmax) * 16;
+            I.rec = d_rec + static_cast<size_t>(k) * static_cast<size_t>(this->gmax) * 2 * REC_STRIDE;
             I.epoch = d_epoch + k;
             I.status = mem[static_cast<size_t>(k)].d_status;
             I.out = d_out + k;
@@ -4483,7 +4513,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
                 H.hmax = std::max(H.hmax, static_cast<int>(cols.size()));
                 H.smax = std::max(H.smax, a1 - a0);
                 remote.add_cta(sb * 32, se * 32, cols);
-                H.lcsb = std::max(H.lcsb, cgcg_lcs_bytes(h_slice_w.data(), sb, se, BATCH_THREADS / 32, cgcg_round(p.rmax)));
+                H.lcsb = std::max(H.lcsb, cgcg_lcs_bytes(h_slice_w.data(), sb, se, nwarps, cgcg_round(H.rows)));
             }
             cta += G[j];
         }
@@ -4497,7 +4527,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
     for (size_t w = 0; w < hw.size(); ++w) {
         const HostWave& H = hw[w];
         Wave& W = nw[w];
-        W.G = H.G; W.rmax = p.rmax;
+        W.G = H.G; W.rmax = H.rows; W.threads = nt;
         const size_t s64 = cgcg_lcs_off(H.hmax + 1, H.rmost) + H.lcsb;
         const size_t s32 = static_cast<size_t>(H.hmax) * 16 + static_cast<size_t>(H.smax) * 6 + 16;
         auto fits = [&](const void* fn, size_t smem) {
@@ -4507,13 +4537,36 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
                 return false;
             }
             int per = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, BATCH_THREADS, smem) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, nt, smem) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
             }
             return per * sms >= H.G;
         };
-        if (mixed && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
+        if (nt == 512) {
+            // the slots of a row in tensor memory padded to the wave's widest
+            int wmx = 0;
+            for (const PcgInst& I : H.inst)
+                for (int q = I.s0; q < I.s1; ++q) wmx = std::max(wmx, h_slice_w[static_cast<size_t>(q)]);
+            const int ch = cgcg_round(H.rows), tw = (wmx + ch - 1) / ch * ch;
+            W.fn = fn_cgcg_batch512(H.rows);
+            W.smem = s64;
+            if (H.hmax > CGCG_HALO_MAX || (H.rows > 1 && std::min(H.rows, 4) * tw > 64) || !fits(W.fn, s64)) {
+                if (why) *why = "a wave does not fit co-resident at this tiling";
+                return false;
+            }
+            W.tm_w = tw;
+            // the rows' diagonal, and their pressure where the kernel keeps it
+            // in memory, behind that
+            for (int what = 0; what < 2; ++what) {
+                if (what == 1 && !(H.rows == 3 || H.rows > 4)) continue;
+                const size_t off = (W.smem + 15) & ~static_cast<size_t>(15), with = off + static_cast<size_t>(H.rows) * nt * 8;
+                if (!fits(W.fn, with)) continue;
+                (what ? W.xs_off : W.pds_off) = static_cast<int>(off);
+                W.smem = with;
+            }
+        }
+        else if (mixed && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
         else if (H.hmax <= CGCG_HALO_MAX && fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
         else {
             if (why) *why = "a wave does not fit co-resident at this tiling";
@@ -4549,6 +4602,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
         W.dev.rem_ptr = W.d_rptr;
         W.dev.rem = W.d_rem;
         W.dev.rem_max = H.rmost;
+        W.dev.tm_w = W.tm_w; W.dev.pds_off = W.pds_off; W.dev.xs_off = W.xs_off;
         if (!W.mixed) {
             W.dev.halo_max = H.hmax + 1;   // the spare place
             W.dev.lcs_off = static_cast<int>(cgcg_lcs_off(H.hmax + 1, H.rmost));
@@ -4603,7 +4657,7 @@ void PcgBatch::solve(cudaStream_t st)
     CUDA_OK(cudaMemsetAsync(d_out, 0, mem.size() * sizeof(CgOut), st));
     for (Wave& W : waves) {
         void* args[] = {&W.dev};
-        CUDA_OK(cudaLaunchCooperativeKernel(W.fn, dim3(static_cast<unsigned>(W.G)), dim3(BATCH_THREADS), args, W.smem, st));
+        CUDA_OK(cudaLaunchCooperativeKernel(W.fn, dim3(static_cast<unsigned>(W.G)), dim3(static_cast<unsigned>(W.threads)), args, W.smem, st));
     }
 }
 

@@ -252,8 +252,9 @@ public:
     bool mixed_any = false;      // some wave runs the mixed-precision kernel
 
 private:
+    bool plan_threads(const PcgBatchPlan& p, int nt, std::string* why);
     struct Wave {
-        int G = 0, rmax = 4;
+        int G = 0, rmax = 4, threads = 0, tm_w = 0, pds_off = 0, xs_off = 0;
         bool mixed = false;
         size_t smem = 0;
         const void* fn = nullptr;

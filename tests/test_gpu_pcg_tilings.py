@@ -101,3 +101,22 @@ def test_cluster_with_fixed_and_inactive_rows():
         b.step(2)
         for x, y in zip(a.fields(), b.fields()):
             assert bitwise(x, y)
+
+
+@pytest.mark.parametrize("rows,spread", [(1, True), (4, False), (8, False)])
+def test_batch_tilings_with_a_large_instance(rows, spread):
+    """Waves of 512-thread CTAs at one, several and the most rows per thread
+    (a tiling whose CTAs do not fit takes the 256-thread kernels): every
+    instance as on its own, to the solves' tolerance."""
+    from cbs3d import cases
+    gpu = _gpu()
+    cs = [cases.cavity(n, re=100.0, ntime=10 ** 6) for n in (30, 5, 14)]
+    b = gpu.Batch(cs, autotune=False, rows_per_thread=rows, spread=spread)
+    bst, _ = b.step(2)
+    for i, c in enumerate(cs):
+        x = gpu.Context(c)
+        st = x.step(2)
+        assert abs(bst[i].cg.iterations - st.cg.iterations) <= 2
+        for p, q in zip(b.fields(i)[:2], x.fields()[:2]):
+            assert rel_l2(p, q) <= 1e-8
+        x.close()
