@@ -1030,6 +1030,10 @@ __device__ __forceinline__ void ld_tag(const TagVal* p, double& v, unsigned long
     v = __longlong_as_double(b);
 }
 
+// Slots per round of k_pcg64c's products: every row of a thread at once (at
+// four rows 2 measured as fast as 4; at two rows 2 instead of 8 took 48^3 from 4.46 to 4.12 us).
+constexpr int CGCG_ROUND = 2;
+
 // One solve's side of the exchange, for this CTA.
 struct TagComm {
     TagVal* rec;                 // 2 x G all-reduce records of REC_STRIDE
@@ -1863,8 +1867,8 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     double* xs = !XM ? nullptr
                : D.xs_off ? reinterpret_cast<double*>(smem_raw + D.xs_off) + threadIdx.x : D.pres + row0;
     double* ps = PM ? D.pA + row0 : nullptr;
-    // slots per round (measured at four rows per thread: 2 rather than 4)
-    constexpr int CH = RMAX == 2 ? 8 : 2;
+    // slots per round
+    constexpr int CH = CGCG_ROUND;
     // one row per thread: the first RW slots' coefficients and local columns
     // in registers for the solve
     constexpr int RW = RMAX == 1 ? 16 : 0;
@@ -3420,9 +3424,7 @@ size_t cgcg_lcs_bytes(const int* slice_w, int sb, int se, int nwarps, int ch)
     }
     return n;
 }
-// slots per round of k_pcg64c at `rmax` rows per thread, and the largest halo
-// whose byte offsets fit 16 bits
-constexpr int cgcg_round(int rmax) { return rmax == 2 ? 8 : 2; }
+// the largest halo whose byte offsets fit 16 bits
 constexpr int CGCG_HALO_MAX = 8190;
 
 // Instantiations of the single-reduction kernels by rows per thread, batch
@@ -3757,7 +3759,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 hmax = std::max(hmax, static_cast<int>(cols.size()));
                 smax = std::max(smax, a1 - a0);
                 remote.add_cta(sb * 32, se * 32, hcols);
-                lcsb = std::max(lcsb, cgcg_lcs_bytes(P.slice_w.data(), sb, se, nwarps, cgcg_round(rr)));
+                lcsb = std::max(lcsb, cgcg_lcs_bytes(P.slice_w.data(), sb, se, nwarps, CGCG_ROUND));
             }
             if (!fits || (want == 4 && hmax > CGCG_HALO_MAX)) continue;
             if (want == 4) ++hmax;   // the spare place
@@ -3810,7 +3812,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (want == 4 && kernel_choice != 10) {
                 int wmx = 0;
                 for (int q = 0; q < nslices; ++q) wmx = std::max(wmx, P.slice_w[static_cast<size_t>(q)]);
-                const int chw = cgcg_round(rr), tw = (wmx + chw - 1) / chw * chw;
+                const int chw = CGCG_ROUND, tw = (wmx + chw - 1) / chw * chw;
                 if (kernel_choice == 11 && (rr == 2 || rr == 4) && tw > 0 && (rr - 1) * tw <= 64) {
                     long long cmax = 0;
                     for (int bb = 0; bb < g; ++bb) {
@@ -4513,7 +4515,7 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, std::string* why)
                 H.hmax = std::max(H.hmax, static_cast<int>(cols.size()));
                 H.smax = std::max(H.smax, a1 - a0);
                 remote.add_cta(sb * 32, se * 32, cols);
-                H.lcsb = std::max(H.lcsb, cgcg_lcs_bytes(h_slice_w.data(), sb, se, nwarps, cgcg_round(H.rows)));
+                H.lcsb = std::max(H.lcsb, cgcg_lcs_bytes(h_slice_w.data(), sb, se, nwarps, CGCG_ROUND));
             }
             cta += G[j];
         }
@@ -4548,7 +4550,7 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, std::string* why)
             int wmx = 0;
             for (const PcgInst& I : H.inst)
                 for (int q = I.s0; q < I.s1; ++q) wmx = std::max(wmx, h_slice_w[static_cast<size_t>(q)]);
-            const int ch = cgcg_round(H.rows), tw = (wmx + ch - 1) / ch * ch;
+            const int ch = CGCG_ROUND, tw = (wmx + ch - 1) / ch * ch;
             W.fn = fn_cgcg_batch512(H.rows);
             W.smem = s64;
             if (H.hmax > CGCG_HALO_MAX || (H.rows > 1 && std::min(H.rows, 4) * tw > 64) || !fits(W.fn, s64)) {
