@@ -18,7 +18,9 @@
 // matvec (double-buffered p; neighbours' new p formed on the fly from z and
 // the previous p), and every CTA reduces the per-CTA partials in the same
 // fixed order, so alpha, beta and the stopping decision are identical in all
-// CTAs and reproducible run to run.
+// CTAs and reproducible run to run.  That is k_pcg64 with its variants; the
+// kernels that solves run by default (k_pcg64c, k_pcg64g, further down) take
+// the single-reduction form, one all-reduce per iteration.
 #include "pcg.cuh"
 #include "mg.cuh"
 
@@ -101,33 +103,37 @@ __global__ void k_ell_from_gstif(const double* gstif, const long long* cptr, con
     if (val32) val32[s] = (float)v;
 }
 
-// impose_pressure_constraints (src/linalg/ConjugateGradient.cpp:188-214)
-__global__ void k_impose(PcgDev D)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.NN) return;
-    const uint8_t f = D.nflag[i];
-    if (!(f & 1)) {
-        D.pres[i] = 0.0; D.rhs1[i] = 0.0; D.pdiag[i] = 0.0;
-    } else if (f & 4) {
-        D.pres[i] = D.pfix[i]; D.rhs1[i] = D.pfix[i]; D.pdiag[i] = 1.0;
-    }
-}
-
-// Node order -> row-position order of the solver's inputs, and back for the
-// pressure.  Padding positions get inactive flags and zeros.
-__global__ void k_perm_in(PcgDev D, const double* pres, const double* rhs1, const double* pdiag,
-                          const uint8_t* nflag, double* xp, double* bp, double* dp, uint8_t* fp)
+// impose_pressure_constraints (src/linalg/ConjugateGradient.cpp:188-214) on
+// the node-ordered arrays, and the solver's inputs from them in row-position
+// order (every node has one position; padding positions get inactive flags
+// and zeros).  One launch: on small meshes a step's time outside the solve is
+// its launches.
+__global__ void k_impose_perm_in(PcgDev D, double* xp, double* bp, double* dp, uint8_t* fp)
 {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= D.N) return;
     const int i = D.row_node[pos];
-    xp[pos] = i >= 0 ? pres[i] : 0.0;
-    bp[pos] = i >= 0 ? rhs1[i] : 0.0;
-    dp[pos] = i >= 0 ? pdiag[i] : 0.0;
-    fp[pos] = i >= 0 ? (uint8_t)(nflag[i] & 5) : (uint8_t)0;
+    double x = 0.0, b = 0.0, d = 0.0;
+    uint8_t f = 0;
+    if (i >= 0) {
+        f = D.nflag[i] & 5;
+        if (!(f & 1)) {
+            D.pres[i] = 0.0; D.rhs1[i] = 0.0; D.pdiag[i] = 0.0;
+        } else if (f & 4) {
+            x = b = D.pfix[i];
+            d = 1.0;
+            D.pres[i] = x; D.rhs1[i] = b; D.pdiag[i] = d;
+        } else {
+            x = D.pres[i]; b = D.rhs1[i]; d = D.pdiag[i];
+        }
+    }
+    xp[pos] = x;
+    bp[pos] = b;
+    dp[pos] = d;
+    fp[pos] = f;
 }
 
+// The pressure back to node order.
 __global__ void k_perm_out(PcgDev D, const double* xp, double* pres)
 {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3511,8 +3517,8 @@ cudaError_t pcg_raise_smem_limit(const void* fn, size_t smem) { return raise_sme
 
 int PcgEngine::launches_per_solve() const
 {
-    if (mgh) return 4 + mgh->launches_per_setup();
-    return coarse ? 6 : 4;
+    if (mgh) return 3 + mgh->launches_per_setup();
+    return coarse ? 5 : 3;
 }
 
 void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
@@ -3872,6 +3878,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             h_hidx = hidx;
             if (want == 4) {
                 dev_rem_max = remote.most;
+                rem_total = static_cast<long long>(remote.rem.size());
                 cgcg_lcs = static_cast<int>(cgcg_lcs_off(hmax, remote.most));
                 d_rem_ptr = dalloc<int>(remote.ptr.size());
                 d_rem = dalloc<int2>(remote.rem.size());
@@ -4026,7 +4033,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     }
 
     dev = PcgDev{};
-    dev.N = NP; dev.NN = N; dev.E = E; dev.nslices = nslices; dev.nblocks = nblocks;
+    dev.N = NP; dev.E = E; dev.nslices = nslices; dev.nblocks = nblocks;
     dev.slice_off = d_slice_off; dev.slice_w = d_slice_w; dev.col = d_col; dev.val = d_val;
     dev.val32 = d_val32; dev.cptr = d_cptr; dev.cent = d_cent;
     dev.nflag = d_nflag; dev.pfix = d_pfix;
@@ -4128,8 +4135,7 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
     D.pres = pres; D.rhs1 = rhs1; D.pdiag = pdiag;
     D.precond = precond; D.conv_test = conv_test; D.max_iter = max_iter;
     D.rel_tol = rel_tol; D.abs_tol = abs_tol; D.inner_tol = inner_tol;
-    k_impose<<<(N + 255) / 256, 256, 0, st>>>(D);
-    k_perm_in<<<(NP + 255) / 256, 256, 0, st>>>(D, pres, rhs1, pdiag, D.nflag, d_xp, d_bp, d_dp, d_fp);
+    k_impose_perm_in<<<(NP + 255) / 256, 256, 0, st>>>(D, d_xp, d_bp, d_dp, d_fp);
     D.pres = d_xp; D.rhs1 = d_bp; D.pdiag = d_dp; D.nflag = d_fp;
     CUDA_OK(cudaMemsetAsync(d_bar, 0, 4 * sizeof(unsigned), st));
     CUDA_OK(cudaMemsetAsync(d_out, 0, sizeof(CgOut), st));
@@ -4236,10 +4242,10 @@ size_t PcgEngine::bytes_per_iter() const
         return static_cast<size_t>(N) * 48;
     }
     if (variant == 4) {
-        // coefficient per pair entry; per node: r, w, s of the previous
-        // iteration read once for staging (24), r, s, w written (24), pressure
-        // read and written (16), pdiag read (8)
-        return static_cast<size_t>(nnz_offdiag) * 8 + static_cast<size_t>(N) * 72;
+        // coefficient per pair entry and the diagonal per node (both on chip
+        // for the solve); per remote halo entry the record of its w written
+        // and read (32)
+        return static_cast<size_t>(nnz_offdiag) * 8 + static_cast<size_t>(N) * 8 + static_cast<size_t>(rem_total) * 32;
     }
     if (variant == 3) {
         // coefficient per pair entry; per node: halo staging of z and the
@@ -4260,7 +4266,8 @@ size_t PcgEngine::bytes_per_iter() const
     // shared-memory halo the columns are 16-bit and every halo entry's z and
     // previous p are read once per iteration.
     if (global_halo && global_cgcg) {
-        // single reduction: coefficient + 16-bit column per pair entry; per
+        // single reduction: coefficient + 16-bit column per pair entry (those
+        // of the rows in tensor memory included); per
         // node r, s, w of the previous iteration, p, pressure, inverse
         // diagonal and diagonal read (56), node flag (1), p, pressure and the
         // new r, s, w written (40); per halo entry r, s, w (24) and, with
@@ -4641,16 +4648,13 @@ void PcgBatch::prepare(int k, const DevState& S, cudaStream_t st)
         k_ell_from_state<<<static_cast<unsigned>((nslot[kk] + T - 1) / T), T, 0, st>>>(
             S, d_cptr[kk], d_cent[kk], d_val + slot0[kk], d_val32 ? d_val32 + slot0[kk] : nullptr, nslot[kk]);
     PcgDev D = base;
-    D.NN = N_k[kk];
     D.nflag = mem[kk].d_nflag;
     D.pfix = mem[kk].d_pfix;
     D.pres = S.pres; D.rhs1 = S.rhs1; D.pdiag = S.pdiag;
-    k_impose<<<(N_k[kk] + T - 1) / T, T, 0, st>>>(D);
     const int p0 = slice0[kk] * 32, np = nsl[kk] * 32;
     D.N = np;
     D.row_node = d_row_node + p0;
-    k_perm_in<<<(np + T - 1) / T, T, 0, st>>>(D, S.pres, S.rhs1, S.pdiag, mem[kk].d_nflag, d_xp + p0, d_bp + p0,
-                                               d_dp + p0, d_fp + p0);
+    k_impose_perm_in<<<(np + T - 1) / T, T, 0, st>>>(D, d_xp + p0, d_bp + p0, d_dp + p0, d_fp + p0);
 }
 
 void PcgBatch::solve(cudaStream_t st)

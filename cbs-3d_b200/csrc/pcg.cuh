@@ -35,7 +35,6 @@ struct PcgInst {
 
 struct PcgDev {
     int N;                       // row positions (nslices*32); the solver's vectors use this order
-    int NN;                      // nodes (the caller's arrays)
     int E, nslices;
     int nblocks;
     int precond, conv_test, max_iter;
@@ -132,7 +131,7 @@ public:
     cbs3d_status solve(double* d_pres, double* d_rhs1, double* d_pdiag, int precond, int conv_test,
                        int max_iter, double rel_tol, double abs_tol, cudaStream_t st, bool sync,
                        cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr);
-    // impose, permute in, solver, permute out (+ the preconditioner's set-up)
+    // impose and permute in, solver, permute out (+ the preconditioner's set-up)
     int launches_per_solve() const;
     cbs3d_status read_result(cbs3d_cg_result& r, cudaStream_t st);
     // y = A x with the assembled operator (identity rows on fixed nodes).
@@ -178,6 +177,7 @@ public:
     int *d_rem_ptr = nullptr, *d_own = nullptr;   // remote halo entries and own rows' places (k_pcg64c)
     int2* d_rem = nullptr;
     int dev_rem_max = 0;
+    long long rem_total = 0;      // remote halo entries over all CTAs (k_pcg64c)
     int cluster = 0;         // >0: the CG-CG kernel runs on one cluster of that many CTAs
     int cgcg_cl_off = 0, dev_push_max = 0;
     int* d_push_ptr = nullptr;
@@ -246,8 +246,8 @@ public:
     void finish(int k, double* d_pres, cudaStream_t st);
     CgOut* out(int k) const { return d_out + k; }
     int nwaves() const { return static_cast<int>(waves.size()); }
-    // launches per step: assemble, impose, permute in and out per instance; one per wave
-    int launches_per_instance() const { return 4; }
+    // launches per step: assemble, impose and permute in, permute out per instance; one per wave
+    int launches_per_instance() const { return 3; }
     PcgBatchPlan current{};
     bool mixed_any = false;      // some wave runs the mixed-precision kernel
 
