@@ -3496,11 +3496,7 @@ const void* fn_cgcg_batch512(int rmax)
                      : reinterpret_cast<const void*>(k_pcg64c<8, true, 512, 0, 4>);
 }
 // ... and the form that runs on one cluster
-const void* fn_cgcg_cluster(int rmax)
-{
-    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 0, true>)
-                     : reinterpret_cast<const void*>(k_pcg64c<2, false, 512, 0, 2, true>);
-}
+const void* fn_cgcg_cluster() { return reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 0, true>); }
 
 // The mixed batch, and tilings whose 512-thread CTAs do not fit, run
 // 256-thread CTAs, two per SM, with their coefficients streamed from L2.
@@ -3720,7 +3716,6 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (kernel_choice == 0 && blocks_override <= 0 && nslices <= CLUSTER_MAX * nwarps) tilings.push_back({1, true});
             for (int r = 1; r <= 6; ++r) tilings.push_back({r, false});
         }
-        const int grid0 = nblocks;
         for (int c = 0; c < static_cast<int>(tilings.size()) && variant == 1; ++c) {
             const int rr = tilings[static_cast<size_t>(c)].rows;
             const bool cl = tilings[static_cast<size_t>(c)].cluster;
@@ -3783,7 +3778,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 push_lists(remote, row0, pptr, push, pmost);
                 cl_off = (smem + 15) & ~static_cast<size_t>(15);
                 cl_smem = cl_off + static_cast<size_t>(remote.most) * 16 + static_cast<size_t>(rr) * nt * 8 + static_cast<size_t>(pmost) * 6;
-                if (cluster_fits(fn_cgcg_cluster(rr), g, cl_smem + static_cast<size_t>(rr) * nt * 8 + 16)) cluster = g;
+                if (cluster_fits(fn_cgcg_cluster(), g, cl_smem + static_cast<size_t>(rr) * nt * 8 + 16)) cluster = g;
                 else continue;
             }
             CUDA_OK(raise_smem_limit(fn, smem));
@@ -3806,7 +3801,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             cgcg_coef_off = cgcg_tm_w = 0;
             if (cluster) cgcg_smem = cl_smem;
             auto resident = [&](int ks, int kt, size_t bytes) {
-                if (cluster) return cluster_fits(fn_cgcg_cluster(rr), g, bytes);
+                if (cluster) return cluster_fits(fn_cgcg_cluster(), g, bytes);
                 const void* fk = fn_cgcg_single(rr, ks, kt);
                 int per2 = 0;
                 const bool ok = bytes <= 227 * 1024 && raise_smem_limit(fk, bytes) == cudaSuccess &&
@@ -3837,12 +3832,6 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 }
                 const int kt = rr == 1 ? 0 : std::min(rr, 4);
                 if (!cgcg_ks && kt > 0 && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
-                else if (cluster && kt > 0) {   // its rows are too wide for tensor memory
-                    variant = 1;
-                    cluster = 0;
-                    nblocks = grid0;
-                    continue;
-                }
                 if (cgcg_kt) cgcg_tm_w = tw;
             }
             // the rows' diagonal in shared memory (64^3: 12.05 -> 11.95 us
@@ -4159,7 +4148,7 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
         fn = fn_mixed<false, 512>(rmax);
         smem = mixed_smem;
     } else if (variant == 4) {
-        fn = cluster ? fn_cgcg_cluster(rmax) : fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
+        fn = cluster ? fn_cgcg_cluster() : fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
         smem = cgcg_smem;
     }
     CoarseDev C = cdev;
