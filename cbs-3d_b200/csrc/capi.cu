@@ -980,6 +980,18 @@ cbs3d_status cbs3d_coarse_inverse(int device, int g, const double* a, double* ai
     }
 }
 
+cbs3d_status cbs3d_probe_pcg_partition(int nelem, int npoin, const int* intma, const int* mat_elem,
+                                       const double* coord, int ctas, cbs3d_pcg_partition* out)
+{
+    try {
+        return probe_partition(nelem, npoin, intma, mat_elem, coord, ctas, out);
+    } catch (const Error& e) {
+        return e.code;
+    } catch (const std::exception&) {
+        return CBS3D_INTERNAL;
+    }
+}
+
 cbs3d_status cbs3d_selftest_wait_timeout(int device, int* observed_status)
 {
     try {

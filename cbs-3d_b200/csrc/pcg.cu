@@ -2372,10 +2372,11 @@ __global__ void __launch_bounds__(512, 1) k_pcg64d(PcgDev D, CoarseDev C)
     const int nsl = (int)(D.slice_off[s_end] - S0);
     const int h0 = D.halo_ptr[blockIdx.x];
     const int nh = D.halo_ptr[blockIdx.x + 1] - h0;
+    const TwoLevelLayout L(D.halo_max, D.slot_max, C.nbr_max, C.G);
     double* vh = reinterpret_cast<double*>(smem_raw);
     double* dzh = vh + D.halo_max;
-    int* hidx = reinterpret_cast<int*>(dzh + D.halo_max);
-    unsigned short* lcs = reinterpret_cast<unsigned short*>(hidx + D.halo_max);
+    int* hidx = reinterpret_cast<int*>(smem_raw + L.hidx);
+    unsigned short* lcs = reinterpret_cast<unsigned short*>(smem_raw + L.lcs);
     for (int k = threadIdx.x; k < nh; k += NT) hidx[k] = D.halo_idx[h0 + k];
     for (int k = threadIdx.x; k < nsl; k += NT) lcs[k] = D.lcol[S0 + k];
     // coarse space: this CTA's rows of the coarse inverse (its own and its
@@ -2384,13 +2385,12 @@ __global__ void __launch_bounds__(512, 1) k_pcg64d(PcgDev D, CoarseDev C)
     const int GC = C.G;
     const int nb0 = C.nbr_ptr[blockIdx.x];
     const int nn = C.nbr_ptr[blockIdx.x + 1] - nb0;
-    double* ainv = reinterpret_cast<double*>(
-        (reinterpret_cast<uintptr_t>(lcs + D.slot_max) + 15) & ~static_cast<uintptr_t>(15));
+    double* ainv = reinterpret_cast<double*>(smem_raw + L.ainv);
     double* cr = ainv + (size_t)C.nbr_max * GC;
     double* cs = cr + GC;
     double* cw = cs + GC;
     double* ec = cw + GC;
-    unsigned char* hown = reinterpret_cast<unsigned char*>(ec + C.nbr_max);
+    unsigned char* hown = smem_raw + L.hown;
     __shared__ int s_own;
     __shared__ double s_ecp;   // this CTA's coarse correction of the previous iteration's z
     if (threadIdx.x == 0)
@@ -3433,6 +3433,101 @@ size_t cgcg_lcs_bytes(const int* slice_w, int sb, int se, int nwarps, int ch)
 // the largest halo whose byte offsets fit 16 bits
 constexpr int CGCG_HALO_MAX = 8190;
 
+// The rows split over g CTAs of nwarps warps: each CTA's halo (the distinct
+// columns of its slots) in the order of its places in shared memory, its
+// slots' columns as places, its remote entries, and the largest of each.
+struct Partition {
+    std::vector<int> hptr, hidx;
+    std::vector<unsigned short> lcol;
+    int hmax = 0;            // halo entries
+    long long smax = 0;      // slots
+    RemoteLists remote;
+    size_t lcsb = 0;         // bytes of k_pcg64c's padded local columns
+    bool fits = true;        // every place fits 16 bits
+    explicit Partition(size_t rows) : remote(rows) {}
+};
+Partition partition_rows(const PressurePattern& P, const std::vector<int>& colp, int g, int nwarps)
+{
+    Partition o(static_cast<size_t>(P.nslices) * 32);
+    o.hptr.assign(static_cast<size_t>(g) + 1, 0);
+    o.lcol.assign(static_cast<size_t>(P.nslots), 0);
+    std::vector<int> cols, hpos, hcols;
+    for (int bb = 0; bb < g; ++bb) {
+        const int sb = static_cast<int>(static_cast<long long>(bb) * P.nslices / g);
+        const int se = static_cast<int>(static_cast<long long>(bb + 1) * P.nslices / g);
+        const long long a0 = P.slice_off[static_cast<size_t>(sb)], a1 = P.slice_off[static_cast<size_t>(se)];
+        cols.assign(colp.begin() + a0, colp.begin() + a1);
+        std::sort(cols.begin(), cols.end());
+        cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
+        if (cols.size() > 65535) { o.fits = false; return o; }
+        for (long long t = a0; t < a1; ++t)
+            o.lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(
+                std::lower_bound(cols.begin(), cols.end(), colp[static_cast<size_t>(t)]) - cols.begin());
+        // the halo's order in shared memory: bank-spread
+        const int nh = static_cast<int>(cols.size());
+        bank_spread_halo(nh, o.lcol.data() + a0, P.slice_off.data(), P.slice_w.data(), sb, se, a0, hpos);
+        for (long long t = a0; t < a1; ++t)
+            o.lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(hpos[o.lcol[static_cast<size_t>(t)]]);
+        hcols.resize(cols.size());
+        for (int e = 0; e < nh; ++e) hcols[static_cast<size_t>(hpos[static_cast<size_t>(e)])] = cols[static_cast<size_t>(e)];
+        o.hidx.insert(o.hidx.end(), hcols.begin(), hcols.end());
+        o.hptr[static_cast<size_t>(bb) + 1] = static_cast<int>(o.hidx.size());
+        o.hmax = std::max(o.hmax, nh);
+        o.smax = std::max(o.smax, a1 - a0);
+        o.remote.add_cta(sb * 32, se * 32, hcols);
+        o.lcsb = std::max(o.lcsb, cgcg_lcs_bytes(P.slice_w.data(), sb, se, nwarps, CGCG_ROUND));
+    }
+    return o;
+}
+
+// Columns as row positions: the solver works in row-position order.
+std::vector<int> columns_by_position(const PressurePattern& P, int N)
+{
+    std::vector<int> pos_of(static_cast<size_t>(N), 0);
+    for (size_t p = 0; p < P.row_node.size(); ++p)
+        if (P.row_node[p] >= 0) pos_of[static_cast<size_t>(P.row_node[p])] = static_cast<int>(p);
+    std::vector<int> colp(static_cast<size_t>(P.nslots));
+    for (size_t t = 0; t < colp.size(); ++t) colp[t] = pos_of[static_cast<size_t>(P.col[t])];
+    return colp;
+}
+
+// Each CTA's neighbours for the two-level kernel (itself and the owners of
+// its halo entries), and every halo entry's owner as its place in that list.
+struct CoarseNeighbours {
+    std::vector<int> ptr{0}, ids;
+    std::vector<unsigned char> hown;
+    int most = 0;
+    bool fits = true;        // every place fits 8 bits
+};
+CoarseNeighbours coarse_neighbours(int nslices, const std::vector<int>& hptr, const std::vector<int>& hidx)
+{
+    CoarseNeighbours o;
+    const int G = static_cast<int>(hptr.size()) - 1;
+    std::vector<int> cta_of_slice(static_cast<size_t>(nslices), 0);
+    for (int b = 0; b < G; ++b) {
+        const int sb = static_cast<int>(static_cast<long long>(b) * nslices / G);
+        const int se = static_cast<int>(static_cast<long long>(b + 1) * nslices / G);
+        for (int q = sb; q < se; ++q) cta_of_slice[static_cast<size_t>(q)] = b;
+    }
+    o.hown.assign(hidx.size(), 0);
+    for (int b = 0; b < G; ++b) {
+        std::vector<int> l(1, b);
+        for (int k = hptr[static_cast<size_t>(b)]; k < hptr[static_cast<size_t>(b) + 1]; ++k)
+            l.push_back(cta_of_slice[static_cast<size_t>(hidx[static_cast<size_t>(k)] / 32)]);
+        std::sort(l.begin(), l.end());
+        l.erase(std::unique(l.begin(), l.end()), l.end());
+        if (l.size() > 255) { o.fits = false; return o; }
+        for (int k = hptr[static_cast<size_t>(b)]; k < hptr[static_cast<size_t>(b) + 1]; ++k) {
+            const int w = cta_of_slice[static_cast<size_t>(hidx[static_cast<size_t>(k)] / 32)];
+            o.hown[static_cast<size_t>(k)] = static_cast<unsigned char>(std::lower_bound(l.begin(), l.end(), w) - l.begin());
+        }
+        o.ids.insert(o.ids.end(), l.begin(), l.end());
+        o.ptr.push_back(static_cast<int>(o.ids.size()));
+        o.most = std::max(o.most, static_cast<int>(l.size()));
+    }
+    return o;
+}
+
 // Instantiations of the single-reduction kernels by rows per thread, batch
 // mode and CTA size.
 template <int NT>
@@ -3511,6 +3606,28 @@ void coarse_invert_launch(int g, double* a, cudaStream_t st)
 
 cudaError_t pcg_raise_smem_limit(const void* fn, size_t smem) { return raise_smem_limit(fn, smem); }
 
+cbs3d_status probe_partition(int nelem, int npoin, const int* intma, const int* mat_elem, const double* coord, int ctas,
+                             cbs3d_pcg_partition* out)
+{
+    if (nelem < 1 || npoin < 1 || !intma || ctas < 1 || !out) return CBS3D_INVALID_INPUT;
+    const std::vector<int> conn(intma, intma + 4 * static_cast<size_t>(nelem));
+    for (int v : conn)
+        if (v < 1 || v > npoin) return CBS3D_INVALID_INPUT;
+    std::vector<int> mat(static_cast<size_t>(nelem), 0), n2e_ptr, n2e;
+    if (mat_elem) mat.assign(mat_elem, mat_elem + nelem);
+    build_incidence(conn, npoin, n2e_ptr, n2e);
+    PressurePattern P;
+    build_pressure_pattern(conn, mat, npoin, n2e_ptr, n2e, P, coord);
+    const int g = std::min(ctas, P.nslices);
+    const Partition part = partition_rows(P, columns_by_position(P, npoin), g, PCG_THREADS / 32);
+    if (!part.fits) return CBS3D_INVALID_INPUT;
+    const CoarseNeighbours nb = coarse_neighbours(P.nslices, part.hptr, part.hidx);
+    const int hmax = part.hmax + 1;   // the spare place
+    *out = cbs3d_pcg_partition{g, hmax, static_cast<int>(part.smax), part.remote.most, nb.most,
+                               static_cast<long long>(TwoLevelLayout(hmax, static_cast<int>(part.smax), nb.most, g).bytes)};
+    return CBS3D_OK;
+}
+
 int PcgEngine::launches_per_solve() const
 {
     if (mgh) return 3 + mgh->launches_per_setup();
@@ -3561,28 +3678,9 @@ void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
             ptr.push_back(static_cast<int>(ent.size()));
             ij.push_back(make_int2(I, J));
         }
-    // each CTA's neighbour list: itself and the owners of its halo entries
-    std::vector<int> nptr(1, 0), nids;
-    std::vector<unsigned char> hown(h_hidx.size(), 0);
-    int nmax = 0;
-    for (int b = 0; b < G; ++b) {
-        std::vector<int> l(1, b);
-        for (int k = h_hptr[static_cast<size_t>(b)]; k < h_hptr[static_cast<size_t>(b) + 1]; ++k)
-            l.push_back(cta_of_slice[static_cast<size_t>(h_hidx[static_cast<size_t>(k)] / 32)]);
-        std::sort(l.begin(), l.end());
-        l.erase(std::unique(l.begin(), l.end()), l.end());
-        if (l.size() > 255) return;
-        for (int k = h_hptr[static_cast<size_t>(b)]; k < h_hptr[static_cast<size_t>(b) + 1]; ++k) {
-            const int o = cta_of_slice[static_cast<size_t>(h_hidx[static_cast<size_t>(k)] / 32)];
-            hown[static_cast<size_t>(k)] = static_cast<unsigned char>(std::lower_bound(l.begin(), l.end(), o) - l.begin());
-        }
-        nids.insert(nids.end(), l.begin(), l.end());
-        nptr.push_back(static_cast<int>(nids.size()));
-        nmax = std::max(nmax, static_cast<int>(l.size()));
-    }
-    const size_t base = (halo_smem + 15) & ~static_cast<size_t>(15);
-    const size_t smem = base + (static_cast<size_t>(nmax) * G + 3 * static_cast<size_t>(G) + nmax) * 8 +
-                        static_cast<size_t>(dev_halo_max) + 16;
+    const CoarseNeighbours nb = coarse_neighbours(nslices, h_hptr, h_hidx);
+    if (!nb.fits) return;
+    const size_t smem = TwoLevelLayout(dev_halo_max, dev_slot_max, nb.most, G).bytes;
     const size_t ismem = (static_cast<size_t>(G) * G + 2 * static_cast<size_t>(G)) * 8;
     const void* fn = fn_twolevel(rmax);
     int per = 0;
@@ -3597,16 +3695,16 @@ void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
     d_pair_ij = dalloc<int2>(ij.size());
     d_pair_ent = dalloc<int>(ent.size());
     d_ac = dalloc<double>(static_cast<size_t>(G) * G);
-    d_nbr_ptr = dalloc<int>(nptr.size());
-    d_nbr_ids = dalloc<int>(nids.size());
-    d_hown = dalloc<unsigned char>(hown.size());
+    d_nbr_ptr = dalloc<int>(nb.ptr.size());
+    d_nbr_ids = dalloc<int>(nb.ids.size());
+    d_hown = dalloc<unsigned char>(nb.hown.size());
     CUDA_OK(cudaMemcpy(d_pair_ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
     CUDA_OK(cudaMemcpy(d_pair_ij, ij.data(), ij.size() * sizeof(int2), cudaMemcpyHostToDevice));
     CUDA_OK(cudaMemcpy(d_pair_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_OK(cudaMemcpy(d_nbr_ptr, nptr.data(), nptr.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_OK(cudaMemcpy(d_nbr_ids, nids.data(), nids.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (!hown.empty()) CUDA_OK(cudaMemcpy(d_hown, hown.data(), hown.size(), cudaMemcpyHostToDevice));
-    cdev = CoarseDev{G, nmax, d_nbr_ptr, d_nbr_ids, d_hown, d_ac};
+    CUDA_OK(cudaMemcpy(d_nbr_ptr, nb.ptr.data(), nb.ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMemcpy(d_nbr_ids, nb.ids.data(), nb.ids.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if (!nb.hown.empty()) CUDA_OK(cudaMemcpy(d_hown, nb.hown.data(), nb.hown.size(), cudaMemcpyHostToDevice));
+    cdev = CoarseDev{G, nb.most, d_nbr_ptr, d_nbr_ids, d_hown, d_ac};
     coarse_smem = smem;
     coarse_ismem = ismem;
     coarse = true;
@@ -3628,12 +3726,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     NP = nslices * 32;
     d_row_node = dalloc<int>(P.row_node.size());
     CUDA_OK(cudaMemcpy(d_row_node, P.row_node.data(), P.row_node.size() * sizeof(int), cudaMemcpyHostToDevice));
-    // columns as row positions: the solver works in row-position order
-    std::vector<int> pos_of(static_cast<size_t>(N), 0);
-    for (size_t p = 0; p < P.row_node.size(); ++p)
-        if (P.row_node[p] >= 0) pos_of[static_cast<size_t>(P.row_node[p])] = static_cast<int>(p);
-    std::vector<int> colp(static_cast<size_t>(nslots));
-    for (size_t t = 0; t < colp.size(); ++t) colp[t] = pos_of[static_cast<size_t>(P.col[t])];
+    const std::vector<int> colp = columns_by_position(P, N);
     d_slice_off = dalloc<long long>(P.slice_off.size());
     d_slice_w = dalloc<int>(P.slice_w.size());
     d_col = dalloc<int>(static_cast<size_t>(nslots));
@@ -3728,43 +3821,13 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (g > nslices) g = nslices > 0 ? nslices : 1;
             const int per_cta = (nslices + g - 1) / g;
             if ((per_cta + nwarps - 1) / nwarps > rr) continue;
-            // halo of every CTA: distinct columns of its slot range
-            std::vector<int> hptr(static_cast<size_t>(g) + 1, 0), hidx;
-            std::vector<unsigned short> lcol(static_cast<size_t>(nslots), 0);
-            int hmax = 0;
-            long long smax = 0;
-            bool fits = true;
-            std::vector<int> cols, hpos, hcols;
-            RemoteLists remote(static_cast<size_t>(NP));
-            size_t lcsb = 0;
-            for (int bb = 0; bb < g && fits; ++bb) {
-                const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
-                const int se = static_cast<int>(static_cast<long long>(bb + 1) * nslices / g);
-                const long long a0 = P.slice_off[static_cast<size_t>(sb)], a1 = P.slice_off[static_cast<size_t>(se)];
-                cols.assign(colp.begin() + a0, colp.begin() + a1);
-                std::sort(cols.begin(), cols.end());
-                cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-                if (cols.size() > 65535) { fits = false; break; }
-                for (long long t = a0; t < a1; ++t)
-                    lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(
-                        std::lower_bound(cols.begin(), cols.end(), colp[static_cast<size_t>(t)]) - cols.begin());
-                // the halo's order in shared memory: bank-spread
-                const int nh = static_cast<int>(cols.size());
-                bank_spread_halo(nh, lcol.data() + a0, P.slice_off.data(), P.slice_w.data(), sb, se, a0, hpos);
-                for (long long t = a0; t < a1; ++t)
-                    lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(hpos[lcol[static_cast<size_t>(t)]]);
-                hcols.resize(cols.size());
-                for (int e = 0; e < nh; ++e) hcols[static_cast<size_t>(hpos[static_cast<size_t>(e)])] = cols[static_cast<size_t>(e)];
-                hidx.insert(hidx.end(), hcols.begin(), hcols.end());
-                hptr[static_cast<size_t>(bb) + 1] = static_cast<int>(hidx.size());
-                hmax = std::max(hmax, static_cast<int>(cols.size()));
-                smax = std::max(smax, a1 - a0);
-                remote.add_cta(sb * 32, se * 32, hcols);
-                lcsb = std::max(lcsb, cgcg_lcs_bytes(P.slice_w.data(), sb, se, nwarps, CGCG_ROUND));
-            }
-            if (!fits || (want == 4 && hmax > CGCG_HALO_MAX)) continue;
+            Partition part = partition_rows(P, colp, g, nwarps);
+            int hmax = part.hmax;
+            const long long smax = part.smax;
+            const RemoteLists& remote = part.remote;
+            if (!part.fits || (want == 4 && hmax > CGCG_HALO_MAX)) continue;
             if (want == 4) ++hmax;   // the spare place
-            const size_t smem = want == 4 ? cgcg_lcs_off(hmax, remote.most) + lcsb
+            const size_t smem = want == 4 ? cgcg_lcs_off(hmax, remote.most) + part.lcsb
                                           : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
             if (smem > (want == 4 ? 220 : 200) * 1024) continue;
             std::vector<int> pptr;
@@ -3855,16 +3918,16 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                     cgcg_xs_off = static_cast<int>(off);
                 }
             }
-            d_halo_ptr = dalloc<int>(hptr.size());
-            d_halo_idx = dalloc<int>(hidx.size());
-            d_lcol = dalloc<unsigned short>(lcol.size());
-            CUDA_OK(cudaMemcpy(d_halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CUDA_OK(cudaMemcpy(d_halo_idx, hidx.data(), hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-            if (!lcol.empty()) CUDA_OK(cudaMemcpy(d_lcol, lcol.data(), lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+            d_halo_ptr = dalloc<int>(part.hptr.size());
+            d_halo_idx = dalloc<int>(part.hidx.size());
+            d_lcol = dalloc<unsigned short>(part.lcol.size());
+            CUDA_OK(cudaMemcpy(d_halo_ptr, part.hptr.data(), part.hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+            CUDA_OK(cudaMemcpy(d_halo_idx, part.hidx.data(), part.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
+            if (!part.lcol.empty()) CUDA_OK(cudaMemcpy(d_lcol, part.lcol.data(), part.lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
             dev_halo_max = hmax;
             dev_slot_max = static_cast<int>(smax);
-            h_hptr = hptr;
-            h_hidx = hidx;
+            h_hptr = part.hptr;
+            h_hidx = part.hidx;
             if (want == 4) {
                 dev_rem_max = remote.most;
                 rem_total = static_cast<long long>(remote.rem.size());

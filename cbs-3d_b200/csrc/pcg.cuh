@@ -104,6 +104,27 @@ struct CoarseDev {
     const double* ainv;
 };
 
+// The two-level kernel's dynamic shared memory, for the kernel and for the
+// host that sizes it: z and inverse diagonal of the halo from byte 0 on
+// (halo_max doubles each), then at the offsets below its positions, the local
+// columns, the neighbours' rows of the coarse inverse with the coarse vectors
+// behind them (nbr_max*g + 3*g + nbr_max doubles) and every halo entry's owner.
+struct TwoLevelLayout {
+    size_t hidx, lcs, ainv, hown, bytes;
+    __host__ __device__ TwoLevelLayout(int halo_max, int slot_max, int nbr_max, int g)
+        : hidx(16 * static_cast<size_t>(halo_max)), lcs(hidx + 4 * static_cast<size_t>(halo_max)),
+          ainv((lcs + 2 * static_cast<size_t>(slot_max) + 15) & ~static_cast<size_t>(15)),
+          hown(ainv + 8 * (static_cast<size_t>(nbr_max) * (g + 1) + 3 * static_cast<size_t>(g))),
+          bytes(hown + static_cast<size_t>(halo_max))
+    {
+    }
+};
+
+// One row partition's sizes and the shared memory that the kernels on it get
+// (cbs3d_probe_pcg_partition).
+cbs3d_status probe_partition(int nelem, int npoin, const int* intma, const int* mat_elem, const double* coord, int ctas,
+                             cbs3d_pcg_partition* out);
+
 // Owns the device copies of the pattern and the PCG work vectors.
 class PcgEngine {
 public:
@@ -160,7 +181,7 @@ public:
     size_t global_halo_smem = 0;
     long long global_halo_total = 0;   // halo entries over all CTAs
     int global_halo_parts = 1;         // parts per CTA, each with its own halo
-    size_t halo_smem = 0;    // dynamic shared memory of the halo kernel
+    size_t halo_smem = 0;    // dynamic shared memory of the two-reduction halo kernel
     size_t cgcg_smem = 0;    // ... of the CG-CG kernel (halo, remote entries, its rows' diagonal)
     int cgcg_ks = 0;         // 1: the kernel reads its warps' first rows' coefficients from shared memory
     int cgcg_coef_off = 0;   // where they start

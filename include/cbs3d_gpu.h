@@ -432,6 +432,19 @@ cbs3d_status cbs3d_probe_allreduce(int device, int iters, double* us_per_allredu
 cbs3d_status cbs3d_probe_halo_placement(int nh, int nslices, const long long* slice_off, const int* slice_w,
                                         const unsigned short* lc, int* pos, long long* wavefronts);
 
+/* Row partition probe (no reference counterpart; host only, touches no
+ * device).  The mesh's pressure rows split over `ctas` CTAs of 512 threads as
+ * the PCG engine splits them: coord (3*npoin, may be NULL as for the
+ * coordinate-free pressure solver) sets the rows' order.  Returns the largest
+ * halo, slots, remote halo entries and neighbours of a CTA and the dynamic
+ * shared memory in bytes that the engine allocates to the two-level kernel. */
+typedef struct cbs3d_pcg_partition {
+    int ctas, halo_max, slot_max, remote_max, neighbour_max;
+    long long two_level_bytes;
+} cbs3d_pcg_partition;
+cbs3d_status cbs3d_probe_pcg_partition(int nelem, int npoin, const int* intma, const int* mat_elem,
+                                       const double* coord, int ctas, cbs3d_pcg_partition* out);
+
 #ifdef __cplusplus
 }
 #endif

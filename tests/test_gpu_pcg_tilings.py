@@ -120,3 +120,17 @@ def test_batch_tilings_with_a_large_instance(rows, spread):
         for p, q in zip(b.fields(i)[:2], x.fields()[:2]):
             assert rel_l2(p, q) <= 1e-8
         x.close()
+
+
+def test_two_level_kernel_at_eight_rows_per_thread():
+    """The two-level kernel on a uniform mesh, where its layout is larger than
+    the single-reduction kernel's: the Jacobi engine's pressure to the solves'
+    tolerance, in far fewer iterations."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(74, re=400.0, ntime=10 ** 6)
+    a, b = gpu.Context(case, two_level=True), gpu.Context(case)
+    sa, sb = a.step(1), b.step(1)
+    assert sa.pcg_kernel == 6
+    assert sa.cg.iterations < sb.cg.iterations
+    assert rel_l2(a.fields()[1], b.fields()[1]) <= 1e-8

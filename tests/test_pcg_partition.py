@@ -1,0 +1,42 @@
+"""The PCG kernels' shared memory against their layouts, host only: for a mesh
+split over the engine's grid, what the engine allocates covers what the kernel
+addresses (restated here from the arrays that it keeps)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+
+class Partition(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in ("ctas", "halo_max", "slot_max", "remote_max", "neighbour_max")] + [
+        ("two_level_bytes", ctypes.c_longlong)]
+
+
+def partition(mesh, ctas=148, coord=True):
+    from cbs3d import gpu
+    L = gpu.lib()
+    L.cbs3d_probe_pcg_partition.restype = ctypes.c_int
+    P = ctypes.c_void_p
+    xyz = np.ascontiguousarray(mesh.coord, dtype=np.float64)
+    conn = np.ascontiguousarray(mesh.intma, dtype=np.int32)
+    out = Partition()
+    rc = L.cbs3d_probe_pcg_partition(conn.shape[0], xyz.shape[0], P(conn.ctypes.data), None,
+                                     P(xyz.ctypes.data) if coord else None, ctas, ctypes.byref(out))
+    assert rc == 0
+    return out
+
+
+# the sizes at which the tilings of four and eight rows per thread end, and
+# grids of fewer CTAs, where the own rows are more of a halo
+@pytest.mark.parametrize("shape,ctas", [((72, 72, 72), 148), ((74, 74, 74), 148), ((76, 76, 76), 148),
+                                        ((61, 81, 83), 148), ((63, 63, 63), 128), ((48, 48, 48), 64), ((5, 5, 5), 148)])
+def test_two_level_kernel_has_the_shared_memory_it_addresses(shape, ctas):
+    from cbs3d import cases
+    p = partition(cases.box_mesh(*shape), ctas)
+    # z, inverse diagonal (8 bytes) and position (4) per halo entry; columns
+    need = 20 * p.halo_max + 2 * p.slot_max
+    need = (need + 15) // 16 * 16
+    # the neighbours' rows of the coarse inverse, three coarse vectors, a correction per neighbour
+    need += 8 * (p.neighbour_max * p.ctas + 3 * p.ctas + p.neighbour_max)
+    need += p.halo_max   # every entry's owner
+    assert p.two_level_bytes >= need
