@@ -4444,13 +4444,19 @@ void PcgBatch::free_waves()
 
 bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
 {
-    // One 512-thread CTA per SM with the coefficients in tensor memory (one
-    // row per thread: in registers), else two 256-thread CTAs per SM.  12
+    // FP64: one 512-thread CTA per SM with the coefficients in tensor memory
+    // (one row per thread: in registers), else two 256-thread CTAs per SM.  12
     // cavities of 10..32 hexes per side, two steps: 10.2 -> 5.7 ms.
-    return (!mixed && plan_threads(p, 512, why)) || plan_threads(p, BATCH_THREADS, why);
+    // Mixed: the FP32 kernel (two 256-thread CTAs per SM) where every wave's
+    // coefficients fit its shared memory; a plan of which some wave would run
+    // in FP64 anyway runs there as a whole (48 cavities of 10..40, a step:
+    // 22.1 ms in FP32 and FP64 waves of 256 threads, 12.2 in FP64 waves of 512).
+    const bool fp32 = mixed && !p.fp64;
+    return (fp32 && plan_threads(p, BATCH_THREADS, true, why)) || plan_threads(p, 512, false, why) ||
+           plan_threads(p, BATCH_THREADS, false, why);
 }
 
-bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, std::string* why)
+bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::string* why)
 {
     const int gmax = nt == 512 ? sms : 2 * sms, nwarps = nt / 32;
     if (p.rmax != 1 && p.rmax != 2 && p.rmax != 4 && p.rmax != 8) {
@@ -4627,8 +4633,8 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, std::string* why)
                 W.smem = with;
             }
         }
-        else if (mixed && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
-        else if (H.hmax <= CGCG_HALO_MAX && fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
+        else if (mixed && !p.fp64 && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
+        else if (!all_fp32 && H.hmax <= CGCG_HALO_MAX && fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
         else {
             if (why) *why = "a wave does not fit co-resident at this tiling";
             return false;

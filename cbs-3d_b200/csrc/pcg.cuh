@@ -246,10 +246,12 @@ struct PcgBatchMember {
 };
 
 // A tiling of the batch: rows per thread (1, 2, 4 or 8 slices of 32 rows per
-// warp) and whether the spare CTAs of a wave are shared out by instance size.
+// warp), whether the spare CTAs of a wave are shared out by instance size, and
+// for a mixed-precision batch whether it runs the FP64 kernels all the same.
 struct PcgBatchPlan {
     int rmax = 4;
     int spread = 1;
+    int fp64 = 0;
 };
 
 class PcgBatch {
@@ -273,7 +275,7 @@ public:
     bool mixed_any = false;      // some wave runs the mixed-precision kernel
 
 private:
-    bool plan_threads(const PcgBatchPlan& p, int nt, std::string* why);
+    bool plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::string* why);
     struct Wave {
         int G = 0, rmax = 4, threads = 0, tm_w = 0, pds_off = 0, xs_off = 0;
         bool mixed = false;

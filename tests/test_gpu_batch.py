@@ -173,3 +173,21 @@ def test_gpu_runner_drives_the_batch_on_one_device():
     for m in whole:
         assert abs(split[m["instance"]]["cg_iterations"] - m["cg_iterations"]) <= 2
         assert split[m["instance"]]["nelem"] == m["nelem"]
+
+
+def test_mixed_batch_is_no_slower_than_the_fp64_batch():
+    """The autotuner of a mixed-precision batch also times the FP64 waves, so
+    its choice is about as fast as the FP64 batch's (those waves are several
+    times faster than the FP32 kernel here; a quarter is left for noise), and
+    the solutions agree."""
+    from cbs3d import cases
+    gpu = _gpu()
+    cs = cases.cavity_batch(12, 10, 32)
+    a, m = gpu.Batch(cs), gpu.Batch(cs, precision=gpu.MIXED)
+    a.step(3)
+    m.step(3)
+    best = [min(ms for _, _, ms in x.info()["candidates_timed"] if ms > 0) for x in (a, m)]
+    assert best[1] <= 1.25 * best[0]
+    for i in range(len(cs)):
+        (u0, p0, _), (u1, p1, _) = a.fields(i), m.fields(i)
+        assert rel_l2(u1, u0) <= MIXED_TOL and rel_l2(p1, p0) <= MIXED_TOL
