@@ -1765,7 +1765,16 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
 // KT > 0: the coefficients of each thread's rows KS .. KS+KT-1 live in TMEM
 // for the solve (D.tm_w slots per row, zero-padded past the slice's width);
 // `tm` is the CTA's TMEM base address (0 when KT = 0).
-template <int RMAX, bool BATCH, int NT, int KS, int KT, bool CL>
+//
+// RG: for CTAs whose halo is mostly remote (thin meshes, orders without
+// coordinates) the 30 bytes per remote entry do not fit beside the halo.
+// Their positions, places and inverse diagonals are then read from global
+// memory as one 16-byte record each, r and s stay in shared memory where those
+// fit (else in global memory too, always touched by the same thread), the
+// local columns are places instead of byte offsets (halos up to 65,534), and
+// slots past tm_w stream from L2, so that every mesh the halo itself fits for
+// has this kernel.
+template <int RMAX, bool BATCH, int NT, int KS, int KT, bool CL, bool RG>
 __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsigned long long epoch)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1787,17 +1796,39 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     double* dzh = sh + D.rem_max;
     int* rgi = reinterpret_cast<int*>(dzh + D.rem_max);        // rem_max: their row positions
     unsigned short* rhp = reinterpret_cast<unsigned short*>(rgi + D.rem_max);   // ... and places in vh
+    RemoteState* rst = nullptr;
+    if constexpr (RG) {
+        rst = D.rem_state + q0;
+        rh = D.rs_off ? reinterpret_cast<double*>(smem_raw + D.rs_off) : D.rem_rs + 2 * (size_t)q0;
+        sh = rh + (D.rs_off ? D.rem_max : nr);
+    }
     // the own rows' diagonal, kept in shared memory for the solve where the
     // engine sized it so
     double* pds = NT == 512 && D.pds_off ? reinterpret_cast<double*>(smem_raw + D.pds_off) : nullptr;
     for (int k = threadIdx.x; k < nr; k += NT) {
         const int2 e = D.rem[q0 + k];
         const uint8_t f = D.nflag[e.x];
-        if (!CL) rgi[k] = e.x;
-        rhp[k] = (unsigned short)e.y;
-        dzh[k] = (f & 1) && !(f & 4) ? (g.precond ? 1.0 / D.pdiag[e.x] : 1.0) : 0.0;
+        const double dj = (f & 1) && !(f & 4) ? (g.precond ? 1.0 / D.pdiag[e.x] : 1.0) : 0.0;
+        if constexpr (RG) {
+            rst[k].dz = dj;
+        } else {
+            if (!CL) rgi[k] = e.x;
+            rhp[k] = (unsigned short)e.y;
+            dzh[k] = dj;
+        }
         sh[k] = 0.0;
     }
+    // place and inverse diagonal of remote entry e
+    auto remote = [&](int e, int& place, double& dj) {
+        if constexpr (RG) {
+            const RemoteState x = rst[e];
+            place = x.place;
+            dj = x.dz;
+        } else {
+            place = rhp[e];
+            dj = dzh[e];
+        }
+    };
     // CL: the exchange through the cluster's shared memory.  cwx: 2 x rem_max
     // values of the remote entries, as their owners push them; cwo: the own
     // rows' value; cpu, cpl: where each pushed value goes (in the consumer's
@@ -1904,7 +1935,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
             const unsigned pad = wr[k] > 0 ? src[0] : 0;
             for (int j = 0; j < wmax / 2; ++j) {
                 const unsigned lo = 2 * j < wr[k] ? src[64 * j] : pad, hi = 2 * j + 1 < wr[k] ? src[64 * j + 32] : pad;
-                mine[(k * (wmax / 2) + j) * 32] = lo * 8 | hi * 8 << 16;
+                mine[(k * (wmax / 2) + j) * 32] = RG ? lo | hi << 16 : lo * 8 | hi * 8 << 16;
             }
         }
         lcp = mine;
@@ -1941,6 +1972,11 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 #pragma unroll
         for (int u = 0; u < XW; ++u) vx[u] = u < wr[k] ? __ldcg(D.val + S0 + lbase[k] + 32 * u) : 0.0;
     };
+    // z at a local column
+    auto zcol = [&](unsigned c) -> double {
+        if constexpr (RG) return vh[c];
+        else return *reinterpret_cast<const double*>(smem_raw + c);
+    };
     auto offdiag_all = [&](double* off) {
 #pragma unroll
         for (int k = 0; k < RMAX; ++k) off[k] = 0.0;
@@ -1948,20 +1984,21 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 #pragma unroll
             for (int j = 0; j < RW / 2; ++j)
                 if (2 * j < wmax) {
-                    const double x0 = *reinterpret_cast<const double*>(smem_raw + (crow[j] & 0xffffu));
-                    const double x1 = *reinterpret_cast<const double*>(smem_raw + (crow[j] >> 16));
+                    const double x0 = zcol(crow[j] & 0xffffu);
+                    const double x1 = zcol(crow[j] >> 16);
                     off[0] = fma(vrow[2 * j], x0, off[0]);
                     off[0] = fma(vrow[2 * j + 1], x1, off[0]);
                 }
             for (int u = RW; u < wr[0]; ++u) {
                 const unsigned c = lcp[(u >> 1) * 32] >> (16 * (u & 1));
                 off[0] = fma(__ldcg(D.val + S0 + lbase[0] + 32 * u),
-                             *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[0]);
+                             zcol(c & 0xffffu), off[0]);
             }
             return;
         }
         const unsigned* lc = lcp;
-        for (int k0 = 0; k0 < wmax; k0 += CH, lc += CH / 2 * 32) {
+        const int wt = RG && KT > 0 ? min(wmax, D.tm_w) : wmax;
+        for (int k0 = 0; k0 < wt; k0 += CH, lc += CH / 2 * 32) {
             double v[RMAX][CH], x[RMAX][CH];
             uint32_t tv[KT > 0 ? KT : 1][2 * CH];
             if constexpr (KT > 0) {
@@ -1983,8 +2020,8 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 #pragma unroll
                     for (int j = 0; j < CH / 2; ++j) {
                         const unsigned c = lc[(k * (wmax / 2) + j) * 32];
-                        x[k][2 * j] = *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu));
-                        x[k][2 * j + 1] = *reinterpret_cast<const double*>(smem_raw + (c >> 16));
+                        x[k][2 * j] = zcol(c & 0xffffu);
+                        x[k][2 * j + 1] = zcol(c >> 16);
                     }
                 }
             if constexpr (KT > 0) {
@@ -2004,6 +2041,23 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
                     for (int u = 0; u < CH; ++u) off[k] = fma(v[k][u], x[k][u], off[k]);
                 }
         }
+        if constexpr (RG && KT > 0) {
+            for (int k0 = wt; k0 < wmax; k0 += CH, lc += CH / 2 * 32)
+#pragma unroll
+                for (int k = 0; k < RMAX - KX; ++k)
+                    if (k < nk) {
+                        double v[CH];
+#pragma unroll
+                        for (int u = 0; u < CH; ++u)
+                            v[u] = k0 + u < wr[k] ? __ldcg(D.val + S0 + lbase[k] + 32 * (k0 + u)) : 0.0;
+#pragma unroll
+                        for (int j = 0; j < CH / 2; ++j) {
+                            const unsigned c = lc[(k * (wmax / 2) + j) * 32];
+                            off[k] = fma(v[2 * j], zcol(c & 0xffffu), off[k]);
+                            off[k] = fma(v[2 * j + 1], zcol(c >> 16), off[k]);
+                        }
+                    }
+        }
         if constexpr (KX > 0) {
 #pragma unroll
             for (int k = RMAX - KX; k < RMAX; ++k)
@@ -2014,13 +2068,13 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
                     for (int j = 0; j < XW / 2; ++j)
                         if (2 * j < wmax) {
                             const unsigned c = lx[j * 32];
-                            off[k] = fma(vx[2 * j], *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[k]);
-                            off[k] = fma(vx[2 * j + 1], *reinterpret_cast<const double*>(smem_raw + (c >> 16)), off[k]);
+                            off[k] = fma(vx[2 * j], zcol(c & 0xffffu), off[k]);
+                            off[k] = fma(vx[2 * j + 1], zcol(c >> 16), off[k]);
                         }
                     for (int u = XW; u < wr[k]; ++u) {
                         const unsigned c = lx[(u >> 1) * 32] >> (16 * (u & 1));
                         off[k] = fma(__ldcg(D.val + S0 + lbase[k] + 32 * u),
-                                     *reinterpret_cast<const double*>(smem_raw + (c & 0xffffu)), off[k]);
+                                     zcol(c & 0xffffu), off[k]);
                     }
                 }
         }
@@ -2039,6 +2093,10 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
     // this thread are requested with request() and all are waited for and
     // handed to use(entry, value) by collect()
     constexpr int RP = RMAX >= 8 ? 2 : RMAX;
+    auto row_of = [&](int e) -> int {
+        if constexpr (RG) return rst[e].row;
+        else return rgi[e];
+    };
     auto store = [&](const double (&v)[RMAX]) {
         if constexpr (CL) {
 #pragma unroll
@@ -2060,7 +2118,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         for (int u = 0; u < RP; ++u) {
             const int e = threadIdx.x + u * NT;
             xt[u] = 0;
-            if (e < nr) ld_tag(o + rgi[e], xv[u], xt[u]);
+            if (e < nr) ld_tag(o + row_of(e), xv[u], xt[u]);
         }
     };
     auto collect = [&](int ph, auto&& use) -> bool {
@@ -2078,7 +2136,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
                 for (int u = 0; u < RP; ++u) {
                     const int e = e0 + u * NT;
                     xt[u] = 0;
-                    if (e < nr) ld_tag(o + rgi[e], xv[u], xt[u]);
+                    if (e < nr) ld_tag(o + row_of(e), xv[u], xt[u]);
                 }
             }
 #pragma unroll
@@ -2087,7 +2145,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
                 if (e < nr) {
                     while (xt[u] != want) {
                         if (lim.expired(comm.status)) { ok = false; break; }
-                        ld_tag(o + rgi[e], xv[u], xt[u]);
+                        ld_tag(o + row_of(e), xv[u], xt[u]);
                     }
                     use(e, xv[u]);
                 }
@@ -2201,8 +2259,11 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 
     // ---- phase 0b: z0 = M^-1 r0, w0 = A z0, gamma0 = (r0,z0), delta0 = (z0,w0)
     bool got = collect(phase, [&](int e, double v) {
+        int place;
+        double dj;
+        remote(e, place, dj);
         rh[e] = v;
-        vh[rhp[e]] = v * dzh[e];
+        vh[place] = v * dj;
     });
 #pragma unroll
     for (int k = 0; k < RMAX; ++k)
@@ -2244,11 +2305,14 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         // z_it of the halo: s = w + beta*s, r -= alpha*s, z = r * dz, for the
         // remote entries from their owners' w and for the own rows
         got = collect(wph, [&](int e, double v) {
+            int place;
+            double dj;
+            remote(e, place, dj);
             const double sj = fma(beta, sh[e], v);
             const double rj = fma(-alpha, sj, rh[e]);
             sh[e] = sj;
             rh[e] = rj;
-            vh[rhp[e]] = rj * dzh[e];
+            vh[place] = rj * dj;
         });
         // own rows: p = z_o + beta*p, s = w + beta*s, r -= alpha*s
 #pragma unroll
@@ -2329,13 +2393,13 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
 // tensor memory before the solve and returns it after; every exit of the
 // body (converged, an error status, a timed-out wait) is CTA-uniform and
 // comes back here, so the memory is freed on every path.
-template <int RMAX, bool BATCH, int NT, int KS = 0, int KT = 0, bool CL = false>
+template <int RMAX, bool BATCH, int NT, int KS = 0, int KT = 0, bool CL = false, bool RG = false>
 __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
 {
     unsigned long long epoch;
     if (!tag_begin<BATCH>(D, epoch)) return;
     if constexpr (KT == 0) {
-        pcg64c_body<RMAX, BATCH, NT, KS, 0, CL>(D, 0u, epoch);
+        pcg64c_body<RMAX, BATCH, NT, KS, 0, CL, RG>(D, 0u, epoch);
     } else {
         static_assert(NT == 512, "TMEM rows: one CTA per SM");
         __shared__ uint32_t s_tm;
@@ -2345,7 +2409,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_pcg64c(PcgDev D)
         __syncthreads();
         tmem_fence_after_sync();
         const uint32_t tm = s_tm;
-        pcg64c_body<RMAX, BATCH, NT, KS, KT, CL>(D, tm, epoch);
+        pcg64c_body<RMAX, BATCH, NT, KS, KT, CL, RG>(D, tm, epoch);
         tmem_fence_before_sync();
         __syncthreads();
         tmem_fence_after_sync();
@@ -3432,6 +3496,41 @@ size_t cgcg_lcs_bytes(const int* slice_w, int sb, int se, int nwarps, int ch)
 }
 // the largest halo whose byte offsets fit 16 bits
 constexpr int CGCG_HALO_MAX = 8190;
+// k_pcg64c's form for a halo of hmax entries (with the spare place), rem_max
+// of them remote, and lcsb bytes of columns: the remote entries' state in
+// shared memory where it fits `limit` bytes, else in global memory, r and s
+// staying where they alone fit.  64^3 without coordinates: 226,880 bytes in
+// the first form, 183,608 in the second.
+struct CgcgLayout {
+    bool rg;
+    size_t lcs, rs, bytes;
+    CgcgLayout(int hmax, int rem_max, size_t lcsb, size_t limit, bool global_only = false)
+        : rg(global_only || hmax - 1 > CGCG_HALO_MAX || cgcg_lcs_off(hmax, rem_max) + lcsb > limit),
+          lcs(rg ? (8 * static_cast<size_t>(hmax) + 15) & ~static_cast<size_t>(15) : cgcg_lcs_off(hmax, rem_max)), rs(0),
+          bytes(lcs + lcsb)
+    {
+        const size_t off = (bytes + 15) & ~static_cast<size_t>(15), with = off + 16 * static_cast<size_t>(rem_max);
+        if (rg && rem_max > 0 && with <= limit) {
+            rs = off;
+            bytes = with;
+        }
+    }
+};
+constexpr size_t CGCG_SMEM_MAX = 220 * 1024;
+// The second form is taken with r and s in shared memory and up to four rows
+// per thread: 64^3 without coordinates 10.25 us per iteration against 11.6 on
+// the global-vector kernel, a 900x16x16 channel 10.4 against 12.2; at five
+// rows (70^3) 22.6 against 14.1, with r and s in global memory (a 1200x16x16
+// channel) 20.7 against 14.5.
+constexpr int RG_ROWS_MAX = 4;
+
+// The remote entries and their state's initial content.
+std::vector<RemoteState> remote_states(const std::vector<int2>& rem)
+{
+    std::vector<RemoteState> o;
+    for (const int2& e : rem) o.push_back(RemoteState{0.0, e.x, e.y});
+    return o;
+}
 
 // The rows split over g CTAs of nwarps warps: each CTA's halo (the distinct
 // columns of its slots) in the order of its places in shared memory, its
@@ -3530,13 +3629,14 @@ CoarseNeighbours coarse_neighbours(int nslices, const std::vector<int>& hptr, co
 
 // Instantiations of the single-reduction kernels by rows per thread, batch
 // mode and CTA size.
-template <int NT>
-const void* fn_cgcg_batch(int rmax)
+// ... of the batch's 256-thread CTAs
+template <bool RG>
+const void* fn_cgcg_batch256(int rmax)
 {
-    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, true, NT>)
-         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, true, NT>)
-         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, true, NT>)
-                     : reinterpret_cast<const void*>(k_pcg64c<8, true, NT>);
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, true, 256, 0, 0, false, RG>)
+         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, true, 256, 0, 0, false, RG>)
+         : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, true, 256, 0, 0, false, RG>)
+                     : reinterpret_cast<const void*>(k_pcg64c<8, true, 256, 0, 0, false, RG>);
 }
 template <bool BATCH, int NT>
 const void* fn_mixed(int rmax)
@@ -3577,6 +3677,16 @@ const void* fn_cgcg_single(int rmax, int ks, int kt)
          : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512>)
          : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512>)
                      : reinterpret_cast<const void*>(k_pcg64c<8, false, 512>);
+}
+
+// ... with the remote entries' state in global memory, up to four rows
+template <bool BATCH>
+const void* fn_cgcg_rg(int rmax)
+{
+    return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, BATCH, 512, 0, 0, false, true>)
+         : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, BATCH, 512, 0, 2, false, true>)
+         : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, BATCH, 512, 0, 3, false, true>)
+                     : reinterpret_cast<const void*>(k_pcg64c<4, BATCH, 512, 0, 4, false, true>);
 }
 
 // ... of the batch, one 512-thread CTA per SM
@@ -3623,8 +3733,11 @@ cbs3d_status probe_partition(int nelem, int npoin, const int* intma, const int* 
     if (!part.fits) return CBS3D_INVALID_INPUT;
     const CoarseNeighbours nb = coarse_neighbours(P.nslices, part.hptr, part.hidx);
     const int hmax = part.hmax + 1;   // the spare place
+    const CgcgLayout lay(hmax, part.remote.most, part.lcsb, CGCG_SMEM_MAX);
     *out = cbs3d_pcg_partition{g, hmax, static_cast<int>(part.smax), part.remote.most, nb.most,
-                               static_cast<long long>(TwoLevelLayout(hmax, static_cast<int>(part.smax), nb.most, g).bytes)};
+                               lay.bytes > CGCG_SMEM_MAX ? -1 : !lay.rg ? 0 : lay.rs ? 1 : 2,
+                               static_cast<long long>(TwoLevelLayout(hmax, static_cast<int>(part.smax), nb.most, g).bytes),
+                               static_cast<long long>(lay.bytes)};
     return CBS3D_OK;
 }
 
@@ -3825,11 +3938,14 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             int hmax = part.hmax;
             const long long smax = part.smax;
             const RemoteLists& remote = part.remote;
-            if (!part.fits || (want == 4 && hmax > CGCG_HALO_MAX)) continue;
+            if (!part.fits) continue;
             if (want == 4) ++hmax;   // the spare place
-            const size_t smem = want == 4 ? cgcg_lcs_off(hmax, remote.most) + part.lcsb
-                                          : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
-            if (smem > (want == 4 ? 220 : 200) * 1024) continue;
+            const CgcgLayout lay(hmax, remote.most, part.lcsb, CGCG_SMEM_MAX);
+            const bool rg = want == 4 && lay.rg;
+            if (rg && (cl || !lay.rs || rr > RG_ROWS_MAX)) continue;
+            const size_t smem = want == 4 ? lay.bytes : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
+            if (smem > (want == 4 ? CGCG_SMEM_MAX : 200 * 1024)) continue;
+            if (rg) fn = fn_cgcg_rg<false>(rr);
             std::vector<int> pptr;
             std::vector<int2> push;
             int pmost = 0;
@@ -3853,6 +3969,8 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             nblocks = g;
             halo_smem = smem;
             cgcg_smem = smem;
+            cgcg_rg = rg;
+            cgcg_rs_off = rg ? static_cast<int>(lay.rs) : 0;
             // Tensor memory: 128 columns = 64 doubles per thread, the slots
             // of a row padded to the widest slice of the mesh.  Up to four
             // rows all live there, of more the first four; choice 11 (two or
@@ -3865,7 +3983,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (cluster) cgcg_smem = cl_smem;
             auto resident = [&](int ks, int kt, size_t bytes) {
                 if (cluster) return cluster_fits(fn_cgcg_cluster(), g, bytes);
-                const void* fk = fn_cgcg_single(rr, ks, kt);
+                const void* fk = rg ? fn : fn_cgcg_single(rr, ks, kt);
                 int per2 = 0;
                 const bool ok = bytes <= 227 * 1024 && raise_smem_limit(fk, bytes) == cudaSuccess &&
                                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, fk, nt, bytes) == cudaSuccess &&
@@ -3877,7 +3995,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                 int wmx = 0;
                 for (int q = 0; q < nslices; ++q) wmx = std::max(wmx, P.slice_w[static_cast<size_t>(q)]);
                 const int chw = CGCG_ROUND, tw = (wmx + chw - 1) / chw * chw;
-                if (kernel_choice == 11 && (rr == 2 || rr == 4) && tw > 0 && (rr - 1) * tw <= 64) {
+                if (kernel_choice == 11 && !rg && (rr == 2 || rr == 4) && tw > 0 && (rr - 1) * tw <= 64) {
                     long long cmax = 0;
                     for (int bb = 0; bb < g; ++bb) {
                         const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
@@ -3894,8 +4012,13 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                     }
                 }
                 const int kt = rr == 1 ? 0 : std::min(rr, 4);
-                if (!cgcg_ks && kt > 0 && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
-                if (cgcg_kt) cgcg_tm_w = tw;
+                if (rg) {
+                    // the slots of a row that fit; any others stream from L2
+                    if (kt > 0) cgcg_tm_w = std::min(tw, 64 / kt / chw * chw);
+                } else {
+                    if (!cgcg_ks && kt > 0 && tw > 0 && kt * tw <= 64 && resident(0, kt, cgcg_smem)) cgcg_kt = kt;
+                    if (cgcg_kt) cgcg_tm_w = tw;
+                }
             }
             // the rows' diagonal in shared memory (64^3: 12.05 -> 11.95 us
             // per iteration; in registers it was slower)
@@ -3931,12 +4054,17 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (want == 4) {
                 dev_rem_max = remote.most;
                 rem_total = static_cast<long long>(remote.rem.size());
-                cgcg_lcs = static_cast<int>(cgcg_lcs_off(hmax, remote.most));
+                cgcg_lcs = static_cast<int>(lay.lcs);
                 d_rem_ptr = dalloc<int>(remote.ptr.size());
                 d_rem = dalloc<int2>(remote.rem.size());
                 d_own = dalloc<int>(remote.own.size());
                 CUDA_OK(cudaMemcpy(d_rem_ptr, remote.ptr.data(), remote.ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
                 if (!remote.rem.empty()) CUDA_OK(cudaMemcpy(d_rem, remote.rem.data(), remote.rem.size() * sizeof(int2), cudaMemcpyHostToDevice));
+                if (rg) {
+                    const std::vector<RemoteState> st = remote_states(remote.rem);
+                    d_rem_state = dalloc<RemoteState>(st.size());
+                    CUDA_OK(cudaMemcpy(d_rem_state, st.data(), st.size() * sizeof(RemoteState), cudaMemcpyHostToDevice));
+                }
                 CUDA_OK(cudaMemcpy(d_own, remote.own.data(), remote.own.size() * sizeof(int), cudaMemcpyHostToDevice));
                 if (cluster) {
                     cgcg_cl_off = static_cast<int>(cl_off);
@@ -4100,6 +4228,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
     dev.rec = d_rec; dev.xw = d_xw; dev.epoch = d_epoch;
     dev.push_ptr = d_push_ptr; dev.push = d_push; dev.push_max = dev_push_max; dev.cl_off = cgcg_cl_off;
     dev.rem_ptr = d_rem_ptr; dev.rem = d_rem; dev.own = d_own; dev.rem_max = dev_rem_max;
+    dev.rem_state = d_rem_state; dev.rs_off = cgcg_rs_off;
     dev.lcs_off = cgcg_lcs;
     dev.coef_off = cgcg_coef_off;
     dev.pds_off = cgcg_pds_off;
@@ -4120,13 +4249,14 @@ void PcgEngine::release()
     mg_ready = false;
     void* ptrs[] = {d_slice_off, d_slice_w, d_col, d_cptr, d_cent, d_val, d_val32, d_r, d_z, d_pA,
                     d_pB, d_q, d_f32, d_part, d_bar, d_out, d_halo_ptr, d_halo_idx, d_lcol, d_row_node,
-                    d_rec, d_xw, d_epoch, d_rem_ptr, d_rem, d_own, d_push_ptr, d_push,
+                    d_rec, d_xw, d_epoch, d_rem_ptr, d_rem, d_own, d_push_ptr, d_push, d_rem_state,
                     d_xp, d_bp, d_dp, d_fp, d_pair_ptr, d_pair_ij, d_pair_ent, d_ac, d_nbr_ptr, d_nbr_ids, d_hown};
     for (void* p : ptrs) if (p) cudaFree(p);
     d_pair_ptr = nullptr; d_pair_ij = nullptr; d_pair_ent = nullptr; d_ac = nullptr;
     d_nbr_ptr = nullptr; d_nbr_ids = nullptr; d_hown = nullptr;
     coarse = false;
     d_rec = d_xw = nullptr; d_epoch = nullptr; d_rem_ptr = d_own = d_push_ptr = nullptr; d_rem = d_push = nullptr;
+    d_rem_state = nullptr;
     d_slice_off = nullptr; d_slice_w = nullptr; d_col = nullptr; d_cptr = nullptr; d_cent = nullptr;
     d_val = nullptr; d_val32 = nullptr; d_r = d_z = d_pA = d_pB = d_q = nullptr; d_f32 = nullptr;
     d_part = nullptr; d_bar = nullptr; d_out = nullptr;
@@ -4211,7 +4341,7 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
         fn = fn_mixed<false, 512>(rmax);
         smem = mixed_smem;
     } else if (variant == 4) {
-        fn = cluster ? fn_cgcg_cluster() : fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
+        fn = cluster ? fn_cgcg_cluster() : cgcg_rg ? fn_cgcg_rg<false>(rmax) : fn_cgcg_single(rmax, cgcg_ks, cgcg_kt);
         smem = cgcg_smem;
     }
     CoarseDev C = cdev;
@@ -4436,7 +4566,7 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
 void PcgBatch::free_waves()
 {
     for (Wave& w : waves) {
-        void* ptrs[] = {w.d_cta_inst, w.d_inst, w.d_hptr, w.d_hidx, w.d_rptr, w.d_rem};
+        void* ptrs[] = {w.d_cta_inst, w.d_inst, w.d_hptr, w.d_hidx, w.d_rptr, w.d_rem, w.d_rem_state, w.d_rem_rs};
         for (void* p : ptrs) if (p) cudaFree(p);
     }
     waves.clear();
@@ -4486,8 +4616,6 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
         packs[w].push_back(k);
         used[w] += minc[static_cast<size_t>(k)];
     }
-    const void* c64[4] = {fn_cgcg_batch<BATCH_THREADS>(1), fn_cgcg_batch<BATCH_THREADS>(2), fn_cgcg_batch<BATCH_THREADS>(4),
-                          fn_cgcg_batch<BATCH_THREADS>(8)};
     const void* c32[4] = {fn_mixed<true, BATCH_THREADS>(1), fn_mixed<true, BATCH_THREADS>(2), fn_mixed<true, BATCH_THREADS>(4),
                           fn_mixed<true, BATCH_THREADS>(8)};
     const int ci = p.rmax == 1 ? 0 : p.rmax == 2 ? 1 : p.rmax == 4 ? 2 : 3;
@@ -4595,7 +4723,6 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
         const HostWave& H = hw[w];
         Wave& W = nw[w];
         W.G = H.G; W.rmax = H.rows; W.threads = nt;
-        const size_t s64 = cgcg_lcs_off(H.hmax + 1, H.rmost) + H.lcsb;
         const size_t s32 = static_cast<size_t>(H.hmax) * 16 + static_cast<size_t>(H.smax) * 6 + 16;
         auto fits = [&](const void* fn, size_t smem) {
             if (smem > 220 * 1024) return false;
@@ -4615,14 +4742,18 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
             int wmx = 0;
             for (const PcgInst& I : H.inst)
                 for (int q = I.s0; q < I.s1; ++q) wmx = std::max(wmx, h_slice_w[static_cast<size_t>(q)]);
-            const int ch = CGCG_ROUND, tw = (wmx + ch - 1) / ch * ch;
-            W.fn = fn_cgcg_batch512(H.rows);
-            W.smem = s64;
-            if (H.hmax > CGCG_HALO_MAX || (H.rows > 1 && std::min(H.rows, 4) * tw > 64) || !fits(W.fn, s64)) {
+            const int ch = CGCG_ROUND, tw = (wmx + ch - 1) / ch * ch, kt = std::min(H.rows, 4);
+            const CgcgLayout lay(H.hmax + 1, H.rmost, H.lcsb, CGCG_SMEM_MAX);
+            W.rg = lay.rg;
+            W.fn = lay.rg ? fn_cgcg_rg<true>(H.rows) : fn_cgcg_batch512(H.rows);
+            W.smem = lay.bytes;
+            W.lcs_off = static_cast<int>(lay.lcs);
+            W.rs_off = static_cast<int>(lay.rs);
+            if ((lay.rg ? !lay.rs || H.rows > RG_ROWS_MAX : H.rows > 1 && kt * tw > 64) || !fits(W.fn, W.smem)) {
                 if (why) *why = "a wave does not fit co-resident at this tiling";
                 return false;
             }
-            W.tm_w = tw;
+            W.tm_w = std::min(tw, 64 / kt / ch * ch);
             // the rows' diagonal, and their pressure where the kernel keeps it
             // in memory, behind that
             for (int what = 0; what < 2; ++what) {
@@ -4634,7 +4765,24 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
             }
         }
         else if (mixed && !p.fp64 && fits(c32[ci], s32)) { W.mixed = true; W.fn = c32[ci]; W.smem = s32; }
-        else if (!all_fp32 && H.hmax <= CGCG_HALO_MAX && fits(c64[ci], s64)) { W.mixed = false; W.fn = c64[ci]; W.smem = s64; }
+        else if (!all_fp32) {
+            // as much of the remote entries' state in shared memory as lets
+            // the wave's CTAs be resident together
+            W.mixed = false;
+            W.smem = CGCG_SMEM_MAX + 1;
+            for (int form = 0; form < 3 && !fits(W.fn, W.smem); ++form) {
+                const CgcgLayout lay(H.hmax + 1, H.rmost, H.lcsb, form < 2 ? CGCG_SMEM_MAX : 0, form > 0);
+                W.rg = lay.rg;
+                W.fn = lay.rg ? fn_cgcg_batch256<true>(p.rmax) : fn_cgcg_batch256<false>(p.rmax);
+                W.smem = lay.bytes;
+                W.lcs_off = static_cast<int>(lay.lcs);
+                W.rs_off = static_cast<int>(lay.rs);
+            }
+            if (!fits(W.fn, W.smem)) {
+                if (why) *why = "a wave does not fit co-resident at this tiling";
+                return false;
+            }
+        }
         else {
             if (why) *why = "a wave does not fit co-resident at this tiling";
             return false;
@@ -4672,7 +4820,16 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
         W.dev.tm_w = W.tm_w; W.dev.pds_off = W.pds_off; W.dev.xs_off = W.xs_off;
         if (!W.mixed) {
             W.dev.halo_max = H.hmax + 1;   // the spare place
-            W.dev.lcs_off = static_cast<int>(cgcg_lcs_off(H.hmax + 1, H.rmost));
+            W.dev.lcs_off = W.lcs_off;
+            W.dev.rs_off = W.rs_off;
+        }
+        if (W.rg) {
+            const std::vector<RemoteState> st = remote_states(H.rem);
+            W.d_rem_state = dalloc<RemoteState>(st.size());
+            W.d_rem_rs = dalloc<double>(W.rs_off ? 0 : 2 * st.size());
+            if (!st.empty()) CUDA_OK(cudaMemcpy(W.d_rem_state, st.data(), st.size() * sizeof(RemoteState), cudaMemcpyHostToDevice));
+            W.dev.rem_state = W.d_rem_state;
+            W.dev.rem_rs = W.d_rem_rs;
         }
         W.dev.slot_max = static_cast<int>(H.smax);
         mixed_any = mixed_any || W.mixed;

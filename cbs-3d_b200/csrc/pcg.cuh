@@ -19,6 +19,14 @@ struct __align__(16) TagVal {
     unsigned long long tag;
 };
 
+// A remote halo entry of a CTA whose remote entries' state does not fit its
+// shared memory: its row position, its place in the halo and, written by the
+// kernel, its inverse diagonal (0 off the free rows).
+struct __align__(16) RemoteState {
+    double dz;
+    int row, place;
+};
+
 // One instance of a batched solve: CTAs [cta0, cta0+ncta) of the launch own
 // slices [s0, s1); its own scalars, barrier counter, partials, status, result.
 struct PcgInst {
@@ -73,6 +81,9 @@ struct PcgDev {
     int cl_off;                  // memory of the exchange's buffers
     int lcs_off;                 // byte offset in shared memory of the local columns (k_pcg64c)
     int rem_max;                 // most remote entries of a CTA (shared-memory sizing)
+    RemoteState* rem_state;      // the remote entries where their state is in global memory, and
+    double* rem_rs;              // r and s of each (2 per entry), unless rs_off is
+    int rs_off;                  // the byte offset in shared memory of r and s (rem_max doubles each)
     DevStatus* status;
     CgOut* out;
     const int* cta_inst;         // batched launch: instance of each CTA (else null)
@@ -197,6 +208,9 @@ public:
     unsigned short* d_lcol = nullptr;
     int *d_rem_ptr = nullptr, *d_own = nullptr;   // remote halo entries and own rows' places (k_pcg64c)
     int2* d_rem = nullptr;
+    bool cgcg_rg = false;    // the remote entries' state is in global memory
+    int cgcg_rs_off = 0;     // ... but r and s in shared memory from there on
+    RemoteState* d_rem_state = nullptr;
     int dev_rem_max = 0;
     long long rem_total = 0;      // remote halo entries over all CTAs (k_pcg64c)
     int cluster = 0;         // >0: the CG-CG kernel runs on one cluster of that many CTAs
@@ -286,6 +300,10 @@ private:
         PcgInst* d_inst = nullptr;
         int *d_hptr = nullptr, *d_hidx = nullptr, *d_rptr = nullptr;
         int2* d_rem = nullptr;
+        bool rg = false;
+        int lcs_off = 0, rs_off = 0;
+        RemoteState* d_rem_state = nullptr;
+        double* d_rem_rs = nullptr;
     };
     void free_waves();
     std::vector<PcgBatchMember> mem;

@@ -437,10 +437,13 @@ cbs3d_status cbs3d_probe_halo_placement(int nh, int nslices, const long long* sl
  * the PCG engine splits them: coord (3*npoin, may be NULL as for the
  * coordinate-free pressure solver) sets the rows' order.  Returns the largest
  * halo, slots, remote halo entries and neighbours of a CTA and the dynamic
- * shared memory in bytes that the engine allocates to the two-level kernel. */
+ * shared memory in bytes that the engine allocates to the two-level kernel
+ * and, before its optional parts, to the single-reduction one, whose form is 0
+ * with the remote entries' state in shared memory, 1 with r and s of them
+ * there, 2 with all of it in global memory, -1 where none fits. */
 typedef struct cbs3d_pcg_partition {
-    int ctas, halo_max, slot_max, remote_max, neighbour_max;
-    long long two_level_bytes;
+    int ctas, halo_max, slot_max, remote_max, neighbour_max, single_form;
+    long long two_level_bytes, single_bytes;
 } cbs3d_pcg_partition;
 cbs3d_status cbs3d_probe_pcg_partition(int nelem, int npoin, const int* intma, const int* mat_elem,
                                        const double* coord, int ctas, cbs3d_pcg_partition* out);

@@ -191,3 +191,18 @@ def test_mixed_batch_is_no_slower_than_the_fp64_batch():
     for i in range(len(cs)):
         (u0, p0, _), (u1, p1, _) = a.fields(i), m.fields(i)
         assert rel_l2(u1, u0) <= MIXED_TOL and rel_l2(p1, p0) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("rows,spread", [(4, True), (8, False)])
+def test_batch_of_a_thin_channel(rows, spread):
+    """A long channel, most of whose halos are remote, alone in a batch (CTAs
+    of 512 threads; of 256 with eight rows per thread): as on its own, to the
+    solves' tolerance."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.channel(900, 16, 16, length=56.0, ntime=10 ** 6)
+    b, a = gpu.Batch([case], autotune=False, rows_per_thread=rows, spread=spread), gpu.Context(case)
+    b.step(2)
+    a.step(2)
+    for x, y in zip(b.fields(0)[:2], a.fields()[:2]):
+        assert rel_l2(x, y) <= RUN_TOL

@@ -3,6 +3,7 @@ to six rows per thread, grids of a few CTAs) against the global-vector
 single-reduction kernel, which performs the same operations row by row with
 its vectors in global memory: fields and iteration counts agree bit for bit.
 Their grids are the same, so no tolerance is involved."""
+import numpy as np
 import pytest
 
 from helpers import bitwise, rel_l2
@@ -134,3 +135,50 @@ def test_two_level_kernel_at_eight_rows_per_thread():
     assert sa.pcg_kernel == 6
     assert sa.cg.iterations < sb.cg.iterations
     assert rel_l2(a.fields()[1], b.fields()[1]) <= 1e-8
+
+
+def test_thin_channel_stays_on_the_register_kernel():
+    """A long channel's halos are mostly remote: their state is read from
+    global memory, row by row the operations of the global-vector kernel."""
+    from cbs3d import cases
+    _same(cases.channel(900, 16, 16, length=56.0, ntime=10 ** 6), steps=1)
+
+
+# tetrahedra between random nodes, so that nearly all columns are remote: about
+# 13, 9 and 6 neighbours at one, two and three rows per thread; the box in
+# breadth-first order at four
+@pytest.mark.parametrize("rows,tets_per_node", [(1, 4.5), (2, 3.0), (3, 2.0), (4, None)])
+def test_remote_entries_in_global_memory(rows, tets_per_node):
+    """The solved pressure against the operator restated here: the residual is
+    the solve's 1e-10 and rounding (well-conditioned operators, sums of 1e5)."""
+    from cbs3d import cases
+    from test_pcg_partition import partition
+    gpu = _gpu()
+    rng = np.random.default_rng(rows)
+    if tets_per_node is None:
+        mesh = cases.box_mesh(64, 64, 64)
+    else:
+        n = 148 * 512 * rows - 4000
+        nodes = np.concatenate([rng.permutation(n) for _ in range(int(np.ceil(tets_per_node)))])
+        intma = nodes[:int(n * tets_per_node / 4) * 4].reshape(-1, 4)
+        intma = np.concatenate([intma, [[n - 1, 0, 1, 2]]])
+        intma = intma[[len(set(t)) == 4 for t in intma.tolist()]]
+        mesh = cases.Mesh(coord=np.zeros((n, 3)), intma=(intma + 1).astype(np.int32), bfaces=None, lattice=None, shape=())
+    assert partition(mesh, 148, coord=False).single_form == 1
+    it, n = mesh.intma - 1, mesh.npoin
+    w = -rng.uniform(0.5, 1.5, (it.shape[0], 6))
+    pairs = ((0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3))
+    diag = np.ones(n)
+    for k, (a, b) in enumerate(pairs):
+        diag -= np.bincount(it[:, a], w[:, k], n) + np.bincount(it[:, b], w[:, k], n)
+    rhs = rng.standard_normal(n)
+    solver = gpu.PressureSolver(mesh.intma, None, np.array([1]), np.array([0.0]))
+    for _ in range(2):
+        x, _, _, res = solver.solve(w, diag, rhs, np.zeros(n))
+        assert res["status"] == 0 and res["iterations"] > 5
+        r = rhs - diag * x
+        for k, (a, b) in enumerate(pairs):
+            r -= np.bincount(it[:, a], w[:, k] * x[it[:, b]], n) + np.bincount(it[:, b], w[:, k] * x[it[:, a]], n)
+        assert x[0] == 0.0
+        assert np.linalg.norm(r[1:]) <= 1e-9 * np.linalg.norm(rhs)
+    solver.close()

@@ -8,8 +8,8 @@ import pytest
 
 
 class Partition(ctypes.Structure):
-    _fields_ = [(n, ctypes.c_int) for n in ("ctas", "halo_max", "slot_max", "remote_max", "neighbour_max")] + [
-        ("two_level_bytes", ctypes.c_longlong)]
+    _fields_ = [(n, ctypes.c_int) for n in ("ctas", "halo_max", "slot_max", "remote_max", "neighbour_max", "single_form")] + [
+        ("two_level_bytes", ctypes.c_longlong), ("single_bytes", ctypes.c_longlong)]
 
 
 def partition(mesh, ctas=148, coord=True):
@@ -40,3 +40,16 @@ def test_two_level_kernel_has_the_shared_memory_it_addresses(shape, ctas):
     need += 8 * (p.neighbour_max * p.ctas + 3 * p.ctas + p.neighbour_max)
     need += p.halo_max   # every entry's owner
     assert p.two_level_bytes >= need
+
+
+# thin meshes and orders without coordinates, whose halos are mostly remote
+@pytest.mark.parametrize("shape,coord", [((900, 16, 16), True), ((64, 64, 64), False), ((66, 66, 66), False),
+                                         ((64, 64, 64), True)])
+def test_single_reduction_kernel_has_a_form_that_fits(shape, coord):
+    from cbs3d import cases
+    p = partition(cases.box_mesh(*shape), 148, coord)
+    assert p.single_form == (0 if coord and shape[0] == 64 else 1)
+    # z per halo entry; per remote entry r, s and, in the first form, inverse
+    # diagonal, position (4) and place (2); columns
+    need = 8 * p.halo_max + (30 if p.single_form == 0 else 16) * p.remote_max + 2 * p.slot_max
+    assert need <= p.single_bytes <= 220 * 1024
