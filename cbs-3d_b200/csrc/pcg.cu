@@ -3579,6 +3579,55 @@ Partition partition_rows(const PressurePattern& P, const std::vector<int>& colp,
     return o;
 }
 
+// Halos of the global-vector kernels: each CTA's slices in the fewest parts (at
+// most 8) of which each part's halo (16 bytes an entry) fits shared memory, the
+// single-reduction kernel's table of the CTA's slices behind it included.
+struct GlobalHalo {
+    int parts = 0;           // 0: none fits
+    int hmax = 0;
+    size_t table = 0, table_bytes = 0;   // offset and size of the slice table
+    std::vector<int> hptr, hidx;
+    std::vector<unsigned short> lcol;
+};
+// 227 KB less the kernels' static shared memory (2,064 bytes)
+constexpr size_t GLOBAL_SMEM_MAX = 229888;
+GlobalHalo global_halo_in_parts(const PressurePattern& P, const std::vector<int>& colp, int g, bool with_table)
+{
+    GlobalHalo o;
+    o.lcol.assign(static_cast<size_t>(P.nslots), 0);
+    o.table_bytes = with_table ? static_cast<size_t>((P.nslices + g - 1) / g) * sizeof(int2) : 0;
+    std::vector<int> cols;
+    for (int kp = 1; kp <= 8 && o.parts == 0; ++kp) {
+        o.hptr.assign(static_cast<size_t>(g) * kp + 1, 0);
+        o.hidx.clear();
+        o.hmax = 0;
+        bool fits = true;
+        for (int bb = 0; bb < g && fits; ++bb) {
+            const int sb = static_cast<int>(static_cast<long long>(bb) * P.nslices / g);
+            const int se = static_cast<int>(static_cast<long long>(bb + 1) * P.nslices / g);
+            for (int q = 0; q < kp && fits; ++q) {
+                const int pb = sb + static_cast<int>(static_cast<long long>(q) * (se - sb) / kp);
+                const int pe = sb + static_cast<int>(static_cast<long long>(q + 1) * (se - sb) / kp);
+                const long long a0 = P.slice_off[static_cast<size_t>(pb)], a1 = P.slice_off[static_cast<size_t>(pe)];
+                cols.assign(colp.begin() + a0, colp.begin() + a1);
+                std::sort(cols.begin(), cols.end());
+                cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
+                const size_t bytes = cols.size() * 16 + 16;
+                if (cols.size() > 65535 || bytes > 220 * 1024 || bytes + o.table_bytes > GLOBAL_SMEM_MAX) { fits = false; break; }
+                for (long long t = a0; t < a1; ++t)
+                    o.lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(
+                        std::lower_bound(cols.begin(), cols.end(), colp[static_cast<size_t>(t)]) - cols.begin());
+                o.hidx.insert(o.hidx.end(), cols.begin(), cols.end());
+                o.hptr[static_cast<size_t>(bb) * kp + q + 1] = static_cast<int>(o.hidx.size());
+                o.hmax = std::max(o.hmax, static_cast<int>(cols.size()));
+            }
+        }
+        if (fits) o.parts = kp;
+    }
+    o.table = static_cast<size_t>(o.hmax) * 16 + 16;
+    return o;
+}
+
 // Columns as row positions: the solver works in row-position order.
 std::vector<int> columns_by_position(const PressurePattern& P, int N)
 {
@@ -3730,14 +3779,23 @@ cbs3d_status probe_partition(int nelem, int npoin, const int* intma, const int* 
     build_pressure_pattern(conn, mat, npoin, n2e_ptr, n2e, P, coord);
     const int g = std::min(ctas, P.nslices);
     const Partition part = partition_rows(P, columns_by_position(P, npoin), g, PCG_THREADS / 32);
-    if (!part.fits) return CBS3D_INVALID_INPUT;
+    const GlobalHalo gh = global_halo_in_parts(P, columns_by_position(P, npoin), g, true);
+    *out = cbs3d_pcg_partition{};
+    out->ctas = g;
+    out->single_form = -1;
+    out->global_parts = gh.parts;
+    out->global_bytes = static_cast<long long>(gh.table + gh.table_bytes);
+    if (!part.fits) return CBS3D_OK;
     const CoarseNeighbours nb = coarse_neighbours(P.nslices, part.hptr, part.hidx);
     const int hmax = part.hmax + 1;   // the spare place
     const CgcgLayout lay(hmax, part.remote.most, part.lcsb, CGCG_SMEM_MAX);
-    *out = cbs3d_pcg_partition{g, hmax, static_cast<int>(part.smax), part.remote.most, nb.most,
-                               lay.bytes > CGCG_SMEM_MAX ? -1 : !lay.rg ? 0 : lay.rs ? 1 : 2,
-                               static_cast<long long>(TwoLevelLayout(hmax, static_cast<int>(part.smax), nb.most, g).bytes),
-                               static_cast<long long>(lay.bytes)};
+    out->halo_max = hmax;
+    out->slot_max = static_cast<int>(part.smax);
+    out->remote_max = part.remote.most;
+    out->neighbour_max = nb.most;
+    out->single_form = lay.bytes > CGCG_SMEM_MAX ? -1 : !lay.rg ? 0 : lay.rs ? 1 : 2;
+    out->two_level_bytes = static_cast<long long>(TwoLevelLayout(hmax, out->slot_max, nb.most, g).bytes);
+    out->single_bytes = static_cast<long long>(lay.bytes);
     return CBS3D_OK;
 }
 
@@ -4096,47 +4154,17 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         // memory: each CTA's slices in the fewest parts (at most 8) whose
         // halos fit
         const int g = nblocks;
-        std::vector<int> hptr, hidx, cols;
-        std::vector<unsigned short> lcol(static_cast<size_t>(nslots), 0);
-        int hmax = 0;
-        bool fits = false;
-        for (int kp = 1; kp <= 8 && !fits; ++kp) {
-            hptr.assign(static_cast<size_t>(g) * kp + 1, 0);
-            hidx.clear();
-            hmax = 0;
-            fits = true;
-            for (int bb = 0; bb < g && fits; ++bb) {
-                const int sb = static_cast<int>(static_cast<long long>(bb) * nslices / g);
-                const int se = static_cast<int>(static_cast<long long>(bb + 1) * nslices / g);
-                for (int q = 0; q < kp && fits; ++q) {
-                    const int pb = sb + static_cast<int>(static_cast<long long>(q) * (se - sb) / kp);
-                    const int pe = sb + static_cast<int>(static_cast<long long>(q + 1) * (se - sb) / kp);
-                    const long long a0 = P.slice_off[static_cast<size_t>(pb)], a1 = P.slice_off[static_cast<size_t>(pe)];
-                    cols.assign(colp.begin() + a0, colp.begin() + a1);
-                    std::sort(cols.begin(), cols.end());
-                    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-                    if (cols.size() > 65535 || cols.size() * 16 + 16 > 220 * 1024) { fits = false; break; }
-                    for (long long t = a0; t < a1; ++t)
-                        lcol[static_cast<size_t>(t)] = static_cast<unsigned short>(
-                            std::lower_bound(cols.begin(), cols.end(), colp[static_cast<size_t>(t)]) - cols.begin());
-                    hidx.insert(hidx.end(), cols.begin(), cols.end());
-                    hptr[static_cast<size_t>(bb) * kp + q + 1] = static_cast<int>(hidx.size());
-                    hmax = std::max(hmax, static_cast<int>(cols.size()));
-                }
-            }
-            if (fits) global_halo_parts = kp;
-        }
         // automatic and choice 5: the single-reduction kernel; choice 1:
         // the two-reduction one (bitwise the same arithmetic as choices 2, 3)
         global_cgcg = kernel_choice != 1;
         const void* fh = global_cgcg ? reinterpret_cast<const void*>(k_pcg64g) : reinterpret_cast<const void*>(k_pcg64<true>);
-        size_t smem = static_cast<size_t>(hmax) * 16 + 16;
+        const GlobalHalo H = global_halo_in_parts(P, colp, g, global_cgcg);
+        const size_t smem = H.table + H.table_bytes;
         // the slices' slots and widths behind the halo, and rows per warp in
         // tensor memory: rounds of eight slots, 2.5 columns per slot of 128
         cgcg_tm_w = g_tm_rows = cgcg_lcs = 0;
         if (global_cgcg) {
-            cgcg_lcs = static_cast<int>(smem);
-            smem += static_cast<size_t>((nslices + g - 1) / g) * sizeof(int2);
+            cgcg_lcs = static_cast<int>(H.table);
             int wmx = 0;
             for (int q = 0; q < nslices; ++q) wmx = std::max(wmx, P.slice_w[static_cast<size_t>(q)]);
             const int tw = (wmx + 7) / 8 * 8;
@@ -4146,18 +4174,19 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             }
         }
         int per = 0;
-        if (fits && raise_smem_limit(fh, smem) == cudaSuccess &&
+        if (H.parts > 0 && raise_smem_limit(fh, smem) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fh, PCG_THREADS, smem) == cudaSuccess && per * sms >= g) {
-            d_halo_ptr = dalloc<int>(hptr.size());
-            d_halo_idx = dalloc<int>(hidx.size());
-            d_lcol = dalloc<unsigned short>(lcol.size());
-            CUDA_OK(cudaMemcpy(d_halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CUDA_OK(cudaMemcpy(d_halo_idx, hidx.data(), hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CUDA_OK(cudaMemcpy(d_lcol, lcol.data(), lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
-            dev_halo_max = hmax;
+            d_halo_ptr = dalloc<int>(H.hptr.size());
+            d_halo_idx = dalloc<int>(H.hidx.size());
+            d_lcol = dalloc<unsigned short>(H.lcol.size());
+            CUDA_OK(cudaMemcpy(d_halo_ptr, H.hptr.data(), H.hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+            CUDA_OK(cudaMemcpy(d_halo_idx, H.hidx.data(), H.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
+            CUDA_OK(cudaMemcpy(d_lcol, H.lcol.data(), H.lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+            dev_halo_max = H.hmax;
+            global_halo_parts = H.parts;
             global_halo = true;
             global_halo_smem = smem;
-            global_halo_total = static_cast<long long>(hidx.size());
+            global_halo_total = static_cast<long long>(H.hidx.size());
         } else {
             cgcg_tm_w = g_tm_rows = cgcg_lcs = 0;
         }

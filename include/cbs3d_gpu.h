@@ -440,10 +440,12 @@ cbs3d_status cbs3d_probe_halo_placement(int nh, int nslices, const long long* sl
  * shared memory in bytes that the engine allocates to the two-level kernel
  * and, before its optional parts, to the single-reduction one, whose form is 0
  * with the remote entries' state in shared memory, 1 with r and s of them
- * there, 2 with all of it in global memory, -1 where none fits. */
+ * there, 2 with all of it in global memory, -1 where none fits (the other
+ * figures are 0 where a halo passes 65,535 entries); and the
+ * global-vector kernel's parts per CTA (0 where none fit) and bytes. */
 typedef struct cbs3d_pcg_partition {
-    int ctas, halo_max, slot_max, remote_max, neighbour_max, single_form;
-    long long two_level_bytes, single_bytes;
+    int ctas, halo_max, slot_max, remote_max, neighbour_max, single_form, global_parts;
+    long long two_level_bytes, single_bytes, global_bytes;
 } cbs3d_pcg_partition;
 cbs3d_status cbs3d_probe_pcg_partition(int nelem, int npoin, const int* intma, const int* mat_elem,
                                        const double* coord, int ctas, cbs3d_pcg_partition* out);

@@ -182,3 +182,15 @@ def test_remote_entries_in_global_memory(rows, tets_per_node):
         assert x[0] == 0.0
         assert np.linalg.norm(r[1:]) <= 1e-9 * np.linalg.norm(rhs)
     solver.close()
+
+
+def test_global_vector_kernel_takes_one_more_part_for_its_slice_table():
+    """Two CTAs for 49^3: six halo parts per CTA fit shared memory, but not
+    with the table of its 1,954 slices, so it takes seven."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(49, re=400.0, ntime=10 ** 6, jitter=0.15, seed=1234)
+    a, b = gpu.Context(case), gpu.Context(case, pcg_kernel=5, pcg_blocks=2)
+    a.step(1)
+    assert b.step(1).pcg_kernel == 8
+    assert rel_l2(b.fields()[1], a.fields()[1]) <= 1e-8

@@ -8,8 +8,9 @@ import pytest
 
 
 class Partition(ctypes.Structure):
-    _fields_ = [(n, ctypes.c_int) for n in ("ctas", "halo_max", "slot_max", "remote_max", "neighbour_max", "single_form")] + [
-        ("two_level_bytes", ctypes.c_longlong), ("single_bytes", ctypes.c_longlong)]
+    _fields_ = [(n, ctypes.c_int) for n in ("ctas", "halo_max", "slot_max", "remote_max", "neighbour_max", "single_form",
+                                             "global_parts")] + [
+        (n, ctypes.c_longlong) for n in ("two_level_bytes", "single_bytes", "global_bytes")]
 
 
 def partition(mesh, ctas=148, coord=True):
@@ -53,3 +54,13 @@ def test_single_reduction_kernel_has_a_form_that_fits(shape, coord):
     # diagonal, position (4) and place (2); columns
     need = 8 * p.halo_max + (30 if p.single_form == 0 else 16) * p.remote_max + 2 * p.slot_max
     assert need <= p.single_bytes <= 220 * 1024
+
+
+# two CTAs (or three): many slices each, and halos of one part fewer that fit
+# without the slice table (216,352 bytes and a table of 15,632 at 49^3)
+@pytest.mark.parametrize("n,ctas,parts", [(49, 2, 7), (51, 2, 8), (53, 3, 6), (48, 2, 6)])
+def test_global_vector_kernel_counts_its_slice_table(n, ctas, parts):
+    from cbs3d import cases
+    p = partition(cases.box_mesh(n, n, n), ctas)
+    assert p.global_parts == parts
+    assert p.global_bytes <= 227 * 1024 - 2064   # the SM's limit less the kernel's static shared memory
