@@ -992,6 +992,17 @@ cbs3d_status cbs3d_probe_pcg_partition(int nelem, int npoin, const int* intma, c
     }
 }
 
+cbs3d_status cbs3d_selftest_waits(int device, int form, int* incomplete_status, int* complete_status, int* sums_ok)
+{
+    try {
+        return selftest_waits(device, form, incomplete_status, complete_status, sums_ok);
+    } catch (const Error& e) {
+        return e.code;
+    } catch (const std::exception&) {
+        return CBS3D_INTERNAL;
+    }
+}
+
 cbs3d_status cbs3d_selftest_wait_timeout(int device, int* observed_status)
 {
     try {

@@ -124,42 +124,4 @@ __device__ __forceinline__ int ld_relaxed_int(const int* p)
     return v;
 }
 
-// Grid-wide barrier for a cooperatively launched grid.  Every wait is
-// bounded: after ~2^31 SM cycles (about a second) the CTA records
-// CBS3D_TIMEOUT in the status word and returns false; a CTA that sees any
-// failure recorded by another CTA also returns false, so the whole grid
-// leaves the kernel.  count/gen live in device memory zeroed before launch.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned* gen, unsigned nblocks,
-                                             DevStatus* st, int stage)
-{
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned g = ld_acquire(gen);
-        __threadfence();
-        const unsigned arrived = atomicAdd(count, 1u);
-        if (arrived == nblocks - 1) {
-            atomicExch(count, 0u);
-            __threadfence();
-            atomicAdd(gen, 1u);
-        } else {
-            const long long t0 = clock64();
-            while (ld_acquire(gen) == g) {
-                if (ld_relaxed_int(&st->code) != 0) { ok = 0; break; }
-                if (clock64() - t0 > (1LL << 31)) {
-                    set_status(st, 5 /*CBS3D_TIMEOUT*/, stage, 0, R_PCG_BARRIER);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        if (ok && ld_relaxed_int(&st->code) != 0) ok = 0;
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 }  // namespace cbs3d

@@ -1073,6 +1073,17 @@ struct SpinLimit {
     }
 };
 
+// Waits for the record tagged `want` (v, t: what the last poll returned).
+__device__ __forceinline__ bool tag_wait(const TagVal* p, unsigned long long want, double& v, unsigned long long& t,
+                                         SpinLimit& lim, DevStatus* status)
+{
+    while (t != want) {
+        if (lim.expired(status)) return false;
+        ld_tag(p, v, t);
+    }
+    return true;
+}
+
 // The maximum is taken over the bits of magnitudes, whose order is that of
 // the values with infinities and NaN above every finite one: a non-finite
 // entry anywhere shows in the total.
@@ -1291,6 +1302,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
                  : "r"(bar), "r"(parity)
                  : "memory");
     return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, DevStatus* status)
+{
+    SpinLimit lim;
+    while (!mbar_try_wait(bar, parity))
+        if (lim.expired(status)) return false;
+    return true;
 }
 __device__ __forceinline__ void cluster_sync()
 {
@@ -2143,10 +2161,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
             for (int u = 0; u < RP; ++u) {
                 const int e = e0 + u * NT;
                 if (e < nr) {
-                    while (xt[u] != want) {
-                        if (lim.expired(comm.status)) { ok = false; break; }
-                        ld_tag(o + row_of(e), xv[u], xt[u]);
-                    }
+                    if (xt[u] != want && !tag_wait(o + row_of(e), want, xv[u], xt[u], lim, comm.status)) ok = false;
                     use(e, xv[u]);
                 }
             }
@@ -2182,9 +2197,7 @@ __device__ __forceinline__ void pcg64c_body(const PcgDev& D, uint32_t tm, unsign
         if constexpr (CL) {
             const int par = phase & 1;
             const uint32_t bar = smem_addr(&cs.bar[par]);
-            SpinLimit lim;
-            while (!mbar_try_wait(bar, (phase >> 1) & 1))
-                if (lim.expired(comm.status)) { ok = false; break; }
+            if (!mbar_wait(bar, (phase >> 1) & 1, comm.status)) ok = false;
             const int q = lane & 3;
             double a0 = cs.part[par][lane >> 2][q], a1 = cs.part[par][(lane >> 2) + 8][q];
 #pragma unroll
@@ -3214,32 +3227,137 @@ __global__ void __launch_bounds__(512, 1) k_coarse_invert_reg(int G, double* ac)
         }
 }
 
-// Self-test of the bounded device wait: CTA 0 leaves without arriving, so the
-// other CTAs' barrier waits can only end by running out of their spin limit.
-__global__ void k_barrier_selftest(unsigned* bar, DevStatus* st)
+// Self-test of the solvers' bounded waits: CTA `missing` leaves its part of one
+// exchange out, so that the others' waits can only end by their limit (a
+// second); with missing < 0 the exchange is complete and out[CTA] gets its sum.
+// 0: the counter all-reduce; 1: the tagged all-reduce; 2: one row's tagged
+// record, whose failed wait goes through the all-reduce after it as in
+// k_pcg64c; 3: the cluster's mbarrier, every CTA staying to the end.
+enum { WAIT_COUNTER, WAIT_TAGGED, WAIT_ROW, WAIT_CLUSTER, WAIT_FORMS };
+template <int FORM>
+__global__ void __launch_bounds__(512, 1) k_wait_selftest(PcgDev D, int missing, double* out)
 {
-    if (blockIdx.x == 0) return;
-    grid_barrier(bar, bar + 1, gridDim.x, st, ST_PCG);
+    constexpr int NT = 512;
+    const SegView g = seg_view<false>(D);
+    const int b = g.b, G = g.G;
+    bool ok = false;
+    if constexpr (FORM == WAIT_COUNTER) {
+        if (b == missing) return;
+        double v[1] = {1.0}, o[1];
+        ok = grid_allreduce_v<1, 1, NT>(v, D, g, 0, o);
+        if (ok && threadIdx.x == 0) out[b] = o[0];
+    } else {
+        unsigned long long epoch;
+        if (!tag_begin<false>(D, epoch)) return;
+        const TagComm comm = tag_comm(D, g, epoch);
+        const double v[4] = {1.0, 0.0, 0.0, 0.0};
+        double t[4] = {0.0, 0.0, 0.0, 0.0};
+        PollHold hold;
+        if constexpr (FORM == WAIT_TAGGED) {
+            if (b != missing) {
+                tag_allreduce_publish<NT, false, false>(comm, 0, v);
+                ok = tag_allreduce_wait<NT, false, false>(comm, 0, t, true, hold, [] {});
+            }
+        } else if constexpr (FORM == WAIT_ROW) {
+            if (b != missing && threadIdx.x == 0) st_tag(D.xw + b, 0.0, comm.tag(0));
+            double x = 0.0;
+            unsigned long long xt = 0;
+            SpinLimit lim;
+            const bool got = threadIdx.x != 0 || tag_wait(D.xw + (b + 1) % G, comm.tag(0), x, xt, lim, comm.status);
+            tag_allreduce_publish<NT, false, false>(comm, 0, v);
+            ok = tag_allreduce_wait<NT, false, false>(comm, 0, t, got, hold, [] {});
+            // the CTA whose record never came is not there for the next one
+            if (ok) {
+                tag_allreduce_publish<NT, false, false>(comm, 1, v);
+                ok = tag_allreduce_wait<NT, false, false>(comm, 1, t, true, hold, [] {});
+            }
+        } else {
+            __shared__ ClusterShared cs;
+            const uint32_t bar = smem_addr(&cs.bar[0]);
+            if (threadIdx.x == 0) mbar_init(bar);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            cluster_sync();
+            if (threadIdx.x == NT - 1) mbar_expect(bar, 32u * G);
+            cta_reduce4<NT, false>(v, [&](int q, int j, double x) {
+                const uint32_t at = smem_addr(&cs.part[0][b][q]);
+                for (int c = j; c < G && b != missing; c += 8) st_async_f64(cluster_addr(at, c), x, cluster_addr(bar, c));
+            });
+            ok = __syncthreads_and(mbar_wait(bar, 0, comm.status));
+            if (ok)
+                for (int c = 0; c < G; ++c) t[0] += cs.part[0][c][0];
+            cluster_sync();
+        }
+        if (ok && threadIdx.x == 0) out[b] = t[0];
+        tag_end<false>(D, epoch);
+    }
 }
 
 }  // namespace
 
+cbs3d_status selftest_waits(int device, int form, int* incomplete, int* complete, int* sums_ok)
+{
+    if (form < 0 || form >= WAIT_FORMS || !incomplete || !complete || !sums_ok) return CBS3D_INVALID_INPUT;
+    CUDA_OK(cudaSetDevice(device));
+    constexpr int G = 4;
+    const void* fns[WAIT_FORMS] = {reinterpret_cast<const void*>(k_wait_selftest<WAIT_COUNTER>),
+                                   reinterpret_cast<const void*>(k_wait_selftest<WAIT_TAGGED>),
+                                   reinterpret_cast<const void*>(k_wait_selftest<WAIT_ROW>),
+                                   reinterpret_cast<const void*>(k_wait_selftest<WAIT_CLUSTER>)};
+    PcgDev D{};
+    D.N = D.nslices = G;
+    const unsigned long long one = 1;
+    D.rec = dalloc<TagVal>(G * 2 * REC_STRIDE);
+    D.xw = dalloc<TagVal>(2 * G);
+    D.epoch = dalloc<unsigned long long>(1);
+    D.bar = dalloc<unsigned>(4);
+    D.part = dalloc<double>(G * 16);
+    D.status = dalloc<DevStatus>(1);
+    double* out = dalloc<double>(G);
+    CUDA_OK(cudaMemset(D.rec, 0, G * 2 * REC_STRIDE * sizeof(TagVal)));
+    CUDA_OK(cudaMemset(D.xw, 0, 2 * G * sizeof(TagVal)));
+    CUDA_OK(cudaMemcpy(D.epoch, &one, sizeof one, cudaMemcpyHostToDevice));
+    // the incomplete exchange, then the complete one on the same records
+    double sums[G] = {};
+    for (int missing : {1, -1}) {
+        CUDA_OK(cudaMemset(D.bar, 0, 4 * sizeof(unsigned)));
+        CUDA_OK(cudaMemset(D.status, 0, sizeof(DevStatus)));
+        CUDA_OK(cudaMemset(out, 0, G * sizeof(double)));
+        void* args[] = {&D, &missing, &out};
+        if (form == WAIT_CLUSTER) {
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = G;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(G);
+            cfg.blockDim = dim3(512);
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            CUDA_OK(cudaLaunchKernelExC(&cfg, fns[form], args));
+        } else {
+            CUDA_OK(cudaLaunchCooperativeKernel(fns[form], dim3(G), dim3(512), args, 0, nullptr));
+        }
+        CUDA_OK(cudaDeviceSynchronize());
+        DevStatus h{};
+        CUDA_OK(cudaMemcpy(&h, D.status, sizeof h, cudaMemcpyDeviceToHost));
+        (missing < 0 ? *complete : *incomplete) = h.code;
+        CUDA_OK(cudaMemcpy(sums, out, sizeof sums, cudaMemcpyDeviceToHost));
+        const bool none = missing >= 0;   // no CTA may have gone on
+        bool right = true;
+        for (double x : sums) right = right && x == (none ? 0.0 : 512.0 * G);
+        *sums_ok = (none || *sums_ok) && right;
+    }
+    void* ptrs[] = {D.rec, D.xw, D.epoch, D.bar, D.part, D.status, out};
+    for (void* q : ptrs) cudaFree(q);
+    return CBS3D_OK;
+}
+
 cbs3d_status selftest_wait_timeout(int device, int* observed)
 {
-    CUDA_OK(cudaSetDevice(device));
-    unsigned* bar = dalloc<unsigned>(2);
-    DevStatus* st = dalloc<DevStatus>(1);
-    CUDA_OK(cudaMemset(bar, 0, 2 * sizeof(unsigned)));
-    CUDA_OK(cudaMemset(st, 0, sizeof(DevStatus)));
-    k_barrier_selftest<<<4, 32>>>(bar, st);
-    CUDA_OK(cudaGetLastError());
-    CUDA_OK(cudaDeviceSynchronize());
-    DevStatus h{};
-    CUDA_OK(cudaMemcpy(&h, st, sizeof h, cudaMemcpyDeviceToHost));
-    cudaFree(bar);
-    cudaFree(st);
-    if (observed) *observed = h.code;
-    return CBS3D_OK;
+    int complete = 0, sums_ok = 0, code = 0;
+    const cbs3d_status rc = selftest_waits(device, WAIT_COUNTER, &code, &complete, &sums_ok);
+    if (observed) *observed = code;
+    return rc;
 }
 
 namespace {

@@ -340,8 +340,11 @@ private:
 // 512-thread CTA per SM, `iters` back-to-back all-reduces, CUDA events).
 cbs3d_status allreduce_probe(int device, int iters, double* us);
 
-// Launches a grid whose barrier can never complete and reports the status
-// the bounded waits recorded (CBS3D_TIMEOUT when they ran out as designed).
+// Launches an exchange of the given form that can never complete and reports
+// the status the bounded waits recorded (CBS3D_TIMEOUT when they ran out as
+// designed), then a complete one on the same records: its status, and whether
+// every CTA had the sum then and none had one before.
+cbs3d_status selftest_waits(int device, int form, int* incomplete, int* complete, int* sums_ok);
 cbs3d_status selftest_wait_timeout(int device, int* observed);
 
 // Inverts a g x g host matrix with the coarse-operator Gauss-Jordan kernels

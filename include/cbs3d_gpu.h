@@ -389,11 +389,17 @@ cbs3d_status cbs3d_batch_get_info(const cbs3d_batch* b, cbs3d_batch_info* info);
 void cbs3d_batch_destroy(cbs3d_batch* b);
 const char* cbs3d_batch_last_error(const cbs3d_batch* b);
 
-/* Failure-detection self-test (no reference counterpart): launches a small
- * grid whose grid barrier can never complete and returns, in
- * *observed_status, the status its bounded device waits recorded --
- * CBS3D_TIMEOUT after about a second.  The device stays usable. */
+/* Failure-detection self-tests (no reference counterpart).
+ * cbs3d_selftest_wait_timeout launches a small grid whose all-reduce can never
+ * complete and returns, in *observed_status, the status its bounded device
+ * waits recorded -- CBS3D_TIMEOUT after about a second.  The device stays
+ * usable.  cbs3d_selftest_waits does so for each of the solvers' exchanges
+ * (form 0: the all-reduce on a counter, 1: on tagged records, 2: one row's
+ * tagged record, 3: the cluster's mbarrier) and then runs a complete exchange
+ * on the same records: *complete_status is its status, *sums_ok 1 when every
+ * CTA had the right sum then and none went on before. */
 cbs3d_status cbs3d_selftest_wait_timeout(int device, int* observed_status);
+cbs3d_status cbs3d_selftest_waits(int device, int form, int* incomplete_status, int* complete_status, int* sums_ok);
 
 /* Dense inverse of a g x g row-major matrix by the device Gauss-Jordan
  * kernels that invert the two-level preconditioner's aggregated operator

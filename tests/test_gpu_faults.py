@@ -65,3 +65,16 @@ def test_device_wait_times_out_and_device_stays_usable():
     case, _ = load_case(fixture_path("cav4"))
     c = gpu.Context(case)
     c.step(1)
+
+
+@pytest.mark.parametrize("form", ["counter", "tagged", "row", "cluster"])
+def test_every_exchange_times_out_and_works_again(form):
+    """A CTA leaves its part of an exchange out: the others' waits run out and
+    every CTA leaves; the next exchange on the same records is whole."""
+    import ctypes
+    gpu = _gpu()
+    code, after, sums = ctypes.c_int(-1), ctypes.c_int(-1), ctypes.c_int(-1)
+    forms = ["counter", "tagged", "row", "cluster"]
+    rc = gpu.lib().cbs3d_selftest_waits(0, forms.index(form), ctypes.byref(code), ctypes.byref(after), ctypes.byref(sums))
+    assert rc == 0
+    assert (code.value, after.value, sums.value) == (5, 0, 1)
