@@ -1186,12 +1186,18 @@ struct PollHold {
     }
 };
 
+// Records polled per thread, and the largest grid that covers: 256 CTAs of 512
+// threads, 320 of 256.  A record past it would be left out of every sum, so the
+// host keeps the grids of these kernels within it.
+constexpr int tag_records(int nt) { return nt >= 512 ? 2 : 5; }
+constexpr int tag_grid_max(int nt) { return tag_records(nt) * (nt / 4); }
+
 template <int NT, bool ORDERED, bool MX, typename F>
 __device__ __forceinline__ bool tag_allreduce_wait(const TagComm& c, int phase, double (&out)[4], bool ok, PollHold& hold,
                                                    F&& all_in)
 {
     constexpr int NW = NT / 32, STEP = NT / 4;
-    constexpr int MP = NT >= 512 ? 2 : 5;   // records per thread: grids of up to 256 or 320 CTAs
+    constexpr int MP = tag_records(NT);
     __shared__ double sm[NW][4];
     const int lane = threadIdx.x & 31, q = threadIdx.x & 3, j = threadIdx.x >> 2;
     const TagVal* r = c.rec + ((phase & 1) * c.G + j) * REC_STRIDE + q;
@@ -3386,6 +3392,7 @@ cbs3d_status allreduce_probe(int device, int iters, double* us)
     CUDA_OK(cudaSetDevice(device));
     int sms = 0;
     CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    sms = std::min(sms, tag_grid_max(512));
     int per = 0;
     CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_allreduce_probe, 512, 0));
     if (per < 1) return CBS3D_CUDA_ERROR;
@@ -4104,7 +4111,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             const void* fn = want == 4 ? fn_cgcg_single(rr, 0, 0) : hc3[c];
             int per_sm = 0;
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, 0));
-            int g = want == 4 ? sms : sms * (per_sm < 2 ? per_sm : 2);
+            int g = want == 4 ? std::min(sms, tag_grid_max(nt)) : sms * (per_sm < 2 ? per_sm : 2);
             if (cl) g = (nslices + nwarps * rr - 1) / (nwarps * rr);
             if (blocks_override > 0 && blocks_override < g) g = blocks_override;
             if (g > nslices) g = nslices > 0 ? nslices : 1;
@@ -4271,10 +4278,10 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         // the global-vector kernel with its neighbour values staged in shared
         // memory: each CTA's slices in the fewest parts (at most 8) whose
         // halos fit
-        const int g = nblocks;
         // automatic and choice 5: the single-reduction kernel; choice 1:
         // the two-reduction one (bitwise the same arithmetic as choices 2, 3)
         global_cgcg = kernel_choice != 1;
+        const int g = global_cgcg ? std::min(nblocks, tag_grid_max(PCG_THREADS)) : nblocks;
         const void* fh = global_cgcg ? reinterpret_cast<const void*>(k_pcg64g) : reinterpret_cast<const void*>(k_pcg64<true>);
         const GlobalHalo H = global_halo_in_parts(P, colp, g, global_cgcg);
         const size_t smem = H.table + H.table_bytes;
@@ -4301,6 +4308,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             CUDA_OK(cudaMemcpy(d_halo_idx, H.hidx.data(), H.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
             CUDA_OK(cudaMemcpy(d_lcol, H.lcol.data(), H.lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
             dev_halo_max = H.hmax;
+            nblocks = g;
             global_halo_parts = H.parts;
             global_halo = true;
             global_halo_smem = smem;
@@ -4735,7 +4743,7 @@ bool PcgBatch::plan(const PcgBatchPlan& p, std::string* why)
 
 bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::string* why)
 {
-    const int gmax = nt == 512 ? sms : 2 * sms, nwarps = nt / 32;
+    const int gmax = std::min(nt == 512 ? sms : 2 * sms, tag_grid_max(nt)), nwarps = nt / 32;
     if (p.rmax != 1 && p.rmax != 2 && p.rmax != 4 && p.rmax != 8) {
         if (why) *why = "rows per thread must be 1, 2, 4 or 8";
         return false;
