@@ -191,8 +191,6 @@ __device__ __forceinline__ SegView seg_view(const PcgDev& D)
 }
 __device__ __forceinline__ DevStatus* seg_status(const PcgDev& D, const SegView& g) { return g.k < 0 ? D.status : D.inst[g.k].status; }
 __device__ __forceinline__ CgOut* seg_out(const PcgDev& D, const SegView& g) { return g.k < 0 ? D.out : D.inst[g.k].out; }
-__device__ __forceinline__ unsigned* seg_bar(const PcgDev& D, const SegView& g) { return g.k < 0 ? D.bar : D.inst[g.k].bar; }
-__device__ __forceinline__ double* seg_part(const PcgDev& D, const SegView& g) { return g.k < 0 ? D.part : D.inst[g.k].part; }
 
 // ------------------------------------------------- deterministic reductions
 struct Acc4 {
@@ -834,8 +832,8 @@ __device__ __forceinline__ bool grid_allreduce_v(double (&v)[NV], const PcgDev& 
 #pragma unroll
         for (int q = 0; q < NV; ++q) sm[w][q] = v[q];
     __syncthreads();
-    unsigned long long* cnt = reinterpret_cast<unsigned long long*>(seg_bar(D, g));
-    double* part = seg_part(D, g) + (size_t)(phase & 1) * G * 8;
+    unsigned long long* cnt = reinterpret_cast<unsigned long long*>(D.bar);
+    double* part = D.part + (size_t)(phase & 1) * G * 8;
     if (threadIdx.x == 0) {
         double t[NV];
 #pragma unroll
@@ -938,8 +936,8 @@ __device__ __forceinline__ bool grid_allreduce3g(Acc6 v, double x, const PcgDev&
 #pragma unroll
         for (int q = 0; q < 6; ++q) sm[w][q] = vv[q];
     __syncthreads();
-    unsigned long long* cnt = reinterpret_cast<unsigned long long*>(seg_bar(D, g));
-    double* part = seg_part(D, g) + (size_t)(phase & 1) * G * 8;
+    unsigned long long* cnt = reinterpret_cast<unsigned long long*>(D.bar);
+    double* part = D.part + (size_t)(phase & 1) * G * 8;
     if (threadIdx.x == 0) {
         double t[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         for (int k = 0; k < NW; ++k)
@@ -4474,7 +4472,8 @@ cbs3d_status PcgEngine::solve(double* pres, double* rhs1, double* pdiag, int pre
     D.rel_tol = rel_tol; D.abs_tol = abs_tol; D.inner_tol = inner_tol;
     k_impose_perm_in<<<(NP + 255) / 256, 256, 0, st>>>(D, d_xp, d_bp, d_dp, d_fp);
     D.pres = d_xp; D.rhs1 = d_bp; D.pdiag = d_dp; D.nflag = d_fp;
-    CUDA_OK(cudaMemsetAsync(d_bar, 0, 4 * sizeof(unsigned), st));
+    // the counter of the kernels that do not exchange tagged records
+    if (!(variant == 4 && !coarse) && !(global_halo && global_cgcg)) CUDA_OK(cudaMemsetAsync(d_bar, 0, 4 * sizeof(unsigned), st));
     CUDA_OK(cudaMemsetAsync(d_out, 0, sizeof(CgOut), st));
     void* args[] = {&D};
     const void* fn = !global_halo ? reinterpret_cast<const void*>(k_pcg64<false>)
@@ -4688,8 +4687,6 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
         d_f32 = dalloc<float>(8 * n);
         CUDA_OK(cudaMemset(d_f32, 0, 8 * n * sizeof(float)));
     }
-    d_part = dalloc<double>(K * static_cast<size_t>(gmax) * 16);
-    d_bar = dalloc<unsigned>(4 * K);
     d_own = dalloc<int>(n);
     d_rec = dalloc<TagVal>(K * static_cast<size_t>(gmax) * 2 * REC_STRIDE);
     d_xw = dalloc<TagVal>(2 * n);
@@ -4701,7 +4698,6 @@ void PcgBatch::init(const std::vector<PcgBatchMember>& members, int dev_id, bool
         CUDA_OK(cudaMemcpy(d_epoch, one.data(), K * sizeof(unsigned long long), cudaMemcpyHostToDevice));
     }
     d_out = dalloc<CgOut>(K);
-    CUDA_OK(cudaMemset(d_bar, 0, 4 * K * sizeof(unsigned)));
     CUDA_OK(cudaMemset(d_out, 0, K * sizeof(CgOut)));
 
     base = PcgDev{};
@@ -4834,8 +4830,6 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
             I.max_iter = mem[static_cast<size_t>(k)].m->p.cg_max_iter;
             I.rel_tol = mem[static_cast<size_t>(k)].m->p.relToler;
             I.abs_tol = mem[static_cast<size_t>(k)].m->p.absToler;
-            I.bar = d_bar + 4 * k;
-            I.part = d_part + static_cast<size_t>(k) * static_cast<size_t>(this->gmax) * 16;
             I.rec = d_rec + static_cast<size_t>(k) * static_cast<size_t>(this->gmax) * 2 * REC_STRIDE;
             I.epoch = d_epoch + k;
             I.status = mem[static_cast<size_t>(k)].d_status;
@@ -5002,12 +4996,12 @@ void PcgBatch::release()
     d_cptr.clear();
     d_cent.clear();
     void* ptrs[] = {d_slice_off, d_slice_w, d_col, d_row_node, d_lcol, d_val, d_val32, d_r, d_z, d_pA, d_pB, d_q,
-                    d_xp, d_bp, d_dp, d_fp, d_f32, d_part, d_bar, d_out, d_own, d_rec, d_xw, d_epoch};
+                    d_xp, d_bp, d_dp, d_fp, d_f32, d_out, d_own, d_rec, d_xw, d_epoch};
     for (void* p : ptrs) if (p) cudaFree(p);
     d_own = nullptr; d_rec = d_xw = nullptr; d_epoch = nullptr;
     d_slice_off = nullptr; d_slice_w = d_col = d_row_node = nullptr; d_lcol = nullptr; d_val = nullptr;
     d_val32 = nullptr; d_r = d_z = d_pA = d_pB = d_q = nullptr; d_xp = d_bp = d_dp = nullptr; d_fp = nullptr;
-    d_f32 = nullptr; d_part = nullptr; d_bar = nullptr; d_out = nullptr;
+    d_f32 = nullptr; d_out = nullptr;
 }
 
 void PcgBatch::prepare(int k, const DevState& S, cudaStream_t st)
@@ -5029,7 +5023,6 @@ void PcgBatch::prepare(int k, const DevState& S, cudaStream_t st)
 
 void PcgBatch::solve(cudaStream_t st)
 {
-    CUDA_OK(cudaMemsetAsync(d_bar, 0, 4 * mem.size() * sizeof(unsigned), st));
     CUDA_OK(cudaMemsetAsync(d_out, 0, mem.size() * sizeof(CgOut), st));
     for (Wave& W : waves) {
         void* args[] = {&W.dev};

@@ -28,14 +28,12 @@ struct __align__(16) RemoteState {
 };
 
 // One instance of a batched solve: CTAs [cta0, cta0+ncta) of the launch own
-// slices [s0, s1); its own scalars, barrier counter, partials, status, result.
+// slices [s0, s1); its own scalars, records, status, result.
 struct PcgInst {
     int cta0, ncta, s0, s1;
     int precond, conv_test, max_iter, pad;
     double rel_tol, abs_tol;
-    unsigned* bar;               // 64-bit arrival counter (zeroed before each launch)
-    double* part;                // 2 * ncta * 8 partials (double-buffered by phase)
-    TagVal* rec;                 // 2 x ncta all-reduce records, a line each (single-reduction kernel)
+    TagVal* rec;                 // 2 x ncta all-reduce records, a line each
     unsigned long long* epoch;   // ... and the number of its next solve
     DevStatus* status;
     CgOut* out;
@@ -327,8 +325,6 @@ private:
     double *d_xp = nullptr, *d_bp = nullptr, *d_dp = nullptr;
     uint8_t* d_fp = nullptr;
     float* d_f32 = nullptr;
-    double* d_part = nullptr;
-    unsigned* d_bar = nullptr;
     int* d_own = nullptr;
     TagVal *d_rec = nullptr, *d_xw = nullptr;
     unsigned long long* d_epoch = nullptr;
