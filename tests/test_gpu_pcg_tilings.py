@@ -194,3 +194,48 @@ def test_global_vector_kernel_takes_one_more_part_for_its_slice_table():
     a.step(1)
     assert b.step(1).pcg_kernel == 8
     assert rel_l2(b.fields()[1], a.fields()[1]) <= 1e-8
+
+
+# the first and the last size of six rows per thread on 148 SMs
+@pytest.mark.parametrize("n", [72, 75])
+def test_six_rows_match_the_global_vector_kernel(n):
+    from cbs3d import cases
+    _same(cases.cavity(n, re=400.0, ntime=10 ** 6, jitter=0.15, seed=1234), steps=1)
+
+
+# rows of 26 neighbours (centred boxes: one row per thread, two in tensor
+# memory, three to five streamed) and of 18 (three in tensor memory, four
+# streamed): past the 16 slots that registers and requests hold
+@pytest.mark.parametrize("box,n", [("centred_box", 4), ("centred_box", 16), ("centred_box", 28), ("centred_box", 33),
+                                   ("centred_box", 37), ("centred_box", 40), ("five_tet_box", 58), ("five_tet_box", 64)])
+def test_wide_rows_match_the_global_vector_kernel(box, n):
+    import meshes
+    _same(meshes.cavity(getattr(meshes, box)(n, n, n)), steps=1)
+
+
+@pytest.mark.parametrize("n,ctas", [(2, 1), (6, 3), (10, 11)])
+def test_cluster_with_wide_rows(n, ctas):
+    import meshes
+    gpu = _gpu()
+    case = meshes.cavity(meshes.centred_box(n, n, n))
+    a, b = gpu.Context(case), gpu.Context(case, pcg_kernel=4, pcg_blocks=ctas)
+    sa, sb = a.step(2), b.step(2)
+    assert sa.cg_iterations_total == sb.cg_iterations_total
+    for x, y in zip(a.fields(), b.fields()):
+        assert bitwise(x, y)
+
+
+def test_batch_with_wide_rows():
+    import meshes
+    gpu = _gpu()
+    cs = [meshes.cavity(meshes.centred_box(n, n, n), re=100.0) for n in (12, 3, 17)]
+    for rows, spread in ((4, True), (4, False)):
+        b = gpu.Batch(cs, autotune=False, rows_per_thread=rows, spread=spread)
+        b.step(2)
+        for i, c in enumerate(cs):
+            x = gpu.Context(c)
+            x.step(2)
+            for p, q in zip(b.fields(i)[:2], x.fields()[:2]):
+                assert rel_l2(p, q) <= 1e-8
+            x.close()
+        b.close()
