@@ -4123,9 +4123,12 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if (want == 4) ++hmax;   // the spare place
             const CgcgLayout lay(hmax, remote.most, part.lcsb, CGCG_SMEM_MAX);
             const bool rg = want == 4 && lay.rg;
-            if (rg && (cl || !lay.rs || rr > RG_ROWS_MAX)) continue;
             const size_t smem = want == 4 ? lay.bytes : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
-            if (smem > (want == 4 ? CGCG_SMEM_MAX : 200 * 1024)) continue;
+            if ((rg && (cl || !lay.rs || rr > RG_ROWS_MAX)) || smem > (want == 4 ? CGCG_SMEM_MAX : 200 * 1024)) {
+                // more rows per thread on the same grid need as much
+                if (want == 4 && !cl) break;
+                continue;
+            }
             if (rg) fn = fn_cgcg_rg<false>(rr);
             std::vector<int> pptr;
             std::vector<int2> push;
