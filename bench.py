@@ -305,8 +305,10 @@ def timed_run(args, ctx, dist):
 def roofline(st, warm, nelem_fluid, npoin, mixed, n, pr, bound="l2"):
     """PCG kernel roofline: the kernel's own bytes per iteration over its
     CUDA-event time, against the L2 read bandwidth measured in this run
-    (bound "l2": the solve's operator and vectors stay in L2) or the HBM
-    figure (bound "hbm": MEASURED_PEAKS.json, else the fallback)."""
+    (bound "l2": the solve's operator and vectors stay in L2); with bound
+    "hbm" the DRAM bytes of the committed capture over the same time, against
+    the HBM figure (MEASURED_PEAKS.json, else the fallback), and the kernel's
+    own bytes, part of which L2 serves, beside it."""
     hbm, hbm_kind = measured_peak()
     its = st.cg_iterations_total - warm.cg_iterations_total   # totals are cumulative
     kb = float(st.pcg_bytes_per_iter)
@@ -318,9 +320,13 @@ def roofline(st, warm, nelem_fluid, npoin, mixed, n, pr, bound="l2"):
                "(cbs3d_probe_bandwidth, CUDA events)")
     else:
         peak, src = hbm, hbm_kind
+    traffic = ncu_traffic(kname, n, its / max(st.pcg_launches, 1))
+    requested = achieved
+    if bound == "hbm" and traffic and achieved:
+        achieved = traffic * st.pcg_launches / st.pcg_seconds / 1e9
     out = {"bound": bound, "achieved": achieved, "peak": peak, "unit": "GB/s",
            "frac": achieved / peak if achieved and peak else None,
-           "traffic": ncu_traffic(kname, n, its / max(st.pcg_launches, 1)),
+           "traffic": traffic,
            "traffic_unit": "DRAM bytes per launch (one pressure solve): ncu bytes per iteration x this run's "
                            "iterations per launch",
            "kernel": f"{kname} (persistent PCG, one launch per pressure solve)", "peak_source": src,
@@ -331,6 +337,10 @@ def roofline(st, warm, nelem_fluid, npoin, mixed, n, pr, bound="l2"):
         out["operator_storage"] = ("SELL coefficients held on chip in the SM's tensor memory for the whole solve "
                                    "(tcgen05.ld every iteration); kernel_bytes_per_iteration still counts them, "
                                    "with the vectors, as the algorithm's bytes")
+    if bound == "hbm":
+        out["kernel_gbs"] = requested
+        out["achieved_source"] = ("DRAM bytes per iteration of the committed ncu capture over this run's time" if traffic
+                                  else "the kernel's own bytes (no capture of this size): L2 hits included")
     if bound == "l2":
         out["hbm_peak"] = hbm
         out["hbm_peak_source"] = hbm_kind

@@ -4314,6 +4314,19 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             global_halo = true;
             global_halo_smem = smem;
             global_halo_total = static_cast<long long>(H.hidx.size());
+            // the slots that tensor memory holds (every other row of a warp)
+            g_tm_slots = 0;
+            for (int bb = 0; bb < g * PCG_WARPS; ++bb) {
+                const int b = bb / PCG_WARPS, warp = bb % PCG_WARPS;
+                const int sb = static_cast<int>(static_cast<long long>(b) * nslices / g);
+                const int se = static_cast<int>(static_cast<long long>(b + 1) * nslices / g);
+                for (int q = 0, left = g_tm_rows; q < H.parts; ++q) {
+                    const int p1 = sb + static_cast<int>(static_cast<long long>(q + 1) * (se - sb) / H.parts);
+                    for (int sl = sb + static_cast<int>(static_cast<long long>(q) * (se - sb) / H.parts) + warp;
+                         sl < p1 && left > 0; sl += 2 * PCG_WARPS, --left)
+                        g_tm_slots += 32LL * P.slice_w[static_cast<size_t>(sl)];
+                }
+            }
         } else {
             cgcg_tm_w = g_tm_rows = cgcg_lcs = 0;
         }
@@ -4605,13 +4618,14 @@ size_t PcgEngine::bytes_per_iter() const
     // shared-memory halo the columns are 16-bit and every halo entry's z and
     // previous p are read once per iteration.
     if (global_halo && global_cgcg) {
-        // single reduction: coefficient + 16-bit column per pair entry (those
-        // of the rows in tensor memory included); per
-        // node r, s, w of the previous iteration, p, pressure, inverse
-        // diagonal and diagonal read (56), node flag (1), p, pressure and the
-        // new r, s, w written (40); per halo entry r, s, w (24) and, with
-        // several parts per CTA, the inverse diagonal (8)
-        return static_cast<size_t>(nnz_offdiag) * 10 + static_cast<size_t>(N) * 97 +
+        // single reduction: coefficient + 16-bit column per pair entry, but
+        // for the rows in tensor memory; per node r, s, w of the previous
+        // iteration, p, pressure, inverse diagonal and diagonal read (56),
+        // node flag (1), p, pressure and the new r, s, w written (40); per
+        // halo entry r, s, w (24) and, with several parts per CTA, the inverse
+        // diagonal (8).  What L2 serves of that is counted too.
+        const double streamed = nslots > 0 ? 1.0 - static_cast<double>(g_tm_slots) / static_cast<double>(nslots) : 0.0;
+        return static_cast<size_t>(static_cast<double>(nnz_offdiag) * 10.0 * streamed) + static_cast<size_t>(N) * 97 +
                static_cast<size_t>(global_halo_total) * (global_halo_parts > 1 ? 32 : 24);
     }
     if (global_halo)

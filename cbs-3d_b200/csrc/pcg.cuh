@@ -196,6 +196,7 @@ public:
     int cgcg_coef_off = 0;   // where they start
     int cgcg_kt = 0;         // >0: that many rows per thread, after the shared-memory one, read from tensor memory
     int g_tm_rows = 0;       // rows per warp of the global-vector CG-CG kernel in tensor memory
+    long long g_tm_slots = 0;   // ... and the slots of all of them
     int cgcg_tm_w = 0;       // slots per row in tensor memory
     int cgcg_pds_off = 0;    // where the rows' diagonal starts in shared memory (0: global memory)
     int cgcg_xs_off = 0;     // ... and their pressure
