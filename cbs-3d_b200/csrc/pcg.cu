@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64r(PcgDev 
     if (!conv && b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 2, ST_PCG, it, R_PCG_MAXIT);
 }
 
-// ---------------------------------------- halo-staged FP64 PCG (default)
+// --------------------------------------- halo-staged FP64 PCG (choice 3)
 // The register-resident algorithm of k_pcg64r with the neighbour gathers
 // served from shared memory.  Each persistent CTA owns a contiguous block of
 // slices; the host lists, per CTA, the distinct nodes its rows reference (its
@@ -786,17 +786,15 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64h(PcgDev 
     if (!conv && b == 0 && threadIdx.x == 0) set_status(seg_status(D, g), 2, ST_PCG, it, R_PCG_MAXIT);
 }
 
-// --------------------------- single-synchronisation halo PCG (default)
+// ------------------------------------------- single-synchronisation PCG
 // Chronopoulos-Gear form of the same Jacobi-PCG: the matvec is applied to z
 // (w = A z) and the direction's product s = A p follows the recurrence
 // s = w + beta*s, so alpha and beta come from one grid reduction of
 // (r.z, z.w, r.r, max|r|) per iteration instead of two.  Residuals, stopping
 // test, iteration count and breakdown checks keep the reference's meaning
 // (src/linalg/ConjugateGradient.cpp:725-853); in exact arithmetic the iterates
-// equal the standard PCG's.  Neighbour values of the new z are formed while
-// the halo is staged, from the previous iteration's r, w, s (double-buffered
-// by iteration parity) and the diagonal, with the same operations the owner
-// applies to its own rows.
+// equal the standard PCG's.  k_pcg64c (the default), k_pcg64g, k_pcg64d and
+// k_pcg32m are this iteration.
 struct Acc6 {
     double a, b, c, mx, flag;
 };
@@ -1778,11 +1776,12 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_CTAS_PER_SM) k_pcg64g(PcgDev 
 // all-reduce).  The records are requested when the other CTAs' partials have
 // come in -- a CTA stores its w before its partials, so they are there, and
 // polling them earlier would slow their stores -- and travel while the
-// partials are folded; neither exchange needs a fence.  The own rows' new z go from registers into the halo.
+// partials are folded; neither exchange needs a fence.  The own rows' new z go
+// from registers into the halo.
 //
-// Bound at 64^3: shared-memory wavefronts of the gathers (27,000 per CTA and
-// iteration, at two 64-bit wavefronts per 32 and the bank conflicts left) and
-// the latency of the all-reduce.
+// Bound at 64^3 (13,700 cycles per iteration): instruction issue (44% of the
+// cycles), the shared-memory wavefronts (5,630 per CTA and iteration, about
+// 3,280 of them the gathers) and the latency of the all-reduce.
 //
 // KT > 0: the coefficients of each thread's rows KS .. KS+KT-1 live in TMEM
 // for the solve (D.tm_w slots per row, zero-padded past the slice's width);
