@@ -3622,7 +3622,7 @@ constexpr int CGCG_HALO_MAX = 8190;
 // of them remote, and lcsb bytes of columns: the remote entries' state in
 // shared memory where it fits `limit` bytes, else in global memory, r and s
 // staying where they alone fit.  64^3 without coordinates: 226,880 bytes in
-// the first form, 183,608 in the second.
+// the first form, 167,920 in the second.
 struct CgcgLayout {
     bool rg;
     size_t lcs, rs, bytes;

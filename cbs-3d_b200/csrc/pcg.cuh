@@ -137,7 +137,7 @@ cbs3d_status probe_partition(int nelem, int npoin, const int* intma, const int* 
 // Owns the device copies of the pattern and the PCG work vectors.
 class PcgEngine {
 public:
-    // kernel_choice: 0 automatic (4, else 3, else 2, else 5), 1 vectors in global memory,
+    // kernel_choice: 0 automatic (4, else 5, else 2), 1 vectors in global memory,
     // 2 register-resident rows, 3 with the halo staged in shared memory,
     // 4 as 3 with one grid synchronisation per iteration (Chronopoulos-Gear),
     // 5 vectors in global memory with one grid synchronisation per iteration

@@ -353,9 +353,10 @@ cbs3d_status cbs3d_heat_adjoint_run(cbs3d_ctx* ctx, int nsteps, int every, const
 typedef struct cbs3d_batch cbs3d_batch;
 
 typedef struct cbs3d_batch_options {
-    cbs3d_options base;      /* precision, device, inner_tol, use_graph (pcg_kernel/pcg_blocks unused) */
+    cbs3d_options base;      /* precision (MIXED: the FP32 kernel where every wave fits it, else
+                                FP64), device, inner_tol, use_graph (pcg_kernel/pcg_blocks unused) */
     int autotune;            /* 1: on the first step time every feasible PCG tiling on the real
-                                systems and keep the fastest */
+                                systems (MIXED: in FP64 too) and keep the fastest */
     int rows_per_thread;     /* tiling without autotune: 1, 2, 4 or 8 slices of 32 rows per warp
                                 (0: 4) */
     int spread;              /* 1: a wave's spare CTAs are shared out by instance size; 0: each
