@@ -3839,15 +3839,13 @@ const void* fn_cgcg_single(int rmax, int ks, int kt)
              : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, false, 512, 0, 3>)
              : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512, 0, 4>)
              : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512, 0, 4>)
-             : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512, 0, 4>)
-                         : reinterpret_cast<const void*>(k_pcg64c<8, false, 512, 0, 4>);
+                         : reinterpret_cast<const void*>(k_pcg64c<6, false, 512, 0, 4>);
     return rmax == 1 ? reinterpret_cast<const void*>(k_pcg64c<1, false, 512>)
          : rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, false, 512>)
          : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, false, 512>)
          : rmax == 4 ? reinterpret_cast<const void*>(k_pcg64c<4, false, 512>)
          : rmax == 5 ? reinterpret_cast<const void*>(k_pcg64c<5, false, 512>)
-         : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, false, 512>)
-                     : reinterpret_cast<const void*>(k_pcg64c<8, false, 512>);
+                     : reinterpret_cast<const void*>(k_pcg64c<6, false, 512>);
 }
 
 // ... with the remote entries' state in global memory, up to four rows
@@ -3884,6 +3882,25 @@ void coarse_invert_launch(int g, double* a, cudaStream_t st)
 {
     k_coarse_invert_reg<<<1, 512, 0, st>>>(g, a);
 }
+
+namespace {
+// Whether the two-level kernel can run on a partition over G CTAs: its layout,
+// and the coarse inverse's, in one CTA's shared memory.
+bool two_level_fits(const CoarseNeighbours& nb, int G, int rows, int halo_max, int slot_max, int sms, size_t& smem,
+                    size_t& ismem)
+{
+    if (G > 160 || !nb.fits) return false;
+    smem = TwoLevelLayout(halo_max, slot_max, nb.most, G).bytes;
+    ismem = (static_cast<size_t>(G) * G + 2 * static_cast<size_t>(G)) * 8;
+    const void* fn = fn_twolevel(rows);
+    int per = 0;
+    const bool ok = smem <= 220 * 1024 && ismem <= 220 * 1024 && raise_smem_limit(fn, smem) == cudaSuccess &&
+                    raise_smem_limit(reinterpret_cast<const void*>(k_coarse_invert), ismem) == cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 512, smem) == cudaSuccess && per * sms >= G;
+    cudaGetLastError();
+    return ok;
+}
+}  // namespace
 
 cudaError_t pcg_raise_smem_limit(const void* fn, size_t smem) { return raise_smem_limit(fn, smem); }
 
@@ -3931,7 +3948,6 @@ void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
 {
     const int G = nblocks;
     const PressurePattern& P = m.pat;
-    if (G > 160) return;   // the inverse must fit one CTA's shared memory
     std::vector<int> cta_of_slice(static_cast<size_t>(nslices), 0);
     for (int b = 0; b < G; ++b) {
         const int sb = static_cast<int>(static_cast<long long>(b) * nslices / G);
@@ -3972,17 +3988,6 @@ void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
             ij.push_back(make_int2(I, J));
         }
     const CoarseNeighbours nb = coarse_neighbours(nslices, h_hptr, h_hidx);
-    if (!nb.fits) return;
-    const size_t smem = TwoLevelLayout(dev_halo_max, dev_slot_max, nb.most, G).bytes;
-    const size_t ismem = (static_cast<size_t>(G) * G + 2 * static_cast<size_t>(G)) * 8;
-    const void* fn = fn_twolevel(rmax);
-    int per = 0;
-    if (smem > 220 * 1024 || ismem > 220 * 1024 || raise_smem_limit(fn, smem) != cudaSuccess ||
-        raise_smem_limit(reinterpret_cast<const void*>(k_coarse_invert), ismem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 512, smem) != cudaSuccess || per * sms_ < G) {
-        cudaGetLastError();
-        return;
-    }
     npairs = static_cast<int>(ij.size());
     d_pair_ptr = dalloc<int>(ptr.size());
     d_pair_ij = dalloc<int2>(ij.size());
@@ -3998,8 +4003,6 @@ void PcgEngine::build_coarse(const HostModel& m, const std::vector<int>& colp)
     CUDA_OK(cudaMemcpy(d_nbr_ids, nb.ids.data(), nb.ids.size() * sizeof(int), cudaMemcpyHostToDevice));
     if (!nb.hown.empty()) CUDA_OK(cudaMemcpy(d_hown, nb.hown.data(), nb.hown.size(), cudaMemcpyHostToDevice));
     cdev = CoarseDev{G, nb.most, d_nbr_ptr, d_nbr_ids, d_hown, d_ac};
-    coarse_smem = smem;
-    coarse_ismem = ismem;
     coarse = true;
 }
 
@@ -4049,7 +4052,6 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
 
     int sms = 0;
     CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    sms_ = sms;
     // Register-resident kernel when every thread's rows fit its register
     // arrays; otherwise the kernel that keeps the vectors in global memory.
     auto grid_for = [&](const void* fn) {
@@ -4079,6 +4081,19 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
         cudaGetLastError();
         return ok;
     };
+    auto upload_partition = [&](const Partition& part, int hmax) {
+        d_halo_ptr = dalloc<int>(part.hptr.size());
+        d_halo_idx = dalloc<int>(part.hidx.size());
+        d_lcol = dalloc<unsigned short>(part.lcol.size());
+        CUDA_OK(cudaMemcpy(d_halo_ptr, part.hptr.data(), part.hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+        CUDA_OK(cudaMemcpy(d_halo_idx, part.hidx.data(), part.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
+        if (!part.lcol.empty()) CUDA_OK(cudaMemcpy(d_lcol, part.lcol.data(), part.lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+        dev_halo_max = hmax;
+        dev_slot_max = static_cast<int>(part.smax);
+        h_hptr = part.hptr;
+        h_hidx = part.hidx;
+    };
+    bool coarse_planned = false;
     rmax = 0;
     variant = 1;
     nblocks = grid_for(reinterpret_cast<const void*>(k_pcg64<false>));
@@ -4087,25 +4102,30 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                               reinterpret_cast<const void*>(k_pcg64h<4>), reinterpret_cast<const void*>(k_pcg64h<8>)};
         const int want = kernel_choice == 3 ? 3 : 4;
         const int nt = PCG_THREADS, nwarps = nt / 32;
-        // rows per thread: the mixed and the two-level kernel, which share the
-        // single-reduction kernel's partition, have 1, 2, 4 and 8; that one
-        // itself up to six (beyond, the global-vector kernel is as fast:
-        // 76^3 22.0 us per iteration against 25.4 with eight rows)
-        struct Tiling { int rows; bool cluster; };
+        // rows per thread: the mixed and the two-level kernel ("special") have
+        // 1, 2, 4 and 8; the single-reduction kernel up to six (beyond, the
+        // global-vector kernel is as fast: 76^3 22.0 us per iteration against
+        // 25.4 with eight rows).  A mesh that the special kernel does not fit
+        // is tiled as without the option (76^3 in mixed precision, a step: 25.2
+        // ms with eight rows, 16.4 on the kernel that Jacobi takes there).
+        struct Tiling { int rows; bool cluster, special; };
         std::vector<Tiling> tilings;
-        if (want == 3 || mixed || two_level) {
-            tilings = {{1, false}, {2, false}, {4, false}, {8, false}};
-        } else {
+        if (want == 3 || mixed || two_level)
+            for (int r : {1, 2, 4, 8}) tilings.push_back({r, false, want == 4});
+        if (want == 4) {
             // one cluster where it holds the mesh at one row per thread (16^3
             // 2.00 us per iteration against 2.37 on the whole chip; at two
             // rows 3.0 against 2.4, as the chip then has one row per thread)
-            if (kernel_choice == 0 && blocks_override <= 0 && nslices <= CLUSTER_MAX * nwarps) tilings.push_back({1, true});
-            for (int r = 1; r <= 6; ++r) tilings.push_back({r, false});
+            if (kernel_choice == 0 && blocks_override <= 0 && nslices <= CLUSTER_MAX * nwarps) tilings.push_back({1, true, false});
+            for (int r = 1; r <= 6; ++r) tilings.push_back({r, false, false});
         }
+        bool special_fits = true;
         for (int c = 0; c < static_cast<int>(tilings.size()) && variant == 1; ++c) {
             const int rr = tilings[static_cast<size_t>(c)].rows;
             const bool cl = tilings[static_cast<size_t>(c)].cluster;
-            const void* fn = want == 4 ? fn_cgcg_single(rr, 0, 0) : hc3[c];
+            const bool special = tilings[static_cast<size_t>(c)].special;
+            if (special && !special_fits) continue;
+            const void* fn = want == 3 ? hc3[c] : special ? fn_mixed<false, 512>(rr) : fn_cgcg_single(rr, 0, 0);
             int per_sm = 0;
             CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, 0));
             int g = want == 4 ? std::min(sms, tag_grid_max(nt)) : sms * (per_sm < 2 ? per_sm : 2);
@@ -4118,8 +4138,34 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             int hmax = part.hmax;
             const long long smax = part.smax;
             const RemoteLists& remote = part.remote;
-            if (!part.fits) continue;
+            if (!part.fits) {
+                special_fits = false;
+                continue;
+            }
             if (want == 4) ++hmax;   // the spare place
+            if (special) {
+                const size_t ms = static_cast<size_t>(hmax) * 16 + static_cast<size_t>(smax) * 6 + 16;
+                mixed_ok = mixed && ms <= 220 * 1024 && raise_smem_limit(fn, ms) == cudaSuccess &&
+                           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, nt, ms) == cudaSuccess && per_sm * sms >= g;
+                cudaGetLastError();
+                // the two-level kernel needs rows for every warp of the grid
+                const bool two = !mixed_ok && two_level && nslices >= 16 * sms &&
+                                 two_level_fits(coarse_neighbours(nslices, part.hptr, part.hidx), g, rr, hmax,
+                                                static_cast<int>(smax), sms, coarse_smem, coarse_ismem);
+                if (!mixed_ok && !two) {
+                    special_fits = false;
+                    continue;
+                }
+                mixed_smem = ms;
+                coarse_planned = two;
+                variant = 4;
+                nthreads = nt;
+                rmax = rr;
+                nblocks = g;
+                rem_total = static_cast<long long>(remote.rem.size());
+                upload_partition(part, hmax);
+                break;
+            }
             const CgcgLayout lay(hmax, remote.most, part.lcsb, CGCG_SMEM_MAX);
             const bool rg = want == 4 && lay.rg;
             const size_t smem = want == 4 ? lay.bytes : static_cast<size_t>(hmax) * 12 + static_cast<size_t>(smax) * 2 + 16;
@@ -4224,16 +4270,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                     cgcg_xs_off = static_cast<int>(off);
                 }
             }
-            d_halo_ptr = dalloc<int>(part.hptr.size());
-            d_halo_idx = dalloc<int>(part.hidx.size());
-            d_lcol = dalloc<unsigned short>(part.lcol.size());
-            CUDA_OK(cudaMemcpy(d_halo_ptr, part.hptr.data(), part.hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CUDA_OK(cudaMemcpy(d_halo_idx, part.hidx.data(), part.hidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-            if (!part.lcol.empty()) CUDA_OK(cudaMemcpy(d_lcol, part.lcol.data(), part.lcol.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
-            dev_halo_max = hmax;
-            dev_slot_max = static_cast<int>(smax);
-            h_hptr = part.hptr;
-            h_hidx = part.hidx;
+            upload_partition(part, hmax);
             if (want == 4) {
                 dev_rem_max = remote.most;
                 rem_total = static_cast<long long>(remote.rem.size());
@@ -4257,20 +4294,6 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
                     CUDA_OK(cudaMemcpy(d_push_ptr, pptr.data(), pptr.size() * sizeof(int), cudaMemcpyHostToDevice));
                     if (!push.empty()) CUDA_OK(cudaMemcpy(d_push, push.data(), push.size() * sizeof(int2), cudaMemcpyHostToDevice));
                 }
-            }
-            if (mixed && want == 4) {
-                const void* mc[4] = {fn_mixed<false, 512>(1), fn_mixed<false, 512>(2), fn_mixed<false, 512>(4),
-                                     fn_mixed<false, 512>(8)};
-                const size_t ms = static_cast<size_t>(hmax) * 16 + static_cast<size_t>(smax) * 6 + 16;
-                int per = 0;
-                if (ms <= 220 * 1024 &&
-                    raise_smem_limit(mc[c], ms) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, mc[c], nt, ms) == cudaSuccess &&
-                    per * sms >= g) {
-                    mixed_ok = true;
-                    mixed_smem = ms;
-                }
-                cudaGetLastError();
             }
         }
     }
@@ -4343,8 +4366,7 @@ void PcgEngine::init(const HostModel& m, const uint8_t* nflag, const double* pfi
             if ((per_cta + PCG_WARPS - 1) / PCG_WARPS <= rm[c]) { rmax = rm[c]; nblocks = g; variant = 2; break; }
         }
     }
-    // the two-level preconditioner needs rows for every warp of the grid
-    if (two_level && variant == 4 && nslices >= 16 * sms && !mixed_ok) build_coarse(m, colp);
+    if (coarse_planned) build_coarse(m, colp);
     if (multigrid && !mixed && !coarse) {
         mgh = new MgHierarchy;
         bool ok = false;

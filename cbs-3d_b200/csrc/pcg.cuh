@@ -175,7 +175,7 @@ public:
     bool coarse = false;     // two-level preconditioner in use
     bool coarse_ready = false;   // prepare_coarse ran for the next solve
     size_t coarse_smem = 0, coarse_ismem = 0;
-    int npairs = 0, sms_ = 0;
+    int npairs = 0;
     int *d_pair_ptr = nullptr, *d_pair_ent = nullptr, *d_nbr_ptr = nullptr, *d_nbr_ids = nullptr;
     int2* d_pair_ij = nullptr;
     double* d_ac = nullptr;

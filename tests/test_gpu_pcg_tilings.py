@@ -239,3 +239,17 @@ def test_batch_with_wide_rows():
                 assert rel_l2(p, q) <= 1e-8
             x.close()
         b.close()
+
+
+@pytest.mark.parametrize("option,n", [("mixed", 70), ("mixed", 76), ("two_level", 76), ("two_level", 20)])
+def test_options_that_do_not_fit_run_the_plain_engine(option, n):
+    """Where the mixed-precision or the two-level kernel does not fit the mesh
+    (too many rows per CTA, or too few), the solve is the Jacobi engine's."""
+    from cbs3d import cases
+    gpu = _gpu()
+    case = cases.cavity(n, re=400.0, ntime=10 ** 6, jitter=0.15, seed=1234)
+    a = gpu.Context(case)
+    b = gpu.Context(case, precision=gpu.MIXED) if option == "mixed" else gpu.Context(case, two_level=True)
+    assert a.step(1).pcg_kernel == b.step(1).pcg_kernel
+    for x, y in zip(a.fields(), b.fields()):
+        assert bitwise(x, y)
