@@ -3869,6 +3869,13 @@ const void* fn_cgcg_batch512(int rmax)
          : rmax == 6 ? reinterpret_cast<const void*>(k_pcg64c<6, true, 512, 0, 4>)
                      : reinterpret_cast<const void*>(k_pcg64c<8, true, 512, 0, 4>);
 }
+// ... with rows wider than tensor memory holds (up to four)
+const void* fn_cgcg_batch512_wide(int rmax)
+{
+    return rmax == 2 ? reinterpret_cast<const void*>(k_pcg64c<2, true, 512>)
+         : rmax == 3 ? reinterpret_cast<const void*>(k_pcg64c<3, true, 512>)
+                     : reinterpret_cast<const void*>(k_pcg64c<4, true, 512>);
+}
 // ... and the form that runs on one cluster
 const void* fn_cgcg_cluster() { return reinterpret_cast<const void*>(k_pcg64c<1, false, 512, 0, 0, true>); }
 
@@ -4931,12 +4938,18 @@ bool PcgBatch::plan_threads(const PcgBatchPlan& p, int nt, bool all_fp32, std::s
                 for (int q = I.s0; q < I.s1; ++q) wmx = std::max(wmx, h_slice_w[static_cast<size_t>(q)]);
             const int ch = CGCG_ROUND, tw = (wmx + ch - 1) / ch * ch, kt = std::min(H.rows, 4);
             const CgcgLayout lay(H.hmax + 1, H.rmost, H.lcsb, CGCG_SMEM_MAX);
+            // rows too wide for tensor memory stream their coefficients from
+            // L2 (centred boxes of 28 and 32, rows of 26 neighbours: 8.1 ms a
+            // step against 9.4 on 256-thread CTAs).  A wave on at most half
+            // the SMs is faster on twice as many CTAs of 256 threads then
+            // (centred boxes of 6 to 20 on the fewest CTAs: 4.2 against 5.8)
+            const bool wide = !lay.rg && H.rows > 1 && kt * tw > 64;
             W.rg = lay.rg;
-            W.fn = lay.rg ? fn_cgcg_rg<true>(H.rows) : fn_cgcg_batch512(H.rows);
+            W.fn = lay.rg ? fn_cgcg_rg<true>(H.rows) : wide ? fn_cgcg_batch512_wide(H.rows) : fn_cgcg_batch512(H.rows);
             W.smem = lay.bytes;
             W.lcs_off = static_cast<int>(lay.lcs);
             W.rs_off = static_cast<int>(lay.rs);
-            if ((lay.rg ? !lay.rs || H.rows > RG_ROWS_MAX : H.rows > 1 && kt * tw > 64) || !fits(W.fn, W.smem)) {
+            if ((lay.rg && (!lay.rs || H.rows > RG_ROWS_MAX)) || (wide && (2 * H.G <= sms || H.rows > 4)) || !fits(W.fn, W.smem)) {
                 if (why) *why = "a wave does not fit co-resident at this tiling";
                 return false;
             }

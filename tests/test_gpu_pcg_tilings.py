@@ -253,3 +253,19 @@ def test_options_that_do_not_fit_run_the_plain_engine(option, n):
     assert a.step(1).pcg_kernel == b.step(1).pcg_kernel
     for x, y in zip(a.fields(), b.fields()):
         assert bitwise(x, y)
+
+
+def test_large_batch_with_wide_rows():
+    """Four rows per thread of 26 neighbours, which tensor memory does not
+    hold, on CTAs of 512 threads."""
+    import meshes
+    gpu = _gpu()
+    cs = [meshes.cavity(meshes.centred_box(n, n, n), re=100.0) for n in (30, 27)]
+    b = gpu.Batch(cs, autotune=False)
+    b.step(1)
+    for i, c in enumerate(cs):
+        x = gpu.Context(c)
+        x.step(1)
+        for p, q in zip(b.fields(i)[:2], x.fields()[:2]):
+            assert rel_l2(p, q) <= 1e-8
+        x.close()
